@@ -57,6 +57,10 @@ def _compile(src, verbose):
     elif base.startswith("hess_") and base != "hess_dispatch":
         deps += [os.path.join(GEN, base + ".cuh"), os.path.join(GEN, "class_" + base[5:] + ".cuh"),
                  os.path.join(CSRC, "hfgpu_hess_kernels.cuh"), os.path.join(CSRC, "hfgpu_hess_launch.h")]
+    elif base.startswith("rys_"):
+        deps += [os.path.join(GEN, "rys_layout.cuh"), os.path.join(CSRC, "hfgpu_rys.cuh"),
+                 os.path.join(CSRC, "hfgpu_rys_math.cuh"),
+                 os.path.join(CSRC, "hfgpu_rys_launch.h")]
     else:  # hand-written sources: every hand-written header counts
         deps += sorted(glob.glob(os.path.join(CSRC, "*.cuh")) + glob.glob(os.path.join(CSRC, "*.h")))
     stamp = obj + ".sha1"
@@ -79,6 +83,7 @@ def build(jobs: int | None = None, verbose: bool = False) -> str:
     os.makedirs(OBJ, exist_ok=True)
     generate()
     srcs = sorted(glob.glob(os.path.join(GEN, "inst_*.cu"))) + sorted(glob.glob(os.path.join(GEN, "hess_*.cu"))) + \
+        sorted(glob.glob(os.path.join(GEN, "rys_*.cu"))) + \
         [os.path.join(GEN, "dispatch.cu"),
                                                                  os.path.join(CSRC, "hfgpu_host.cu"),
                                                                  os.path.join(CSRC, "hfgpu_noalloc.cu"),

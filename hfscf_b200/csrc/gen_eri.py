@@ -801,23 +801,6 @@ def class_header(c):
         code_g, mg = gen_grad_table(*c)
     parts += [code_g, ""]
     mg["table"] = not straight
-    # the op-table classes also get the warp-per-quartet form (measured faster than one thread
-    # per quartet on global scratch for every one of them).  The straight-line classes keep one
-    # thread per quartet: warp forms generated for those with more than 150 accumulators measured
-    # slower at n-octane and anthracene sizes (29.6 against 25.7 ms and 216 against 189 ms per
-    # gradient), and with the block forms offered to the autotuner as well it kept the four-pass
-    # thread form for all but one of them (octane 17.9 -> 17.0 ms, anthracene 135 -> 121 ms, for
-    # 3-8x the tuning time)
-    gwarp = not straight
-    if gwarp:
-        gwcode, gwmeta = gen_grad_warp(*c)
-        parts += [gwcode, ""]
-        mg["grad_warp"] = gwmeta
-        # and the per-set split of the warp form: four one-set tables, four launches
-        for ps in GRAD_SETS:
-            pcode, pmeta = gen_grad_warp(*c, sets=(ps,), suffix="_" + ps)
-            parts += [pcode, ""]
-            mg["grad_warp_" + ps] = pmeta
     parts.append(f"template <>")
     parts.append(f"struct ClassCode<{la}, {lb}, {lc}, {ld}> {{")
     parts.append(f"  static constexpr bool kGradTable = {'false' if straight else 'true'};")
@@ -825,10 +808,6 @@ def class_header(c):
     parts.append(f"  static constexpr bool kWarpDefault = {'true' if m['vrr_values'] >= WARP_DEFAULT_MIN_VRR else 'false'};")
     parts.append(f"  using WarpTab = {'WarpTab' + t if warp else 'void'};")
     parts.append(f"  using GradTab = {'void' if straight else 'GradTable' + t};")
-    parts.append(f"  static constexpr bool kGradWarp = {'true' if gwarp else 'false'};")
-    parts.append(f"  using GradWarpTab = {'GradWarpTab' + t if gwarp else 'void'};")
-    for pi, ps in enumerate(GRAD_SETS):
-        parts.append(f"  using GradWarpTabP{pi} = {'GradWarpTab' + t + '_' + ps if gwarp else 'void'};")
     parts.append(f"  static constexpr bool kPrimWarp = {'true' if primwarp else 'false'};")
     parts.append(f"  static constexpr int kCapBlocks = {cap_blocks(m['vrr_values'])};")
     # the persistent form with the Boys table in shared memory: classes of total L <= STAGED_MAX_L
@@ -992,54 +971,6 @@ static void launch_grad(const GradArgs<R>& a, int pure, const int2* q, int nq, i
     grad_kernel<{la}, {lb}, {lc}, {ld}, R><<<grid, 128, sm, s>>>(a, pure, q, nq);
   }}
 }}
-template <typename Tab, typename R, int NT>
-static bool launch_grad_warp_nt(const GradArgs<R>& a, int pure, const int2* q, int nq, cudaStream_t s) {{
-  constexpr size_t bytes = sizeof(R) * (size_t)grad_warp_slots<Tab, R>();
-  if (bytes > 232448) return false;  // more shared memory than one block may have
-  auto k = grad_warp_kernel<{la}, {lb}, {lc}, {ld}, R, Tab, NT>;
-  cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
-  k<<<nq, NT, bytes, s>>>(a, pure, q, nq);
-  return true;
-}}
-template <typename Tab, typename R>
-static bool launch_grad_warp_tab(const GradArgs<R>& a, int pure, const int2* q, int nq, cudaStream_t s) {{
-  // one warp per quartet, or one block of four or eight warps per quartet
-  if (a.warp_threads == 256) return launch_grad_warp_nt<Tab, R, 256>(a, pure, q, nq, s);
-  if (a.warp_threads == 128) return launch_grad_warp_nt<Tab, R, 128>(a, pure, q, nq, s);
-  return launch_grad_warp_nt<Tab, R, 32>(a, pure, q, nq, s);
-}}
-template <typename CC, typename R>
-static bool launch_grad_warp_impl(const GradArgs<R>& a, int pure, const int2* q, int nq, cudaStream_t s) {{
-  if constexpr (CC::kGradWarp) {{
-    if (a.warp_split) {{
-      // one launch per accumulator set (smaller tables: more warps per SM); each adds its part
-      return launch_grad_warp_tab<typename CC::GradWarpTabP0, R>(a, pure, q, nq, s) &&
-             launch_grad_warp_tab<typename CC::GradWarpTabP1, R>(a, pure, q, nq, s) &&
-             launch_grad_warp_tab<typename CC::GradWarpTabP2, R>(a, pure, q, nq, s) &&
-             launch_grad_warp_tab<typename CC::GradWarpTabP3, R>(a, pure, q, nq, s);
-    }}
-    return launch_grad_warp_tab<typename CC::GradWarpTab, R>(a, pure, q, nq, s);
-  }} else {{
-    return false;
-  }}
-}}
-template <typename CC, typename R>
-static int grad_warp_bytes_impl() {{
-  if constexpr (CC::kGradWarp) {{
-    return (int)(sizeof(R) * (size_t)grad_warp_slots<typename CC::GradWarpTab, R>());
-  }} else {{
-    return 0;
-  }}
-}}
-static int grad_warp_bytes(int fp32) {{
-  return fp32 ? grad_warp_bytes_impl<ClassCode<{la}, {lb}, {lc}, {ld}>, float>()
-              : grad_warp_bytes_impl<ClassCode<{la}, {lb}, {lc}, {ld}>, double>();
-}}
-template <typename R>
-static bool launch_grad_warp(const GradArgs<R>& a, int pure, const int2* q, int nq, cudaStream_t s) {{
-  if (nq <= 0) return true;
-  return launch_grad_warp_impl<ClassCode<{la}, {lb}, {lc}, {ld}>, R>(a, pure, q, nq, s);
-}}
 template <typename CC, int NCART>
 static int grad_scratch_slots_impl() {{
   if constexpr (CC::kGradTable) {{
@@ -1059,8 +990,6 @@ const ClassLaunchers launchers_{t} = {{{la}, {lb}, {lc}, {ld}, &launch_quartet<d
                                       &launch_primwarp<double>, &launch_primwarp<float>,
                                       ClassCode<{la}, {lb}, {lc}, {ld}>::kWarp,
                                       ClassCode<{la}, {lb}, {lc}, {ld}>::kWarpDefault,
-                                      ClassCode<{la}, {lb}, {lc}, {ld}>::kGradWarp,
-                                      &launch_grad_warp<double>, &launch_grad_warp<float>, &grad_warp_bytes,
                                       ClassCode<{la}, {lb}, {lc}, {ld}>::kCapBlocks > 0,
                                       ClassCode<{la}, {lb}, {lc}, {ld}>::kStaged,
                                       ClassCode<{la}, {lb}, {lc}, {ld}>::kLowRes}};
@@ -1085,45 +1014,9 @@ static int hess_scratch_slots(int) {{
   return HessTable{t}::NVSLOT + HessTable{t}::NHSLOT + 45 +
          3 * BlockDims<{la}, {lb}, {lc}, {ld}, false>::NCART;
 }}
-// block form: the whole table in shared memory when it fits, else the HRR slots in global scratch
-constexpr size_t kSmAll = sizeof(double) * hess_block_shared_doubles<HessBlockTab{t}>(false);
-constexpr size_t kSmPart = sizeof(double) * hess_block_shared_doubles<HessBlockTab{t}>(true);
-constexpr size_t kSmMax = 227 * 1024;
-static int hess_block_global_slots() {{ return kSmAll <= kSmMax ? 0 : HessBlockTab{t}::NHSLOT + 1; }}
-static bool launch_hess_block(const GradArgs<double>& a, const HessOut& o, int pure, const int2* q, int nq, int grid,
-                              cudaStream_t s) {{
-  if (nq <= 0) return true;
-  if constexpr (kSmAll <= kSmMax) {{
-    auto k = hess_block_kernel<{la}, {lb}, {lc}, {ld}, HessBlockTab{t}, false>;
-    if (kSmAll > 48 * 1024) cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmAll);
-    k<<<grid, 128, kSmAll, s>>>(a, o, pure, q, nq);
-    return true;
-  }} else if constexpr (kSmPart <= kSmMax) {{
-    auto k = hess_block_kernel<{la}, {lb}, {lc}, {ld}, HessBlockTab{t}, true>;
-    if (kSmPart > 48 * 1024) cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmPart);
-    k<<<grid, 128, kSmPart, s>>>(a, o, pure, q, nq);
-    return true;
-  }} else {{
-    return false;
-  }}
-}}
-// warp form: four quartets per 128-thread block, one warp each, every warp's tables in shared memory
-static bool launch_hess_warp(const GradArgs<double>& a, const HessOut& o, int pure, const int2* q, int nq,
-                             cudaStream_t s) {{
-  if (nq <= 0) return true;
-  if constexpr (4 * kSmAll <= kSmMax) {{
-    auto k = hess_block_kernel<{la}, {lb}, {lc}, {ld}, HessBlockTab{t}, false, 32>;
-    if (4 * kSmAll > 48 * 1024) cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)(4 * kSmAll));
-    k<<<(nq + 3) / 4, 128, 4 * kSmAll, s>>>(a, o, pure, q, nq);
-    return true;
-  }} else {{
-    return false;
-  }}
-}}
 {line_fn}
 extern const HessLaunchers hess_launchers_{t};
 const HessLaunchers hess_launchers_{t} = {{{la}, {lb}, {lc}, {ld}, &launch_hess, &hess_scratch_slots,
-                                          &launch_hess_block, &hess_block_global_slots, &launch_hess_warp,
                                           {has_line}, &launch_hess_line}};
 }}  // namespace hfgpu
 """
@@ -1145,9 +1038,59 @@ static bool launch_hess_line(const GradArgs<double>&, const HessOut&, int, const
 }"""
 
 
+RYS_INST_TEMPLATE = """// GENERATED by gen_eri.py -- do not edit.
+#include "../hfgpu_rys.cuh"
+#include "../hfgpu_rys_launch.h"
+
+namespace hfgpu {{
+extern const RysLaunchers rys_launchers_{t};
+const RysLaunchers rys_launchers_{t} = {{
+    {la}, {lb}, {lc}, {ld}, {{{g0}, {g1}, {g2}}}, {gv}, {hv},
+    {{&launch_rys<{c}, 1, double, {g0}>, &launch_rys<{c}, 1, double, {g1}>, &launch_rys<{c}, 1, double, {g2}>}},
+    {{&launch_rys<{c}, 1, float, {g0}>, &launch_rys<{c}, 1, float, {g1}>, &launch_rys<{c}, 1, float, {g2}>}},
+    {{&launch_rys<{c}, 2, double, {g0}>, &launch_rys<{c}, 2, double, {g1}>, &launch_rys<{c}, 2, double, {g2}>}}}};
+}}  // namespace hfgpu
+"""
+
+
+def rys_groups(la, lb, lc, ld):
+    """Threads per quartet of the three variants of a class's Rys kernels, by its Cartesian block."""
+    n = ncart(la) * ncart(lb) * ncart(lc) * ncart(ld)
+    if n <= 1:
+        return (2, 4, 8)
+    if n <= 10:
+        return (4, 8, 16)
+    if n <= 36:
+        return (8, 16, 32)
+    if n <= 108:
+        return (16, 32, 64)
+    return (32, 64, 128)
+
+
+# Default forms of the derivative classes, by their Cartesian block, measured per class on n-octane,
+# anthracene and water clusters (device time of the class alone; thread form / Rys quadrature):
+# gradient: the op-table classes take Rys quadrature ((dp|dp) 1.25 / 0.36 ms on octane, (dd|dp) 1.03 /
+# 0.17, (dd|dd) 0.41 / 0.03, against one block per quartet over the op tables); the straight-line
+# ones keep one thread per quartet ((pp|ps) 1.5 / 4.3; (dp|pp) 1.86 / 1.39 on octane but 7.4 / 12.1 on
+# anthracene with its longer contractions).
+# Hessian: Rys quadrature everywhere ((pp|ps) 35 / 12 ms, (dp|dp) 21 / 1.0, (dd|dd) 2.8 / 0.06) but for
+# (ss|ss), (ps|ss) and (ds|ss) (3.3 / 4.9, 8.1 / 14, 4.5 / 5.0).
+RYS_HESS_LINE = ((0, 0, 0, 0), (1, 0, 0, 0), (2, 0, 0, 0))
+
+
+def rys_defaults(c):
+    """(gradient, Hessian) default variant of class c, -1 = the straight-line form."""
+    n = ncart(c[0]) * ncart(c[1]) * ncart(c[2]) * ncart(c[3])
+    grad = -1 if n < 216 else (2 if n == 1296 else 0)
+    hess = -1 if c in RYS_HESS_LINE else (1 if n in (1, 1296) or c in ((2, 1, 0, 0),) else 0)
+    return grad, hess
+
+
 def main(outdir):
     import os
+    import gen_rys
     os.makedirs(outdir, exist_ok=True)
+    gen_rys.emit(outdir)
     pairs, cls = classes()
     meta = {"pair_classes": pairs, "eri": [], "grad": []}
 
@@ -1175,13 +1118,11 @@ def main(outdir):
         t = "".join(map(str, c))
         code_h, mh = gen_hess_table(*c)
         meta["hess"].append(mh)
-        code_b, mb = gen_hess_block(*c)
-        mh["block"] = mb
         code_l, ml = gen_hess_line(*c)
         mh["line"] = ml
         write_if_changed(os.path.join(outdir, f"hess_{t}.cuh"),
                          "// GENERATED by gen_eri.py -- do not edit.\n#pragma once\n#include \"common.cuh\"\n\n" +
-                         code_h + "\n\n" + code_b + "\n" + ("\n" + code_l + "\n" if code_l else ""))
+                         code_h + "\n" + ("\n" + code_l + "\n" if code_l else ""))
         la, lb, lc, ld = c
         line = code_l is not None
         write_if_changed(os.path.join(outdir, f"hess_{t}.cu"), HESS_INST_TEMPLATE.format(
@@ -1190,6 +1131,16 @@ def main(outdir):
             line_fn=(HESS_LINE_LAUNCH.format(t=t, la=la, lb=lb, lc=lc, ld=ld) if line else HESS_LINE_NONE),
             has_line="true" if line else "false"))
         hnames.append(t)
+        g = rys_groups(*c)
+        write_if_changed(os.path.join(outdir, f"rys_{t}.cu"), RYS_INST_TEMPLATE.format(
+            t=t, la=la, lb=lb, lc=lc, ld=ld, c=f"{la}, {lb}, {lc}, {ld}", g0=g[0], g1=g[1], g2=g[2],
+            gv=rys_defaults(c)[0], hv=rys_defaults(c)[1]))
+    rd = ["// GENERATED by gen_eri.py -- do not edit.", '#include "../hfgpu_rys_launch.h"', "namespace hfgpu {"]
+    rd += [f"extern const RysLaunchers rys_launchers_{t};" for t in hnames]
+    rd.append(f"const RysLaunchers* const kRysLaunchers[{len(hnames)}] = {{")
+    rd += [f"  &rys_launchers_{t}," for t in hnames]
+    rd += ["};", "}  // namespace hfgpu"]
+    write_if_changed(os.path.join(outdir, "rys_dispatch.cu"), "\n".join(rd) + "\n")
     hd = ["// GENERATED by gen_eri.py -- do not edit.", '#include "../hfgpu_hess_launch.h"', "namespace hfgpu {"]
     hd += [f"extern const HessLaunchers hess_launchers_{t};" for t in hnames]
     hd.append(f"const HessLaunchers* const kHessLaunchers[{len(hnames)}] = {{")
@@ -1575,143 +1526,6 @@ def _alloc_levels_with_readers(order_by_level, deps_of, lev, pre_slots, live_to_
     return slot, top
 
 
-def gen_grad_warp(la, lb, lc, ld, sets=("U", "A", "B", "C"), suffix=""):
-    """Adjoint gradient of one quartet by one warp: the VRR one order higher and the HRR of
-    the weighted sets are levelised (an op's inputs come from earlier levels), so the
-    32 lanes run one level's ops in parallel out of shared memory; the contractions with
-    the weight block W are ops of the HRR levels that only read.  `sets` restricts the table to
-    some of the four accumulator sets (one pass of the per-set split: the terms that read those
-    sets only, so the four one-set tables add up to the whole gradient)."""
-    L = la + lb + lc + ld + 1
-    order = grad_sets(la, lb, lc, ld)
-    dag = Dag(L)
-    setoff, nacc = {}, 0
-    for k in sets:
-        setoff[k] = nacc
-        nacc += len(order[k])
-    acc_src, acc_set = [], []
-    for k in sets:
-        for (e, f) in order[k]:
-            acc_src.append(dag.get(e, f, 0))
-            acc_set.append(("U", "A", "B", "C").index(k))
-    ops = [(nid, nd) for nid, nd in enumerate(dag.nodes) if nd[0] != "F"]
-    deps = {nid: [x for x in nd[2:7] if x >= 0] for nid, nd in ops}
-    lev = _levelise([(nid, deps[nid]) for nid, _ in ops], L + 1)
-    vorder = sorted([nid for nid, _ in ops], key=lambda n: (lev[n], n))
-    pre = {m: m for m in range(L + 1)}
-    slot, nvs = _alloc_levels(vorder, deps, lev, pre, set(acc_src))
-    ZV = nvs
-    nodes = dict(ops)
-    vrows, vlev, cur = [], [0], 1
-    for nid in vorder:
-        while lev[nid] > cur:
-            vlev.append(len(vrows))
-            cur += 1
-        kind, i, a, b, c, d, g, k1, k2 = nodes[nid]
-        s_ = lambda x: slot[x] if x >= 0 else ZV
-        vrows.append(((1 if kind == "K" else 0) | (i << 2), slot[nid], s_(a), s_(b), s_(c), s_(d), s_(g),
-                      k1 | (k2 << 8)))
-    vlev.append(len(vrows))
-    # HRR of the four sets (accumulator j is value j) and the contractions
-    hnodes, hinfo, hdeps = {}, {}, {}
-    counter = [nacc]
-
-    def new_id():
-        counter[0] += 1
-        return counter[0] - 1
-
-    def ket(k, e, c, d):
-        key = ("k", k, e, c, d)
-        if key in hnodes:
-            return hnodes[key]
-        if sum(d) == 0:
-            v = setoff[k] + order[k].index((e, c))
-        else:
-            i = max(range(3), key=lambda q: (d[q], -q))
-            d1 = add(d, i, -1)
-            x, y = ket(k, e, add(c, i), d1), ket(k, e, c, d1)
-            v = new_id()
-            hinfo[v], hdeps[v] = (1, i, x, y), [x, y]
-        hnodes[key] = v
-        return v
-
-    def bra(k, a, b, c, d):
-        key = ("b", k, a, b, c, d)
-        if key in hnodes:
-            return hnodes[key]
-        if sum(b) == 0:
-            v = ket(k, a, c, d)
-        else:
-            i = max(range(3), key=lambda q: (b[q], -q))
-            b1 = add(b, i, -1)
-            x, y = bra(k, add(a, i), b1, c, d), bra(k, a, b1, c, d)
-            v = new_id()
-            hinfo[v], hdeps[v] = (0, i, x, y), [x, y]
-        hnodes[key] = v
-        return v
-
-    cops = []
-    for (cen, dr), items in grad_terms(la, lb, lc, ld).items():
-        gi = "ABC".index(cen) * 3 + dr
-        for wi, terms in items:
-            x = bra(terms[0][1], *terms[0][2:]) if terms[0][1] in sets else -1
-            if len(terms) > 1 and "U" in sets:
-                y, kk = bra("U", *terms[1][2:]), -terms[1][0]
-            else:
-                y, kk = -1, 0
-            if x < 0 and y < 0:
-                continue
-            cops.append((gi, wi, x, y, kk))
-    hord = sorted(hinfo)
-    hlev = _levelise([(v, hdeps[v]) for v in hord], nacc)
-    clev = [1 + max(hlev[x] if x >= 0 else 0, hlev[y] if y >= 0 else 0) for (_, _, x, y, _) in cops]
-    readers = [(l, ([x] if x >= 0 else []) + ([y] if y >= 0 else [])) for l, (_, _, x, y, _) in zip(clev, cops)]
-    hpre = {j: j for j in range(nacc)}
-    hslot, nhs = _alloc_levels_with_readers(sorted(hord, key=lambda v: (hlev[v], v)), hdeps, hlev, hpre, set(),
-                                            readers)
-    ZH = nhs
-    items = [(hlev[v], 0, v) for v in hord] + [(l, 1, j) for j, l in enumerate(clev)]
-    items.sort()
-    hrows, hlv, cur = [], [0], 1
-    for l, is_c, v in items:
-        while l > cur:
-            hlv.append(len(hrows))
-            cur += 1
-        if is_c:
-            gi, wi, x, y, kk = cops[v]
-            hrows.append((2 | (gi << 2) | (kk << 6), wi, hslot[x] if x >= 0 else ZH, hslot[y] if y >= 0 else ZH))
-        else:
-            kind, i, x, y = hinfo[v]
-            hrows.append((kind | (i << 2), hslot[v], hslot[x], hslot[y]))
-    hlv.append(len(hrows))
-    t = f"{la}{lb}{lc}{ld}{suffix}"
-    ncart_blk = ncart(la) * ncart(lb) * ncart(lc) * ncart(ld)
-    s = [f"// warp-mode adjoint gradient of class {t}: {len(vrows)} VRR ops in {len(vlev) - 1} levels over "
-         f"{nvs} slots, {nacc} accumulators, {len(hrows)} HRR/contraction ops in {len(hlv) - 1} levels over "
-         f"{nhs} slots"]
-    s.append(f"__device__ const int4 gwv_{t}[{max(len(vrows), 1)}] = {{")
-    s += ["  {" + ",".join(map(str, pack_warp_vrr(r))) + "}," for r in vrows]
-    s.append("};")
-    s.append(f"__device__ const int gwv_lv_{t}[{len(vlev)}] = {{{','.join(map(str, vlev))}}};")
-    s.append(f"__device__ const int2 gwa_{t}[{nacc}] = {{" +
-             ",".join("{%d,%d}" % (slot[n], k) for n, k in zip(acc_src, acc_set)) + "};")
-    s.append(f"__device__ const int2 gwh_{t}[{max(len(hrows), 1)}] = {{")
-    s += ["  {" + ",".join(map(str, pack_warp_hrr(r))) + "}," for r in hrows]
-    s.append("};")
-    s.append(f"__device__ const int gwh_lv_{t}[{len(hlv)}] = {{{','.join(map(str, hlv))}}};")
-    s.append(f"struct GradWarpTab{t} {{ static constexpr int L = {L}, NVLEV = {len(vlev) - 1}, NVSLOT = {nvs}, "
-             f"NACC = {nacc}, NHLEV = {len(hlv) - 1}, NHSLOT = {nhs}, NCART = {ncart_blk}; "
-             f"static __device__ const int4* vrr() {{ return gwv_{t}; }} "
-             f"static __device__ const int* vlev() {{ return gwv_lv_{t}; }} "
-             f"static __device__ const int2* acc() {{ return gwa_{t}; }} "
-             f"static __device__ const int2* hrr() {{ return gwh_{t}; }} "
-             f"static __device__ const int* hlev() {{ return gwh_lv_{t}; }} }};")
-    meta = {"class": [la, lb, lc, ld], "grad_warp": True, "vrr_ops": len(vrows), "vrr_levels": len(vlev) - 1,
-            "vrr_slots": nvs, "acc": nacc, "hrr_ops": len(hrows), "hrr_levels": len(hlv) - 1, "hrr_slots": nhs,
-            "smem_doubles_per_warp": nvs + 1 + nhs + 1 + 3 * ncart_blk}
-    return "\n".join(s), meta
-
-
 def gen_warp_class(la, lb, lc, ld):
     L = la + lb + lc + ld
     dag = Dag(L)
@@ -2010,151 +1824,6 @@ def gen_hess_table(la, lb, lc, ld):
              f"static __device__ const int2* hrr() {{ return hhrr_{t}; }} }};")
     meta = {"class": [la, lb, lc, ld], "vrr_ops": len(vrows), "vrr_slots": nvslot, "accumulators": nacc,
             "hrr_ops": len(hrows), "hrr_slots": nhslot, "terms": len(terms)}
-    return "\n".join(s), meta
-
-
-
-def pack_hess_block_hrr(r):
-    """Block-form HRR row {dst, x, y, kind | dir<<2} (kind 0 bra, 1 ket) or contraction row
-    {W index, x, 0, 2 | out<<4 | (coef + 128)<<10}: full 32-bit slot numbers (the level-wise
-    slot allocation of the large classes needs more than 2^16)."""
-    if r[0] == 2:
-        _, hi, wi, x, k = r
-        assert -128 <= k < 128 and 0 <= hi < 45
-        return (wi, x, 0, 2 | hi << 4 | (k + 128) << 10)
-    kind, i, dst, x, y = r
-    return (dst, x, y, kind | i << 2)
-
-
-def gen_hess_block(la, lb, lc, ld):
-    """Levelised op tables of the adjoint Hessian of one class for one block of threads per
-    quartet (hess_block_kernel): the VRR two orders higher and the HRR of the ten weight sets
-    are levelised (an op reads only values of earlier levels), so a level's ops run
-    thread-parallel; each HRR level ends with its contraction rows, sorted by output entry,
-    which the threads take in contiguous chunks (one register sum per run of equal entries)."""
-    L = la + lb + lc + ld + 2
-    terms = hess_terms(la, lb, lc, ld)
-    hnodes, hinfo, hdeps, acc_key = {}, {}, {}, {}
-    nxt = [0]
-
-    def new_id():
-        nxt[0] += 1
-        return ("h", nxt[0] - 1)
-
-    def ket(k, e, c, d):
-        key = ("k", k, e, c, d)
-        if key in hnodes:
-            return hnodes[key]
-        if sum(d) == 0:
-            v = ("acc", k, e, c)
-            acc_key.setdefault(v, len(acc_key))
-        else:
-            i = max(range(3), key=lambda q: (d[q], -q))
-            d1 = add(d, i, -1)
-            x, y = ket(k, e, add(c, i), d1), ket(k, e, c, d1)
-            v = new_id()
-            hinfo[v], hdeps[v] = (1, i, x, y), [x, y]
-        hnodes[key] = v
-        return v
-
-    def bra(k, a, b, c, d):
-        key = ("b", k, a, b, c, d)
-        if key in hnodes:
-            return hnodes[key]
-        if sum(b) == 0:
-            v = ket(k, a, c, d)
-        else:
-            i = max(range(3), key=lambda q: (b[q], -q))
-            b1 = add(b, i, -1)
-            x, y = bra(k, add(a, i), b1, c, d), bra(k, a, b1, c, d)
-            v = new_id()
-            hinfo[v], hdeps[v] = (0, i, x, y), [x, y]
-        hnodes[key] = v
-        return v
-
-    cops = [(hi, wi, bra(si, a, b, c, d), k) for hi, wi, k, si, a, b, c, d in terms]
-    nacc = len(acc_key)
-    # number every HRR value: accumulators 0 .. nacc-1 (the inputs), the rest after
-    num = {v: j for v, j in acc_key.items()}
-    for v in hinfo:
-        num[v] = len(num)
-    hord = [num[v] for v in hinfo]  # creation order is topological
-    hdeps_n = {num[v]: [num[x] for x in hdeps[v]] for v in hinfo}
-    hlev = _levelise([(v, hdeps_n[v]) for v in hord], nacc)
-    clev = [1 + hlev[num[x]] for (_, _, x, _) in cops]
-    readers = [(l, [num[x]]) for l, (_, _, x, _) in zip(clev, cops)]
-    hpre = {j: j for j in range(nacc)}
-    hslot, nhs = _alloc_levels_with_readers(sorted(hord, key=lambda v: (hlev[v], v)), hdeps_n, hlev, hpre, set(),
-                                            readers)
-    inv = {num[v]: v for v in hinfo}
-    maxl = max([hlev[v] for v in hord] + clev + [0])
-    hrows, hlv = [], []
-    by_l = {}
-    for v in hord:
-        by_l.setdefault(hlev[v], [[], []])[0].append(v)
-    for j, l in enumerate(clev):
-        by_l.setdefault(l, [[], []])[1].append(j)
-    for l in range(1, maxl + 1):
-        ops_l, con_l = by_l.get(l, [[], []])
-        start = len(hrows)
-        for v in ops_l:
-            kind, i, x, y = hinfo[inv[v]]
-            hrows.append((kind, i, hslot[v], hslot[num[x]], hslot[num[y]]))
-        mid = len(hrows)
-        for j in sorted(con_l, key=lambda j: (cops[j][0], cops[j][1])):
-            hi, wi, x, k = cops[j]
-            hrows.append((2, hi, wi, hslot[num[x]], k))
-        hlv.append((start, mid))
-    hlv.append((len(hrows), len(hrows)))
-    # VRR, levelised; accumulator j <- weight(set) * value at slot
-    dag = Dag(L)
-    acc_src, acc_set = [0] * nacc, [0] * nacc
-    for (_, k, e, f), j in acc_key.items():
-        acc_src[j] = dag.get(e, f, 0)
-        acc_set[j] = k
-    ops = [(nid, nd) for nid, nd in enumerate(dag.nodes) if nd[0] != "F"]
-    deps = {nid: [x for x in nd[2:7] if x >= 0] for nid, nd in ops}
-    lev = _levelise([(nid, deps[nid]) for nid, _ in ops], L + 1)
-    vorder = sorted([nid for nid, _ in ops], key=lambda n: (lev[n], n))
-    pre = {m: m for m in range(L + 1)}
-    slot, nvs = _alloc_levels(vorder, deps, lev, pre, set(acc_src))
-    ZV = nvs
-    nodes = dict(ops)
-    vrows, vlev, cur = [], [0], 1
-    for nid in vorder:
-        while lev[nid] > cur:
-            vlev.append(len(vrows))
-            cur += 1
-        kind, i, a, b, c, d, g, k1, k2 = nodes[nid]
-        s_ = lambda x: slot[x] if x >= 0 else ZV
-        vrows.append(((1 if kind == "K" else 0) | (i << 2), slot[nid], s_(a), s_(b), s_(c), s_(d), s_(g),
-                      k1 | (k2 << 8)))
-    vlev.append(len(vrows))
-    t = f"{la}{lb}{lc}{ld}"
-    ncart_blk = ncart(la) * ncart(lb) * ncart(lc) * ncart(ld)
-    s = [f"// block-mode adjoint Hessian of class {t}: {len(vrows)} VRR ops in {len(vlev) - 1} levels over "
-         f"{nvs} slots, {nacc} accumulators, {len(hrows)} HRR/contraction ops in {len(hlv) - 1} levels over "
-         f"{nhs} slots"]
-    s.append(f"__device__ const int4 hbv_{t}[{max(len(vrows), 1)}] = {{")
-    s += ["  {" + ",".join(map(str, pack_warp_vrr(r))) + "}," for r in vrows]
-    s.append("};")
-    s.append(f"__device__ const int hbv_lv_{t}[{len(vlev)}] = {{{','.join(map(str, vlev))}}};")
-    s.append(f"__device__ const int2 hba_{t}[{nacc}] = {{" +
-             ",".join("{%d,%d}" % (slot[n], k) for n, k in zip(acc_src, acc_set)) + "};")
-    s.append(f"__device__ const int4 hbh_{t}[{max(len(hrows), 1)}] = {{")
-    s += ["  {" + ",".join(map(str, pack_hess_block_hrr(r))) + "}," for r in hrows]
-    s.append("};")
-    s.append(f"__device__ const int2 hbh_lv_{t}[{len(hlv)}] = {{" + ",".join("{%d,%d}" % p for p in hlv) + "};")
-    s.append(f"struct HessBlockTab{t} {{ static constexpr int L = {L}, NVLEV = {len(vlev) - 1}, NVSLOT = {nvs}, "
-             f"NACC = {nacc}, NHLEV = {len(hlv) - 1}, NHSLOT = {nhs}, NCART = {ncart_blk}; "
-             f"static __device__ const int4* vrr() {{ return hbv_{t}; }} "
-             f"static __device__ const int* vlev() {{ return hbv_lv_{t}; }} "
-             f"static __device__ const int2* acc() {{ return hba_{t}; }} "
-             f"static __device__ const int4* hrr() {{ return hbh_{t}; }} "
-             f"static __device__ const int2* hlev() {{ return hbh_lv_{t}; }} }};")
-    meta = {"class": [la, lb, lc, ld], "vrr_ops": len(vrows), "vrr_levels": len(vlev) - 1, "vrr_slots": nvs,
-            "acc": nacc, "hrr_ops": len(hrows), "hrr_levels": len(hlv) - 1, "hrr_slots": nhs,
-            "slots": nvs + 1 + nhs + 1 + 45 + 3 * ncart_blk}
     return "\n".join(s), meta
 
 

@@ -18,6 +18,8 @@
 #include "hfgpu_launch.h"
 #include "hfgpu_hess_kernels.cuh"
 #include "hfgpu_hess_launch.h"
+#include "hfgpu_rys.cuh"
+#include "hfgpu_rys_launch.h"
 #include "hfgpu_onee.h"
 #include "hfgpu_onee_kernels.cuh"
 #include "hfgpu_batch_eigh.cuh"
@@ -165,6 +167,7 @@ struct hfgpu_handle {
   // the Boys table in the plane layout of the staged kernels, and the device status word
   DevBuf d_boys_pd, d_boys_pf, d_status, d_abort;
   DevBuf d_purify;  // workspace of hfgpu_purify_device
+  const double* rys_tab = nullptr;  // quadrature tables of the Rys kernels on this device
   cudaStream_t ctl_stream = nullptr;  // non-blocking stream of hfgpu_request_abort
   int status_host = 0;  // the status word as the last host-pointer entry point read it
   long long nquartets = 0;
@@ -192,14 +195,13 @@ struct hfgpu_handle {
   // (grad_form_of)
   int grad_form[21];
   unsigned grad_class_mask = ~0u;       // classes a gradient launches (autotuning runs one at a time)
-  // Hessian form (hfgpu_set_hess_form): -1 by class, 0 one thread per quartet, 1 one block per
-  // quartet, 2 one warp per quartet (where the class's tables fit), 3 one thread per quartet on
+  // Hessian form (hfgpu_set_hess_form): -1 by class, 0 one thread per quartet, 1 and 2 a group of
+  // threads per quartet by Rys quadrature (largest, smallest group), 3 one thread per quartet on
   // straight-line code (where the class has it)
   int hess_form = -1;
   int purify_blocks = -1;               // co-resident blocks of the cooperative purification (0: not available)
   int purify_coop = 1;                  // hfgpu_set_purify_mode: 1 one cooperative launch, 0 two launches per step
-  int hess_cls_form[21];                // per class (hfgpu_autotune_hess): 0 thread, 1 block, 2 warp, 3 line,
-                                        // -1 hess_form
+  int hess_cls_form[21];                // per class (hfgpu_autotune_hess): as hess_form; -1 hess_form
   unsigned hess_class_mask = ~0u;       // classes a Hessian launches (autotuning runs one at a time)
 
   hfgpu_handle() : q_beg(21), q_mid(21), q_end(21), q_hik1(21), q_hik2(21), q_prims(21) {
@@ -1326,27 +1328,26 @@ int grad_smem_atoms(const hfgpu_handle* h) {
   return (size_t)h->natoms * 3 * sizeof(double) <= (size_t)kGradSmemBytes ? h->natoms : 0;
 }
 
-// Gradient forms of the op-table classes: 0 one thread per quartet (global scratch), 1 one warp
-// per quartet, 2 one warp per quartet in four one-set launches, 3 one block of 128 threads per
-// quartet, 4 the same in four one-set launches, 5 and 6 the same with 256 threads.
+// Gradient forms of the op-table classes: 0 one thread per quartet (op tables on global scratch);
+// 1..6 a group of threads per quartet by Rys quadrature, 1 and 2 the smallest group size of the
+// class, 3 and 4 the middle one, 5 and 6 the largest.
 constexpr int kGradForms = 7;
-static int grad_form_threads(int form) { return form >= 5 ? 256 : (form >= 3 ? 128 : 32); }
-static bool grad_form_split(int form) { return form == 2 || form == 4 || form == 6; }
+
+// The op-table classes have a choice of forms.
+static bool grad_has_forms(int c) { return hfgpu::kClassLaunchers[c]->grad_scratch_slots(0) > 0; }
 
 // Form of a gradient launch of class c: the one hfgpu_autotune_grad or hfgpu_set_grad_forms
-// chose, else the block form (3), which was the fastest single form on every workload measured
-// (octane, anthracene, the water octamer), when the class has shared-memory tables that fit one
-// block; opts.grad_warp_max_waves <= 0 asks for the thread form instead.
-static int grad_form_of(const hfgpu_handle* h, int c, bool fp32) {
-  const hfgpu::ClassLaunchers* L = hfgpu::kClassLaunchers[c];
-  if (!L->has_grad_warp) return 0;
-  const int bytes = L->grad_warp_bytes(fp32 ? 1 : 0);
-  if (bytes <= 0 || bytes > 232448) return 0;
-  if (h->grad_form[c] >= 0) return h->grad_form[c];
-  return h->opts.grad_warp_max_waves > 0 ? 3 : 0;
+// chose, else the class's default: kGradForms + 1 + v for Rys quadrature in group size v, 0 for one
+// thread per quartet on straight-line code; opts.grad_warp_max_waves <= 0 asks for the thread form
+// of the op-table classes instead.
+static int grad_form_of(const hfgpu_handle* h, int c) {
+  const int v = hfgpu::kRysLaunchers[c]->grad_variant;
+  if (grad_has_forms(c)) {
+    if (h->grad_form[c] >= 0) return h->grad_form[c];
+    if (h->opts.grad_warp_max_waves <= 0) return 0;
+  }
+  return v >= 0 ? kGradForms + 1 + v : 0;
 }
-
-static bool grad_use_warp(const hfgpu_handle* h, int c, bool fp32) { return grad_form_of(h, c, fp32) >= 1; }
 
 // Quartets of a list range of n that this handle's partition processes (every nparts-th,
 // starting at number part).
@@ -1383,6 +1384,7 @@ static int grad_device_impl(hfgpu_handle* h, const double* DJ, double cJ, int nK
   gf.mol_off = gd.mol_off;
   gf.mol_n = gd.mol_n;
   gd.smem_atoms = gf.smem_atoms = grad_smem_atoms(h);
+  const RysOut ro{h->rys_tab, nullptr, h->natoms, gd.smem_atoms};
   gd.part = gf.part = h->part;
   gd.nparts = gf.nparts = h->nparts;
   const int2* q = h->d_quart.as<int2>();
@@ -1405,7 +1407,7 @@ static int grad_device_impl(hfgpu_handle* h, const double* DJ, double cJ, int nK
     const long long nq = h->q_end[c] - h->q_beg[c];
     slice_off[c] = slice_off_f[c] = need_total;
     if (slots <= 0 || nq <= 0) continue;
-    if (grad_use_warp(h, c, false) && grad_use_warp(h, c, true)) continue;  // warp/block form: no scratch
+    if (grad_form_of(h, c) >= 1) continue;  // no scratch
     const size_t one = (size_t)slots * sizeof(double) * (size_t)table_threads(slots, nq);
     need_total += (one + 255) / 256 * 256;
     if (precision == HFGPU_MIXED) {
@@ -1427,16 +1429,16 @@ static int grad_device_impl(hfgpu_handle* h, const double* DJ, double cJ, int nK
     auto run = [&](bool fp32, long long lo, long long hi) -> int {
       const int nq = (int)part_share(h, hi - lo);
       if (nq <= 0) return HFGPU_OK;
-      const int form = grad_form_of(h, c, fp32);
-      gd.warp_split = gf.warp_split = grad_form_split(form) ? 1 : 0;
-      gd.warp_threads = gf.warp_threads = grad_form_threads(form);
+      const int form = grad_form_of(h, c);
       if (form >= 1) {
-        const bool done = fp32 ? L->grad_warp_f(gf, h->pure, q + lo, nq, fp32 ? st_f : st_d)
-                               : L->grad_warp_d(gd, h->pure, q + lo, nq, st_d);
-        if (done) {
-          HF_CHECK_LAUNCH(h, "grad warp kernel");
-          return HFGPU_OK;
-        }
+        const hfgpu::RysLaunchers* Y = hfgpu::kRysLaunchers[c];
+        const int v = form > kGradForms ? form - kGradForms - 1 : (form - 1) / 2;
+        const int most = ro.smem_atoms > 0 ? grad_max_blocks(h) : 0;
+        if (!(fp32 ? Y->grad_f[v](gf, ro, h->pure, q + lo, nq, most, st_f)
+                   : Y->grad_d[v](gd, ro, h->pure, q + lo, nq, most, st_d)))
+          return fail(h, HFGPU_ERR_CUDA, "gradient launch: shared memory");
+        HF_CHECK_LAUNCH(h, "grad kernel");
+        return HFGPU_OK;
       }
       const size_t off = fp32 ? slice_off_f[c] : slice_off[c];
       unsigned char* slice = h->d_scratch.as<unsigned char>() + off;
@@ -1668,7 +1670,7 @@ int hfgpu_create(const hfgpu_basis* b, const hfgpu_opts* opts, hfgpu_handle** ou
       cudaMemcpy(h->d_boys_f.p, btf.data(), sizeof(float) * btf.size(), cudaMemcpyHostToDevice) ||
       cudaMemcpy(h->d_boys_pd.p, bpd.data(), sizeof(double) * bpd.size(), cudaMemcpyHostToDevice) ||
       cudaMemcpy(h->d_boys_pf.p, bpf.data(), sizeof(float) * bpf.size(), cudaMemcpyHostToDevice) ||
-      cudaMemset(h->d_status.p, 0, sizeof(int))) {
+      cudaMemset(h->d_status.p, 0, sizeof(int)) || !(h->rys_tab = hfgpu_rys_table())) {
     hfgpu_destroy(h);
     return HFGPU_ERR_CUDA;
   }
@@ -1969,10 +1971,7 @@ int hfgpu_grad2e_uhf_backward(hfgpu_handle* h, const double* Da, const double* D
 // (enough to fill the GPU for the largest tables), at most one per quartet, and loops over the rest.
 constexpr size_t kHessScratchBudget = (size_t)2 << 30;
 constexpr size_t kHessSmemBytes = 96 * 1024;  // per-block Hessian in shared memory up to 36 atoms
-constexpr int kHessBlockMinSlots = 1000;       // thread-form tables from this size run in the block form,
-constexpr long long kHessBlockMaxQuartets = 4096;  // and so do classes with at most this many quartets
 constexpr long long kHessLineGrid = 4 * 148;     // straight-line form: at most four blocks per SM, grid-stride
-constexpr long long kHessBlockGrid = 296;      // blocks of a block-form launch with global HRR slots
 
 static int hess_device_impl(hfgpu_handle* h, const double* DJ, double cJ, int nK, const double* DK, double cK,
                             double* hess) {
@@ -1993,34 +1992,22 @@ static int hess_device_impl(hfgpu_handle* h, const double* DJ, double cJ, int nK
   const size_t n3 = 3 * (size_t)h->natoms;
   const size_t smem = sizeof(double) * n3 * n3;
   HessOut o{hess, h->natoms, smem <= kHessSmemBytes ? 1 : 0};
+  RysOut ro{h->rys_tab, hess, h->natoms, 0};
   const int2* q = h->d_quart.as<int2>();
   auto threads_of = [&](int slots, long long nq) -> long long {
     long long thr = (long long)(kHessScratchBudget / ((size_t)slots * sizeof(double)));
     thr = std::min<long long>(thr, ((nq + 127) / 128) * 128);
     return std::max<long long>(128, thr / 128 * 128);
   };
-  // form per class: 0 one thread per quartet on global scratch, 1 one block of 128 threads per
-  // quartet over levelised tables, 2 one warp per quartet over the same tables, 3 one thread per
-  // quartet on straight-line register code (the classes that have it; a class without it takes
-  // the default).  Default: the straight-line form where the class has one; else the block form
-  // for the classes whose tables are large or whose quartets are too few to fill the GPU (one
-  // thread would run a long chain of dependent table ops on global scratch), the warp form for
-  // the small many-quartet classes (their levels hold a few dozen ops).
+  // form per class: 0 one thread per quartet on global scratch, 1 and 2 a group of threads per quartet
+  // by Rys quadrature (1 the largest group of the class, 2 the smallest), 3 one thread per quartet on
+  // straight-line register code (the classes that have it; a class without it takes the default).
+  // Default: Rys quadrature with the class's measured group size, or the straight-line form
+  // (rys_defaults in gen_eri.py).
   auto form_of = [&](int c) -> int {
-    const bool line = hfgpu::kHessLaunchers[c]->has_line;
     int f = h->hess_cls_form[c] >= 0 ? h->hess_cls_form[c] : h->hess_form;
-    if (f == 3 && !line) f = -1;
-    if (f >= 0) return f;
-    if (line) return 3;
-    const bool big = hfgpu::kHessLaunchers[c]->scratch_slots(h->pure) >= kHessBlockMinSlots ||
-                     part_share(h, h->q_end[c] - h->q_beg[c]) <= kHessBlockMaxQuartets;
-    return big ? 1 : 2;
-  };
-  auto use_block = [&](int c) -> bool { return form_of(c) == 1 || form_of(c) == 2; };
-  // block-form grid: one block per quartet, or kHessBlockGrid blocks when the HRR slots live in
-  // global scratch (one region per block)
-  auto block_grid = [&](int c, long long nq) -> long long {
-    return hfgpu::kHessLaunchers[c]->block_global_slots() > 0 ? std::min<long long>(nq, kHessBlockGrid) : nq;
+    if (f == 3 && !hfgpu::kHessLaunchers[c]->has_line) f = -1;
+    return f < 0 && hfgpu::kRysLaunchers[c]->hess_variant < 0 ? 3 : f;
   };
   // classes largest first, round-robin over the auxiliary streams; each stream's slice is the
   // largest need of its classes
@@ -2037,12 +2024,8 @@ static int hess_device_impl(hfgpu_handle* h, const double* DJ, double cJ, int nK
     const long long nq = part_share(h, h->q_end[c] - h->q_beg[c]);
     if (nq <= 0 || !((h->hess_class_mask >> c) & 1u)) continue;
     stream_of[c] = rr++ % kS;
-    size_t bytes;
-    if (form_of(c) == 3) {
-      bytes = 0;
-    } else if (use_block(c)) {
-      bytes = sizeof(double) * (size_t)L->block_global_slots() * (size_t)block_grid(c, nq);
-    } else {
+    size_t bytes = 0;
+    if (form_of(c) == 0) {
       const int slots = L->scratch_slots(h->pure);
       bytes = (size_t)slots * sizeof(double) * (size_t)threads_of(slots, nq);
     }
@@ -2067,23 +2050,13 @@ static int hess_device_impl(hfgpu_handle* h, const double* DJ, double cJ, int nK
       HF_CHECK_LAUNCH(h, "hess line kernel");
       continue;
     }
-    if (use_block(c)) {
-      const int st = stream_of[c];
-      const long long grid = block_grid(c, nq);
-      if (sizeof(double) * (size_t)L->block_global_slots() * (size_t)grid > slice[st] ||
-          off[st] + slice[st] > h->d_scratch.bytes)
-        return fail(h, HFGPU_ERR_NOMEM, "Hessian scratch too small");
-      gd.scratch = reinterpret_cast<double*>(h->d_scratch.as<unsigned char>() + off[st]);
-      gd.scratch_threads = 0;
-      if (form_of(c) == 2 && L->launch_warp(gd, o, h->pure, q + h->q_beg[c], (int)nq, h->aux[st])) {
-        HF_CHECK_LAUNCH(h, "hess warp kernel");
-        continue;
-      }
-      if (L->launch_block(gd, o, h->pure, q + h->q_beg[c], (int)nq, (int)grid, h->aux[st])) {
-        HF_CHECK_LAUNCH(h, "hess block kernel");
-        continue;
-      }
-      if (h->hess_form >= 1) return fail(h, HFGPU_ERR_UNSUPPORTED, "class without a Hessian block form");
+    if (form_of(c) != 0) {
+      const hfgpu::RysLaunchers* Y = hfgpu::kRysLaunchers[c];
+      const int v = form_of(c) == 1 ? hfgpu::kRysVariants - 1 : (form_of(c) == 2 ? 0 : Y->hess_variant);
+      if (!Y->hess[v](gd, ro, h->pure, q + h->q_beg[c], (int)nq, 0, h->aux[stream_of[c]]))
+        return fail(h, HFGPU_ERR_CUDA, "Hessian launch: shared memory");
+      HF_CHECK_LAUNCH(h, "hess kernel");
+      continue;
     }
     const int slots = L->scratch_slots(h->pure);
     const long long thr = threads_of(slots, nq);
@@ -2609,13 +2582,13 @@ int hfgpu_set_grad_forms(hfgpu_handle* h, const int* forms) {
   for (int c = 0; c < hfgpu::kNumClasses; ++c)
     if (forms[c] < -1 || forms[c] > kGradForms - 1) return fail(h, HFGPU_ERR_INVALID, "gradient form out of range");
   for (int c = 0; c < hfgpu::kNumClasses; ++c)
-    h->grad_form[c] = hfgpu::kClassLaunchers[c]->has_grad_warp ? forms[c] : -1;
+    h->grad_form[c] = grad_has_forms(c) ? forms[c] : -1;
   return HFGPU_OK;
 }
 
-// Hessian form per class: each class alone, one thread (global scratch), one block or one warp
-// per quartet, or one thread on straight-line code where the class has it, on RHF weights of the
-// device density D; the fastest is kept.
+// Hessian form per class: each class alone, one thread (global scratch), Rys quadrature with the
+// largest or the smallest group of threads per quartet, or one thread on straight-line code where the
+// class has it, on RHF weights of the device density D; the fastest is kept.
 int hfgpu_autotune_hess(hfgpu_handle* h, const double* D, int repeats, int* forms) {
   if (!h || !D) return HFGPU_ERR_INVALID;
   DeviceGuard dev_guard(h);
@@ -2706,12 +2679,12 @@ int hfgpu_autotune_grad(hfgpu_handle* h, const double* D, int precision, int rep
   // RHF weights (cJ = 2, cK = 1) on the given density, one class at a time, each form timed
   for (int c = 0; c < hfgpu::kNumClasses; ++c) {
     const hfgpu::ClassLaunchers* L = hfgpu::kClassLaunchers[c];
-    if (!L->has_grad_warp || h->q_end[c] <= h->q_beg[c]) continue;
+    if (!grad_has_forms(c) || h->q_end[c] <= h->q_beg[c]) continue;
     h->grad_class_mask = 1u << c;
     float best = 1e30f;
     int best_form = 0;
-    // thread, warp, warp split into four one-set passes, block of four or eight warps (whole, split)
-    for (int form = 0; form < kGradForms; ++form) {
+    // one thread per quartet, then the three group sizes (2, 4 and 6 run what 1, 3 and 5 run)
+    for (int form = 0; form < kGradForms; form += form ? 2 : 1) {
       h->grad_form[c] = form;
       float ms = 0.f;
       if ((rc = tuner_time(h, gradient, repeats, e0, e1, restore.flush, &ms))) return rc;
@@ -2734,7 +2707,7 @@ int hfgpu_autotune_grad(hfgpu_handle* h, const double* D, int precision, int rep
   for (int c = 0; c < hfgpu::kNumClasses; ++c) {
     if (h->grad_form[c] < 0) continue;
     const int keep = h->grad_form[c];
-    for (int form = 0; form < kGradForms; ++form) {
+    for (int form = 0; form < kGradForms; form += form ? 2 : 1) {
       if (form == keep) continue;
       const int before = h->grad_form[c];
       h->grad_form[c] = form;

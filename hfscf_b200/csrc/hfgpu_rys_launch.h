@@ -1,0 +1,33 @@
+// Host-visible launchers of the Rys-quadrature derivative kernels (one translation unit per class,
+// generated by gen_eri.py).
+#pragma once
+#include <cuda_runtime.h>
+
+template <typename R>
+struct GradArgs;
+struct RysOut;
+
+namespace hfgpu {
+
+constexpr int kRysVariants = 3;  // threads per quartet: fewest, middle, most
+
+struct RysLaunchers {
+  int la, lb, lc, ld;
+  int group[kRysVariants];  // threads per quartet of each variant
+  int grad_variant, hess_variant;  // default variants (grad_variant -1: straight-line code instead)
+  // quartets q[0, nq) on at most max_blocks blocks (0: no limit); false when the launch's shared
+  // memory could not be had
+  bool (*grad_d[kRysVariants])(const GradArgs<double>&, const RysOut&, int pure, const int2* q, int nq, int max_blocks,
+                               cudaStream_t);
+  bool (*grad_f[kRysVariants])(const GradArgs<float>&, const RysOut&, int pure, const int2* q, int nq, int max_blocks,
+                               cudaStream_t);
+  bool (*hess[kRysVariants])(const GradArgs<double>&, const RysOut&, int pure, const int2* q, int nq, int max_blocks,
+                             cudaStream_t);
+};
+
+extern const RysLaunchers* const kRysLaunchers[];
+
+}  // namespace hfgpu
+
+// Device address of the quadrature tables on the current device (nullptr on failure).
+const double* hfgpu_rys_table();

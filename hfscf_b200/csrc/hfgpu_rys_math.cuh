@@ -1,0 +1,244 @@
+// Arithmetic of the Rys-quadrature kernels (hfgpu_rys.cuh): quadrature values, the recurrences of
+// the two-dimensional integrals, their derivative variants and the contraction of one integral.
+// No CUDA headers, so that a host test can compile it with stand-ins for the qualifiers.
+#pragma once
+#include <type_traits>
+
+#include "generated/rys_layout.cuh"
+
+// Value v of the n-point rule at T: squared root v (v < n) or weight v - n.
+template <int N>
+__device__ __forceinline__ double rys_value(const double* __restrict__ tab, double T, int v) {
+  if (T < rys_tmax(N)) {
+    const int k = (int)(T * kRysInvH);
+    const double d = T - (k + 0.5) * kRysH;
+    const double2* c = reinterpret_cast<const double2*>(tab + rys_offset(N) + (size_t)(k * 2 * N + v) * kRysCoef);
+    double2 q[kRysCoef / 2];
+#pragma unroll
+    for (int j = 0; j < kRysCoef / 2; ++j) q[j] = __ldg(c + j);
+    double f = q[kRysCoef / 2 - 1].y;
+#pragma unroll
+    for (int j = kRysCoef / 2 - 1; j >= 0; --j) {
+      if (j < kRysCoef / 2 - 1) f = q[j].y + f * d;
+      f = q[j].x + f * d;
+    }
+    return f;
+  }
+  const double s = rsqrt(T);
+  return v < N ? c_rys_herm[N - 1][0][v] * s * s : c_rys_herm[N - 1][1][v - N] * s;
+}
+
+// Exponents of x, y, z in component c of a shell of momentum l (order of gen_eri.py cart()).
+__device__ __forceinline__ int3 rys_comp(int l, int c) {
+  const int i = c >= 3 ? 2 : (c >= 1 ? 1 : 0);
+  const int j = c - i * (i + 1) / 2;
+  return make_int3(l - i, i - j, j);
+}
+
+// Sizes of class (LA LB|LC LD) at derivative order ORD, and the layout of one group's shared memory
+// (values of type R): [roots and weights | 2-D integrals of every root | bra variants of one root |
+// variant tables of one root | W]; the first part doubles as the scratch of the weights' pure ->
+// Cartesian transform.
+template <int LA, int LB, int LC, int LD, int ORD>
+struct RysDims {
+  static constexpr int NR = (LA + LB + LC + LD + ORD) / 2 + 1;
+  static constexpr int E = LA + LB + ORD, F = LC + LD + ORD;  // highest bra and ket orders
+  static constexpr int NB = (LA + 1) * (LB + 1), NK = (LC + 1) * (LD + 1), NX = NB * NK;
+  static constexpr int NBV = ORD == 2 ? 6 : 3;   // bra variants: 1, A, B, (AA, BB, AB)
+  static constexpr int NV = ORD == 2 ? 10 : 4;   // all variants, see rys_ket
+  static constexpr int NOUT = ORD == 2 ? 45 : 9;
+  static constexpr int CB = ncart_of(LB), CC = ncart_of(LC), CD = ncart_of(LD);
+  static constexpr int NCART = ncart_of(LA) * CB * CC * CD;
+  static constexpr int kRW = 2 * NR;
+  static constexpr int kG2 = NR * 3 * (E + 1) * (F + 1);
+  static constexpr int kBV = 3 * NBV * NB * (F + 1);
+  static constexpr int kVT = NV * 3 * NX;
+  static constexpr int kMain = kRW + kG2 + kBV + kVT;
+  static constexpr int kWork = kMain > 2 * NCART ? kMain : 2 * NCART;
+  static constexpr int kGroup = kWork + NCART + (ORD == 2 ? 46 : 0);
+};
+
+// The packed 2-D table positions (x | y << 8 | z << 16) of Cartesian integral e of a class: ket tuple
+// times NB plus bra tuple.
+template <int LA, int LB, int LC, int LD>
+__device__ __forceinline__ int rys_index(int e) {
+  constexpr int CB = ncart_of(LB), CC = ncart_of(LC), CD = ncart_of(LD), NB = (LA + 1) * (LB + 1);
+  const int3 a = rys_comp(LA, e / (CB * CC * CD)), b = rys_comp(LB, e / (CC * CD) % CB);
+  const int3 c = rys_comp(LC, e / CD % CC), d = rys_comp(LD, e % CD);
+  auto at = [](int i, int j, int k, int l) { return (k * (LD + 1) + l) * NB + i * (LB + 1) + j; };
+  return at(a.x, b.x, c.x, d.x) | at(a.y, b.y, c.y, d.y) << 8 | at(a.z, b.z, c.z, d.z) << 16;
+}
+
+// Vertical recurrence of the 2-D integrals of one root and direction: g[e (F+1) + f].
+template <int E, int F, typename R>
+__device__ __forceinline__ void rys_vrr(R i00, R C, R Cp, R B00, R B10, R B01, R* __restrict__ g) {
+  R prev2[E + 1], prev[E + 1], cur[E + 1];
+  cur[0] = i00;
+#pragma unroll
+  for (int e = 1; e <= E; ++e) cur[e] = C * cur[e - 1] + (e > 1 ? R(e - 1) * B10 * cur[e - 2] : R(0));
+#pragma unroll
+  for (int e = 0; e <= E; ++e) g[e * (F + 1)] = cur[e];
+#pragma unroll
+  for (int f = 1; f <= F; ++f) {
+#pragma unroll
+    for (int e = 0; e <= E; ++e) {
+      prev2[e] = f > 1 ? prev[e] : R(0);
+      prev[e] = cur[e];
+    }
+#pragma unroll
+    for (int e = 0; e <= E; ++e) {
+      R v = Cp * prev[e];
+      if (f > 1) v += R(f - 1) * B01 * prev2[e];
+      if (e > 0) v += R(e) * B00 * prev[e - 1];
+      cur[e] = v;
+      g[e * (F + 1) + f] = v;
+    }
+  }
+}
+
+// Horizontal transfer of one index pair: h[i][j], i <= I, j <= J, i + j <= N, from h[i][0] = s[i].
+template <int N, int I, int J, typename R>
+__device__ __forceinline__ void rys_hrr(const R (&s)[N + 1], R d, R (&h)[N + 1][J + 1]) {
+#pragma unroll
+  for (int i = 0; i <= N; ++i) h[i][0] = s[i];
+#pragma unroll
+  for (int j = 1; j <= J; ++j)
+#pragma unroll
+    for (int i = 0; i <= N; ++i)
+      if (i + j <= N) h[i][j] = h[i + 1][j - 1] + d * h[i][j - 1];
+}
+
+// Bra variants of one (direction, f): bv[(v NB + ij) (F+1)], from the column g[e (F+1)].
+template <int LA, int LB, int ORD, int F, typename R>
+__device__ __forceinline__ void rys_bra(const R* __restrict__ g, R AB, R wa, R wb, R* __restrict__ bv) {
+  constexpr int E = LA + LB + ORD, J = LB + ORD, NB = (LA + 1) * (LB + 1);
+  R s[E + 1], h[E + 1][J + 1];
+#pragma unroll
+  for (int e = 0; e <= E; ++e) s[e] = g[e * (F + 1)];
+  rys_hrr<E, E, J>(s, AB, h);
+#pragma unroll
+  for (int i = 0; i <= LA; ++i)
+#pragma unroll
+    for (int j = 0; j <= LB; ++j) {
+      const int at = (i * (LB + 1) + j) * (F + 1);
+      auto put = [&](int v, R x) { bv[v * NB * (F + 1) + at] = x; };
+      put(0, h[i][j]);
+      R A = wa * h[i + 1][j], B = wb * h[i][j + 1];
+      if (i > 0) A -= R(i) * h[i - 1][j];
+      if (j > 0) B -= R(j) * h[i][j - 1];
+      put(1, A);
+      put(2, B);
+      if constexpr (ORD == 2) {
+        R AA = wa * (wa * h[i + 2][j] - R(2 * i + 1) * h[i][j]);
+        if (i > 1) AA += R(i * (i - 1)) * h[i - 2][j];
+        R BB = wb * (wb * h[i][j + 2] - R(2 * j + 1) * h[i][j]);
+        if (j > 1) BB += R(j * (j - 1)) * h[i][j - 2];
+        R x = wb * h[i + 1][j + 1];  // B of (i+1, j), then of (i-1, j)
+        if (j > 0) x -= R(j) * h[i + 1][j - 1];
+        R AB2 = wa * x;
+        if (i > 0) {
+          R y = wb * h[i - 1][j + 1];
+          if (j > 0) y -= R(j) * h[i - 1][j - 1];
+          AB2 -= R(i) * y;
+        }
+        put(3, AA);
+        put(4, BB);
+        put(5, AB2);
+      }
+    }
+}
+
+// Ket transfer and C derivatives of one (direction, bra tuple): variant v of ket tuple kl into
+// vt[v VS + kl NB].  Variants: 0 1, 1 A, 2 B, 3 C; second order 4 AA, 5 BB, 6 CC, 7 AB, 8 AC, 9 BC.
+template <int LC, int LD, int ORD, int NB, int VS, typename R>
+__device__ __forceinline__ void rys_ket(const R* __restrict__ bv, R CD, R wc, R* __restrict__ vt) {
+  constexpr int F = LC + LD + ORD;
+  auto transfer = [&](auto cord, int v, auto out) {
+    constexpr int CO = decltype(cord)::value;  // C derivatives this bra variant still takes
+    constexpr int N = LC + LD + CO;
+    R s[N + 1], h[N + 1][LD + 1];
+#pragma unroll
+    for (int f = 0; f <= N; ++f) s[f] = bv[v * NB * (F + 1) + f];
+    rys_hrr<N, N, LD>(s, CD, h);
+#pragma unroll
+    for (int k = 0; k <= LC; ++k)
+#pragma unroll
+      for (int l = 0; l <= LD; ++l) {
+        R* o = vt + (k * (LD + 1) + l) * NB;
+        o[out[0] * VS] = h[k][l];
+        if constexpr (CO >= 1) {
+          R c = wc * h[k + 1][l];
+          if (k > 0) c -= R(k) * h[k - 1][l];
+          o[out[1] * VS] = c;
+        }
+        if constexpr (CO >= 2) {
+          R c = wc * (wc * h[k + 2][l] - R(2 * k + 1) * h[k][l]);
+          if (k > 1) c += R(k * (k - 1)) * h[k - 2][l];
+          o[out[2] * VS] = c;
+        }
+      }
+  };
+  struct Out {
+    int i[3];
+    __device__ constexpr int operator[](int k) const { return i[k]; }
+  };
+  if constexpr (ORD == 2) {
+    transfer(std::integral_constant<int, 2>{}, 0, Out{{0, 3, 6}});
+    transfer(std::integral_constant<int, 1>{}, 1, Out{{1, 8, 0}});
+    transfer(std::integral_constant<int, 1>{}, 2, Out{{2, 9, 0}});
+    transfer(std::integral_constant<int, 0>{}, 3, Out{{4, 0, 0}});
+    transfer(std::integral_constant<int, 0>{}, 4, Out{{5, 0, 0}});
+    transfer(std::integral_constant<int, 0>{}, 5, Out{{7, 0, 0}});
+  } else {
+    transfer(std::integral_constant<int, 1>{}, 0, Out{{0, 3, 0}});
+    transfer(std::integral_constant<int, 0>{}, 1, Out{{1, 0, 0}});
+    transfer(std::integral_constant<int, 0>{}, 2, Out{{2, 0, 0}});
+  }
+}
+
+// Position of second derivative (P, Q) of one direction among the variants, P <= Q in A, B, C.
+__host__ __device__ constexpr int rys_second(int P, int Q) {
+  return P == Q ? 4 + P : 6 + P + Q;  // AB 7, AC 8, BC 9
+}
+// Position of (r, s), r <= s, in the 45-entry upper triangle of the 9 x 9 block (as hess_tri).
+__host__ __device__ constexpr int rys_tri(int r, int s) { return r * 9 - r * (r - 1) / 2 + (s - r); }
+
+// One integral's contribution to the sums: X, Y, Z its variants in the three directions.
+template <int ORD, typename R, int NV, int NOUT>
+__device__ __forceinline__ void rys_accumulate(R w, const R (&X)[NV], const R (&Y)[NV], const R (&Z)[NV],
+                                               R (&acc)[NOUT]) {
+  const R wx = w * X[0], wz = w * Z[0];
+  const R yz = Y[0] * wz, xz = X[0] * wz, xy = wx * Y[0];
+  if constexpr (ORD == 1) {
+#pragma unroll
+    for (int P = 0; P < 3; ++P) {
+      acc[3 * P + 0] += X[1 + P] * yz;
+      acc[3 * P + 1] += Y[1 + P] * xz;
+      acc[3 * P + 2] += Z[1 + P] * xy;
+    }
+  } else {
+    const R wy = w * Y[0];
+#pragma unroll
+    for (int P = 0; P < 3; ++P)
+#pragma unroll
+      for (int Q = P; Q < 3; ++Q) {
+        const int v = rys_second(P, Q);
+        acc[rys_tri(3 * P + 0, 3 * Q + 0)] += X[v] * yz;
+        acc[rys_tri(3 * P + 1, 3 * Q + 1)] += Y[v] * xz;
+        acc[rys_tri(3 * P + 2, 3 * Q + 2)] += Z[v] * xy;
+      }
+#pragma unroll
+    for (int P = 0; P < 3; ++P) {
+      const R xp = X[1 + P] * wz, xq = X[1 + P] * wy, yp = Y[1 + P] * wx;
+#pragma unroll
+      for (int Q = 0; Q < 3; ++Q) {
+        // (P, x) with (Q, y); (P, x) with (Q, z); (P, y) with (Q, z)
+        const int rx = 3 * P, sy = 3 * Q + 1, sz = 3 * Q + 2, ry = 3 * P + 1;
+        acc[rx < sy ? rys_tri(rx, sy) : rys_tri(sy, rx)] += xp * Y[1 + Q];
+        acc[rx < sz ? rys_tri(rx, sz) : rys_tri(sz, rx)] += xq * Z[1 + Q];
+        acc[ry < sz ? rys_tri(ry, sz) : rys_tri(sz, ry)] += yp * Z[1 + Q];
+      }
+    }
+  }
+}
+

@@ -68,9 +68,9 @@ typedef struct {
   int warp_max_quartets;   /* (dd|dp), (dd|dd): one warp per quartet when the class has at most this many
                               quartets, one thread per quartet otherwise (default 2^30 = always; -1 = never) */
   int grad_warp_max_waves;    /* gradient of (dp|dp) (dd|pp) (dd|ds) (dd|dp) (dd|dd) before any
-                                 hfgpu_autotune_grad / hfgpu_set_grad_forms: > 0 (default 48) one block of
-                                 four warps per quartet over shared-memory tables (form 3), 0 = one thread
-                                 per quartet on global scratch (form 0) */
+                                 hfgpu_autotune_grad / hfgpu_set_grad_forms: > 0 (default 48) a group of
+                                 threads per quartet by Rys quadrature, 0 = one thread per quartet on
+                                 global scratch (form 0) */
   int reserved[5];          /* reserved[0] = 1: arm every shared-memory staging wait without issuing its copy,
                               so that the bounded wait runs out (tests the timeout path; builds then report
                               status 2); 0 otherwise.  reserved[1] > 0: at most this many blocks per
@@ -138,16 +138,15 @@ int hfgpu_grad2e_uhf_backward(hfgpu_handle* h, const double* Da, const double* D
  * FP64 only; single-molecule handles (HFGPU_ERR_UNSUPPORTED for a batched handle). */
 int hfgpu_hess2e(hfgpu_handle* h, const double* D, double scale, double* hess);
 int hfgpu_hess2e_uhf(hfgpu_handle* h, const double* Da, const double* Db, double scale, double* hess);
-/* Launch form of the Hessian classes: -1 (default) one thread per quartet on straight-line
- * register code for the many-quartet classes that have it ((ss|ss), (ps|ss), (ps|ps), (pp|ss),
- * (pp|ps), (ds|ss), (ds|ps), (dp|ss)), else one block of 128
- * threads per quartet for the classes with large op tables or few quartets and one warp per
- * quartet for the others; 0 one thread per quartet on global scratch everywhere, 1 one block per
- * quartet everywhere, 2 one warp per quartet wherever four quartets' tables fit one block (the
- * block form elsewhere), 3 the straight-line form wherever the class has it (the default
- * elsewhere).  The results agree to rounding. */
+/* Launch form of the Hessian classes: -1 (default) the faster one measured per class, a group of
+ * threads per quartet by Rys quadrature for most and one thread per quartet on straight-line
+ * register code for (ss|ss), (ps|ss) and (ds|ss); 0 one thread per quartet on global scratch
+ * everywhere, 1 Rys quadrature with the class's largest group of threads per quartet everywhere,
+ * 2 with its smallest group, 3 the straight-line form wherever the class has it ((ss|ss), (ps|ss),
+ * (ps|ps), (pp|ss), (pp|ps), (ds|ss), (ds|ps), (dp|ss); the default elsewhere).  The results agree
+ * to rounding. */
 int hfgpu_set_hess_form(hfgpu_handle* h, int form);
-/* Per class (HFGPU_NUM_CLASSES ints: 0 thread, 1 block, 2 warp, 3 straight-line, -1 the rule of
+/* Per class (HFGPU_NUM_CLASSES ints: 0 thread, 1 largest group, 2 smallest group, 3 straight-line, -1 the rule of
  * hfgpu_set_hess_form), as hfgpu_autotune_hess returns them. */
 int hfgpu_set_hess_forms(hfgpu_handle* h, const int* forms);
 /* Times every class alone in each form on RHF weights of the device density D (median of
@@ -331,16 +330,15 @@ int hfgpu_setup_times(const hfgpu_handle* h, double* ms);
 int hfgpu_autotune(hfgpu_handle* h, const double* D, int precision, int repeats, int* schedule);
 int hfgpu_set_schedule(hfgpu_handle* h, const int* schedule);
 /* Gradient form per class for the classes that have several (the op-table classes (dp|dp) (dd|pp)
- * (dd|ds) (dd|dp) (dd|dd)): times one warp or one 128- or 256-thread block per quartet (whole or split
- * per set) against one thread per quartet for each class alone on the handle's lists and the
+ * (dd|ds) (dd|dp) (dd|dd)): times a group of threads per quartet by Rys quadrature, in three sizes,
+ * against one thread per quartet for each class alone on the handle's lists and the
  * given device density D (RHF weights), keeps the fastest; then, on whole gradients, tries the
  * other forms per class and keeps one where it makes the gradient at least 1% faster (the
  * classes run concurrently; last, one after another on one stream against concurrently, as for
- * the J/K build), and returns the forms in forms[HFGPU_NUM_CLASSES] (0 thread, 1 warp,
- * 2 warp split into four launches of one accumulator set each, 3 block of four warps, 4 block
- * split into four launches, 5 and 6 the same with blocks of eight warps, -1 class without a
- * choice; may be NULL).  Until it runs, the
- * classes use form 3 (opts.grad_warp_max_waves > 0) or form 0 (opts.grad_warp_max_waves = 0).
+ * the J/K build), and returns the forms in forms[HFGPU_NUM_CLASSES] (0 thread; 1, 3, 5 the class's
+ * smallest, middle and largest group, as 2, 4, 6; -1 class without a choice; may be NULL).  Until it
+ * runs, the classes use the size measured best (opts.grad_warp_max_waves > 0) or form 0
+ * (opts.grad_warp_max_waves = 0).
  * Results do not depend on the form beyond FP64 summation order. */
 int hfgpu_autotune_grad(hfgpu_handle* h, const double* D, int precision, int repeats, int* forms);
 /* Sets the gradient forms directly (HFGPU_NUM_CLASSES ints, -1 .. 6, as hfgpu_autotune_grad returns them;
