@@ -579,16 +579,45 @@ __device__ __forceinline__ void grad_weights(const double* __restrict__ DJ, doub
     }
 }
 
+// Adds the N values of every valid lane of a warp to the outputs its key names: put(n, x) adds x to
+// output n of the calling lane's key.  Lanes that share a key with at least three others are summed
+// over the warp first and one of them adds the total; the rest add their own.  Quartet lists are
+// bra-major, so a warp's quartets share their bra atoms and often a ket atom: as one atomic per lane
+// those adds retry against each other (FP64 atomics on shared memory are compare-and-swap loops),
+// 32 rounds per value.  Called by all 32 lanes.
+template <int N, typename Put>
+__device__ __forceinline__ void warp_add_by_key(bool valid, unsigned long long key, const double (&v)[N], Put put) {
+  const unsigned same = __match_any_sync(0xffffffffu, valid ? key : ~0ull);
+  const bool shared_key = valid && __popc(same) >= 4;
+  unsigned todo = __ballot_sync(0xffffffffu, shared_key);
+  const int lane = threadIdx.x & 31;
+  while (todo) {
+    const int leader = __ffs(todo) - 1;
+    const unsigned grp = __shfl_sync(0xffffffffu, same, leader);
+    const bool in = (grp >> lane) & 1u;
+#pragma unroll
+    for (int n = 0; n < N; ++n) {
+      double x = in ? v[n] : 0.0;
+#pragma unroll
+      for (int off = 16; off > 0; off >>= 1) x += __shfl_xor_sync(0xffffffffu, x, off);
+      if (lane == leader) put(n, x);
+    }
+    todo &= ~grp;
+  }
+  if (valid && !shared_key)
+#pragma unroll
+    for (int n = 0; n < N; ++n) put(n, v[n]);
+}
+
 // PASS < 0: the whole gradient of the quartet; PASS = 0..3: the part that accumulator set
 // U, A, B or C carries (classes generated with kGradPasses = 4 run one launch per pass); for
 // kGradPasses = 2, PASS = 0, 1: the part that sets U and A, or B and C, carry.
 template <int LA, int LB, int LC, int LD, typename R, bool PURE, int PASS = -1>
-__device__ __forceinline__ void grad_quartet(const GradArgs<R>& a, int tid, const int2 pq, double* gout) {
+__device__ __forceinline__ void grad_quartet(const GradArgs<R>& a, int tid, const int2 pq, const PairInfo& P,
+                                             const PairInfo& Q, double* gout) {
   using Dm = BlockDims<LA, LB, LC, LD, PURE>;
   using CC = ClassCode<LA, LB, LC, LD>;
   {
-    const PairInfo P = a.pairs[pq.x];
-    const PairInfo Q = a.pairs[pq.y];
     double s = 8.0;
     if (P.sa == P.sb) s *= 0.5;
     if (Q.sa == Q.sb) s *= 0.5;
@@ -670,15 +699,8 @@ __device__ __forceinline__ void grad_quartet(const GradArgs<R>& a, int tid, cons
                              R(Q.ABx), R(Q.ABy), R(Q.ABz), a.boys, Wc, g, g + 3, g + 6);
       }
     }
-    const int at[3] = {P.atom_a, P.atom_b, Q.atom_a};
 #pragma unroll
-    for (int d = 0; d < 3; ++d) {
-      const double gA = double(g[d]), gB = double(g[3 + d]), gC = double(g[6 + d]);
-      atomicAdd(gout + 3 * at[0] + d, gA);
-      atomicAdd(gout + 3 * at[1] + d, gB);
-      atomicAdd(gout + 3 * at[2] + d, gC);
-      atomicAdd(gout + 3 * Q.atom_b + d, -(gA + gB + gC));
-    }
+    for (int x = 0; x < 9; ++x) gout[x] = double(g[x]);
   }
 }
 
@@ -699,12 +721,34 @@ __global__ void __launch_bounds__(128) grad_kernel(GradArgs<R> a, int pure, cons
     gout = grad_sh;
   }
   const int np = a.nparts > 1 ? a.nparts : 1, p0 = np > 1 ? a.part : 0;
-  for (int t = tid; t < nq; t += nthr) {
-    const int2 pq = quartets[(size_t)t * np + p0];
-    if (pure)
-      grad_quartet<LA, LB, LC, LD, R, true, PASS>(a, tid, pq, gout);
-    else
-      grad_quartet<LA, LB, LC, LD, R, false, PASS>(a, tid, pq, gout);
+  // whole warps stay in the loop together (lanes past the end add nothing), for the shuffles of
+  // warp_add_by_key
+  for (int t = tid; t - (int)(threadIdx.x & 31) < nq; t += nthr) {
+    const bool valid = t < nq;
+    double g[9];
+#pragma unroll
+    for (int x = 0; x < 9; ++x) g[x] = 0.0;
+    int atA = 0, atB = 0, atC = 0, atD = 0;
+    if (valid) {
+      const int2 pq = quartets[(size_t)t * np + p0];
+      const PairInfo P = a.pairs[pq.x];
+      const PairInfo Q = a.pairs[pq.y];
+      atA = P.atom_a;
+      atB = P.atom_b;
+      atC = Q.atom_a;
+      atD = Q.atom_b;
+      if (pure)
+        grad_quartet<LA, LB, LC, LD, R, true, PASS>(a, tid, pq, P, Q, g);
+      else
+        grad_quartet<LA, LB, LC, LD, R, false, PASS>(a, tid, pq, P, Q, g);
+    }
+    const double gAB[6] = {g[0], g[1], g[2], g[3], g[4], g[5]}, gC[3] = {g[6], g[7], g[8]};
+    const double gD[3] = {-(g[0] + g[3] + g[6]), -(g[1] + g[4] + g[7]), -(g[2] + g[5] + g[8])};
+    warp_add_by_key<6>(valid, (unsigned long long)atA << 32 | (unsigned)atB, gAB, [&](int n, double x) {
+      atomicAdd(gout + 3 * (n < 3 ? atA : atB) + n % 3, x);
+    });
+    warp_add_by_key<3>(valid, atC, gC, [&](int n, double x) { atomicAdd(gout + 3 * atC + n, x); });
+    warp_add_by_key<3>(valid, atD, gD, [&](int n, double x) { atomicAdd(gout + 3 * atD + n, x); });
   }
   if (nsh > 0) {
     __syncthreads();
