@@ -1013,11 +1013,8 @@ HESS_INST_TEMPLATE = """// GENERATED by gen_eri.py -- do not edit.
 
 namespace hfgpu {{
 static void launch_hess(const GradArgs<double>& a, const HessOut& o, int pure, const int2* q, int nq, int grid,
-                        int smem, cudaStream_t s) {{
-  if (nq <= 0) return;
-  auto k = hess_kernel<{la}, {lb}, {lc}, {ld}, HessTable{t}>;
-  if (smem > 48 * 1024) cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
-  k<<<grid, 128, smem, s>>>(a, o, pure, q, nq);
+                        cudaStream_t s) {{
+  if (nq > 0) hess_kernel<{la}, {lb}, {lc}, {ld}, HessTable{t}><<<grid, 128, 0, s>>>(a, o, pure, q, nq);
 }}
 static int hess_scratch_slots(int) {{
   return HessTable{t}::NVSLOT + HessTable{t}::NHSLOT + 45 +
@@ -1033,33 +1030,48 @@ const HessLaunchers hess_launchers_{t} = {{{la}, {lb}, {lc}, {ld}, &launch_hess,
 # straight-line form (gen_hess_line): one thread per quartet, grid-stride over grid blocks
 HESS_LINE_LAUNCH = """// straight-line form: one thread per quartet on register code, grid blocks of 128 threads
 static bool launch_hess_line(const GradArgs<double>& a, const HessOut& o, int pure, const int2* q, int nq, int grid,
-                             int smem, cudaStream_t s) {{
+                             cudaStream_t s) {{
   if (nq <= 0) return true;
-  auto k = hess_line_kernel<{la}, {lb}, {lc}, {ld}, HessLine{t}>;
-  const int bytes = smem + kHessLineH45Bytes;  // the block's Hessian (smem > 0) and the h45 slices
-  if (bytes > 48 * 1024) cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
-  k<<<grid, kHessLineThreads, bytes, s>>>(a, o, pure, q, nq);
+  static_assert(kHessLineH45Bytes <= 48 * 1024, "shared memory without an attribute");
+  hess_line_kernel<{la}, {lb}, {lc}, {ld}, HessLine{t}><<<grid, kHessLineThreads, kHessLineH45Bytes, s>>>(a, o, pure, q, nq);
   return true;
 }}"""
 HESS_LINE_NONE = """// no straight-line form: the class's passes would spill or be too many (gen_hess_line)
-static bool launch_hess_line(const GradArgs<double>&, const HessOut&, int, const int2*, int, int, int, cudaStream_t) {
+static bool launch_hess_line(const GradArgs<double>&, const HessOut&, int, const int2*, int, int, cudaStream_t) {
   return false;
 }"""
 
 
 RYS_INST_TEMPLATE = """// GENERATED by gen_eri.py -- do not edit.
-#include "../hfgpu_rys.cuh"
+#include "../hfgpu_rys3.cuh"
 #include "../hfgpu_rys_launch.h"
 
 namespace hfgpu {{
 extern const RysLaunchers rys_launchers_{t};
-const RysLaunchers rys_launchers_{t} = {{
-    {la}, {lb}, {lc}, {ld}, {{{g0}, {g1}, {g2}}}, {gv}, {hv},
-    {{&launch_rys<{c}, 1, double, {g0}>, &launch_rys<{c}, 1, double, {g1}>, &launch_rys<{c}, 1, double, {g2}>}},
-    {{&launch_rys<{c}, 1, float, {g0}>, &launch_rys<{c}, 1, float, {g1}>, &launch_rys<{c}, 1, float, {g2}>}},
-    {{&launch_rys<{c}, 2, double, {g0}>, &launch_rys<{c}, 2, double, {g1}>, &launch_rys<{c}, 2, double, {g2}>}}}};
+const RysLaunchers rys_launchers_{t} = {{{la}, {lb}, {lc}, {ld}, {gv}, {p64}, {hv},
+    {{{gd}}},
+    {{{gf}}},
+    {{{hd}}}}};
 }}  // namespace hfgpu
 """
+
+# Cartesian block of the classes that have the form of three threads per quartet, by order and precision
+RYS_THREE_MAX_CART = {(1, "double"): 162, (1, "float"): 0, (2, "double"): 81}
+
+
+def rys_inst(c, t):
+    """Translation unit of a class's Rys-quadrature launchers."""
+    n = ncart(c[0]) * ncart(c[1]) * ncart(c[2]) * ncart(c[3])
+    cl = ", ".join(map(str, c))
+
+    def row(order, real):
+        fns = [f"&launch_rys<{cl}, {order}, {real}, {g}>" for g in rys_groups(*c)]
+        fns.append(f"&launch_rys3<{cl}, {order}, {real}>" if n <= RYS_THREE_MAX_CART[order, real] else "nullptr")
+        return ", ".join(fns)
+
+    gv, p64, hv = rys_defaults(c)
+    return RYS_INST_TEMPLATE.format(t=t, la=c[0], lb=c[1], lc=c[2], ld=c[3], gv=gv, p64=p64, hv=hv, gd=row(1, "double"),
+                                    gf=row(1, "float"), hd=row(2, "double"))
 
 
 def rys_groups(la, lb, lc, ld):
@@ -1076,23 +1088,36 @@ def rys_groups(la, lb, lc, ld):
     return (32, 64, 128)
 
 
-# Default forms of the derivative classes, by their Cartesian block, measured per class on n-octane,
-# anthracene and water clusters (device time of the class alone; thread form / Rys quadrature):
-# gradient: the op-table classes take Rys quadrature ((dp|dp) 1.25 / 0.36 ms on octane, (dd|dp) 1.03 /
-# 0.17, (dd|dd) 0.41 / 0.03, against one block per quartet over the op tables); the straight-line
-# ones keep one thread per quartet ((pp|ps) 1.5 / 4.3; (dp|pp) 1.86 / 1.39 on octane but 7.4 / 12.1 on
-# anthracene with its longer contractions).
-# Hessian: Rys quadrature everywhere ((pp|ps) 35 / 12 ms, (dp|dp) 21 / 1.0, (dd|dd) 2.8 / 0.06) but for
-# (ss|ss), (ps|ss) and (ds|ss) (3.3 / 4.9, 8.1 / 14, 4.5 / 5.0).
-RYS_HESS_LINE = ((0, 0, 0, 0), (1, 0, 0, 0), (2, 0, 0, 0))
+# Default forms of the derivative classes, measured per class (device time of the class alone, ms;
+# n-octane/6-31G** with 1-17 primitive quartets per quartet, anthracene/cc-pVDZ with 1-190).
+#
+# Hessian, octane: (ss|ss) straight-line 2.04 against three-thread Rys 2.24; every other class with a
+# Cartesian block of at most 81 (and (dp|ps), (ds|pp) ... below it) three-thread Rys: (ps|ss) 4.90
+# against 5.03, (ps|ps) 4.0 against 10.5, (pp|ps) 3.0 against 22.7 straight-line and 8.5 in groups,
+# (dp|ps) 3.5 against 6.4 in groups; the larger ones in groups, where three threads spill ((dp|pp) 2.8
+# against 4.2, (dp|ds) 1.7 against 2.3).
+RYS_HESS_LINE = ((0, 0, 0, 0),)
+RYS_HESS_THREE_MAX_CART = 81
+# Gradient: the op-table classes in groups ((dp|dp) 0.35 against 0.74 in three threads).  Of the others,
+# three-thread Rys costs less per quartet and more per primitive quartet than the straight-line code,
+# so it runs up to an average number of primitive quartets per quartet: on octane
+# at 2.9 per quartet (dp|pp) takes 1.20 against 1.84, on anthracene at 7.9 6.0 against 5.3; (pp|pp)
+# 0.48 / 1.25 and 2.0 / 4.5 at 4.1 and 15.4; (pp|ps), (ds|ps) and smaller lose even at 6.  FP64 only: in
+# FP32 its rounding moved the mixed gradient of anthracene by 1.6e-9 of its norm.
+RYS_GRAD_THREE_PRIMS = {(1, 1, 1, 1): 1000, (2, 0, 1, 1): 20, (2, 0, 2, 0): 1000, (2, 1, 1, 0): 9, (2, 1, 1, 1): 6,
+                        (2, 1, 2, 0): 11, (2, 2, 0, 0): 1000, (2, 2, 1, 0): 8}
 
 
 def rys_defaults(c):
-    """(gradient, Hessian) default variant of class c, -1 = the straight-line form."""
+    """(gradient variant, primitive-quartet limit of the three-thread gradient, Hessian variant) of class
+    c; -1 = the straight-line form."""
     n = ncart(c[0]) * ncart(c[1]) * ncart(c[2]) * ncart(c[3])
     grad = -1 if n < 216 else (2 if n == 1296 else 0)
-    hess = -1 if c in RYS_HESS_LINE else (1 if n in (1, 1296) or c in ((2, 1, 0, 0),) else 0)
-    return grad, hess
+    if c in RYS_HESS_LINE:
+        hess = -1
+    else:
+        hess = 3 if n <= RYS_HESS_THREE_MAX_CART else (1 if n == 1296 else 0)
+    return grad, RYS_GRAD_THREE_PRIMS.get(c, 0), hess
 
 
 def main(outdir):
@@ -1140,10 +1165,7 @@ def main(outdir):
             line_fn=(HESS_LINE_LAUNCH.format(t=t, la=la, lb=lb, lc=lc, ld=ld) if line else HESS_LINE_NONE),
             has_line="true" if line else "false"))
         hnames.append(t)
-        g = rys_groups(*c)
-        write_if_changed(os.path.join(outdir, f"rys_{t}.cu"), RYS_INST_TEMPLATE.format(
-            t=t, la=la, lb=lb, lc=lc, ld=ld, c=f"{la}, {lb}, {lc}, {ld}", g0=g[0], g1=g[1], g2=g[2],
-            gv=rys_defaults(c)[0], hv=rys_defaults(c)[1]))
+        write_if_changed(os.path.join(outdir, f"rys_{t}.cu"), rys_inst(c, t))
     rd = ["// GENERATED by gen_eri.py -- do not edit.", '#include "../hfgpu_rys_launch.h"', "namespace hfgpu {"]
     rd += [f"extern const RysLaunchers rys_launchers_{t};" for t in hnames]
     rd.append(f"const RysLaunchers* const kRysLaunchers[{len(hnames)}] = {{")

@@ -18,12 +18,10 @@
 #pragma once
 #include "hfgpu_kernels.cuh"
 
-// Hessian output of a launch: 3 natoms x 3 natoms, row-major.  smem > 0: the block sums its
-// contributions in shared memory (9 natoms^2 doubles) and adds them once at its end.
+// Hessian output of a launch: 3 natoms x 3 natoms, row-major, half of it (HessEntry).
 struct HessOut {
   double* __restrict__ hess;
   int natoms;
-  int smem;
 };
 
 // Executor of a table-mode Hessian class.  Weight sets, in the generator's order:
@@ -116,42 +114,117 @@ __device__ void hess_table(const PrimPair<double>* __restrict__ bp, const double
 // Position of coordinate pair (r, s), r <= s, of the 9 x 9 block in the 45-entry upper triangle.
 __device__ __forceinline__ int hess_tri(int r, int s) { return r * 9 - r * (r - 1) / 2 + (s - r); }
 
-// Adds the quartet's 12 x 12 block over centres A, B, C, D (atoms at[0..3]) into the
-// 3 natoms x 3 natoms Hessian hout: the A, B, C part from the 45 entries h45, a D row or column
-// as minus the sum of the A, B, C ones (translational invariance).
-template <typename H>
-__device__ __forceinline__ void hess_add_block(const H& h45, const int (&at)[4], double* hout, int n3) {
-  // unrolled, so that a register array h45 is read at constant indexes
-#pragma unroll
-  for (int i = 0; i < 3; ++i)
-#pragma unroll
-    for (int j = 0; j < 3; ++j) {
-      double hx[4][4];
-#pragma unroll
-      for (int X = 0; X < 3; ++X)
-#pragma unroll
-        for (int Y = 0; Y < 3; ++Y) {
-          const int r = 3 * X + i, c = 3 * Y + j;
-          hx[X][Y] = r <= c ? h45[hess_tri(r, c)] : h45[hess_tri(c, r)];
-        }
-#pragma unroll
-      for (int X = 0; X < 3; ++X) hx[X][3] = -(hx[X][0] + hx[X][1] + hx[X][2]);
-#pragma unroll
-      for (int Y = 0; Y < 4; ++Y) hx[3][Y] = -(hx[0][Y] + hx[1][Y] + hx[2][Y]);
-#pragma unroll
-      for (int X = 0; X < 4; ++X)
-#pragma unroll
-        for (int Y = 0; Y < 4; ++Y)
-          if (hx[X][Y] != 0.0) atomicAdd(hout + (size_t)(3 * at[X] + i) * n3 + 3 * at[Y] + j, hx[X][Y]);
+// The 3 natoms x 3 natoms output collects, per pair of coordinates, one of its two symmetric
+// entries: U with H = U + U^T (hess_finish_kernel), so that a quartet adds 78 values, not 144.  Of
+// centre blocks X < Y every entry is added, of X = Y those with i < j and half of those with i = j.
+// (Two centres on one atom need no special case.)
+//
+// Entry t of the 78: centres X <= Y of A, B, C, D and directions i, j.  Six centre pairs of nine
+// entries, then four symmetric blocks of six.
+struct HessEntry {
+  int X, i, Y, j;
+  __device__ __forceinline__ explicit HessEntry(int t) {
+    if (t < 54) {
+      const int k = t / 9;
+      X = k < 3 ? 0 : (k < 5 ? 1 : 2);
+      Y = k < 3 ? k + 1 : (k < 5 ? k - 1 : 3);
+      i = t % 9 / 3;
+      j = t % 3;
+    } else {
+      const int n = (t - 54) % 6;
+      X = Y = (t - 54) / 6;
+      i = n < 3 ? 0 : (n < 5 ? 1 : 2);
+      j = n < 3 ? n : (n < 5 ? n - 2 : 2);
     }
+  }
+  // Its value from the quartet's 45 entries over A, B, C: a D row or column is minus the sum of the
+  // others (translational invariance).
+  template <typename H>
+  __device__ __forceinline__ double value(const H& h45) const {
+    double v = 0.0;
+#pragma unroll 1
+    for (int u = X < 3 ? X : 0; u < (X < 3 ? X + 1 : 3); ++u)
+#pragma unroll 1
+      for (int w = Y < 3 ? Y : 0; w < (Y < 3 ? Y + 1 : 3); ++w) {
+        const int m = 3 * u + i, n = 3 * w + j;
+        v += double(h45[m < n ? hess_tri(m, n) : hess_tri(n, m)]);
+      }
+    if ((X == 3) != (Y == 3)) v = -v;
+    return X == Y && i == j ? 0.5 * v : v;
+  }
+  __device__ __forceinline__ long long offset(const int (&at)[4], int n3) const {
+    const int r = X == 0 ? at[0] : (X == 1 ? at[1] : (X == 2 ? at[2] : at[3]));
+    const int c = Y == 0 ? at[0] : (Y == 1 ? at[1] : (Y == 2 ? at[2] : at[3]));
+    return (long long)(3 * r + i) * n3 + 3 * c + j;
+  }
+};
+
+// Adds entries first, first + step, ... of one quartet (atoms at[0..3]) into U.
+template <typename H>
+__device__ __forceinline__ void hess_add_block(const H& h45, const int (&at)[4], double* U, int n3, int first,
+                                               int step) {
+#pragma unroll 1
+  for (int t = first; t < 78; t += step) {
+    const HessEntry e(t);
+    atomicAdd(U + e.offset(at, n3), e.value(h45));
+  }
+}
+
+// Adds the blocks of a warp's quartets (one per valid lane, atoms at, 45 entries in shared memory at
+// h45[x stride + lane qstride]) into U: the warp walks its quartets, each lane owning up to three of the 78
+// entries, and adds to memory only when the entry's place changes.  The lists are bra-major, so the
+// bra atoms hold for most of a warp and a ket atom for runs of it: few atomics, none against each
+// other.  (One lane per quartet adding its own 78 entries retried 32 compare-and-swap loops per
+// value, and as unrolled code it missed the instruction cache.)  Called by all lanes.
+__device__ __forceinline__ void hess_add_warp(bool valid, const double* h45, int stride, int qstride,
+                                              const int (&at)[4], double* U, int n3) {
+  struct Column {
+    const double* p;
+    int stride;
+    __device__ __forceinline__ double operator[](int x) const { return p[x * stride]; }
+  };
+  __syncwarp();
+  const int lane = threadIdx.x & 31;
+  const HessEntry e[3] = {HessEntry(lane), HessEntry(lane + 32), HessEntry(lane + 64 < 78 ? lane + 64 : 77)};
+  double sum[3] = {0.0, 0.0, 0.0};
+  long long cur[3] = {-1, -1, -1};
+#pragma unroll 1
+  for (unsigned m = __ballot_sync(0xffffffffu, valid); m; m &= m - 1) {
+    const int q = __ffs(m) - 1;
+    int aq[4];
+#pragma unroll
+    for (int c = 0; c < 4; ++c) aq[c] = __shfl_sync(0xffffffffu, at[c], q);
+    const Column h{h45 + q * qstride, stride};
+#pragma unroll
+    for (int k = 0; k < 3; ++k) {
+      if (k == 2 && lane + 64 >= 78) continue;
+      const long long off = e[k].offset(aq, n3);
+      if (off != cur[k]) {
+        if (cur[k] >= 0) atomicAdd(U + cur[k], sum[k]);
+        cur[k] = off;
+        sum[k] = 0.0;
+      }
+      sum[k] += e[k].value(h);
+    }
+  }
+#pragma unroll
+  for (int k = 0; k < 3; ++k)
+    if (cur[k] >= 0) atomicAdd(U + cur[k], sum[k]);
+  __syncwarp();
+}
+
+// hess += U + U^T.
+static __global__ void hess_finish_kernel(const double* __restrict__ U, double* __restrict__ hess, int n3) {
+  const size_t e = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
+  if (e >= (size_t)n3 * n3) return;
+  const size_t r = e / n3, c = e % n3;
+  hess[e] += U[e] + U[c * n3 + r];
 }
 
 template <int LA, int LB, int LC, int LD, bool PURE, typename Tab>
-__device__ __forceinline__ void hess_quartet(const GradArgs<double>& a, const HessOut& o, int tid, const int2 pq,
-                                             double* hout, int n3) {
+__device__ __forceinline__ void hess_quartet(const GradArgs<double>& a, int tid, const int2 pq, const PairInfo& P,
+                                             const PairInfo& Q) {
   using Dm = BlockDims<LA, LB, LC, LD, PURE>;
-  const PairInfo P = a.pairs[pq.x];
-  const PairInfo Q = a.pairs[pq.y];
   double s = 8.0;
   if (P.sa == P.sb) s *= 0.5;
   if (Q.sa == Q.sb) s *= 0.5;
@@ -205,35 +278,26 @@ __device__ __forceinline__ void hess_quartet(const GradArgs<double>& a, const He
   hess_table<Tab>(a.prims + P.prim_off, a.alpha_a + P.prim_off, a.alpha_b + P.prim_off, P.nprim,
                   a.prims + Q.prim_off, a.alpha_a + Q.prim_off, Q.nprim, P.ABx, P.ABy, P.ABz, Q.ABx, Q.ABy, Q.ABz,
                   a.boys, Wc, vs, hs, h45);
-  const int at[4] = {P.atom_a, P.atom_b, Q.atom_a, Q.atom_b};
-  hess_add_block(h45, at, hout, n3);
 }
 
 template <int LA, int LB, int LC, int LD, typename Tab>
 __global__ void __launch_bounds__(128) hess_kernel(GradArgs<double> a, HessOut o, int pure,
                                                    const int2* __restrict__ quartets, int nq) {
-  extern __shared__ double hess_sh[];
   const int tid = blockIdx.x * blockDim.x + threadIdx.x;
   const int nthr = gridDim.x * blockDim.x;
-  const int n3 = 3 * o.natoms;
-  double* hout = o.hess;
-  if (o.smem) {
-    for (int i = threadIdx.x; i < n3 * n3; i += blockDim.x) hess_sh[i] = 0.0;
-    __syncthreads();
-    hout = hess_sh;
-  }
+  const Strided<double> h45{a.scratch + tid + (size_t)(Tab::NVSLOT + Tab::NHSLOT) * a.scratch_threads,
+                            a.scratch_threads};
   const int np = a.nparts > 1 ? a.nparts : 1, p0 = np > 1 ? a.part : 0;
   for (int t = tid; t < nq; t += nthr) {
     const int2 pq = quartets[(size_t)t * np + p0];
+    const PairInfo P = a.pairs[pq.x];
+    const PairInfo Q = a.pairs[pq.y];
     if (pure)
-      hess_quartet<LA, LB, LC, LD, true, Tab>(a, o, tid, pq, hout, n3);
+      hess_quartet<LA, LB, LC, LD, true, Tab>(a, tid, pq, P, Q);
     else
-      hess_quartet<LA, LB, LC, LD, false, Tab>(a, o, tid, pq, hout, n3);
-  }
-  if (o.smem) {
-    __syncthreads();
-    for (int i = threadIdx.x; i < n3 * n3; i += blockDim.x)
-      if (hess_sh[i] != 0.0) atomicAdd(o.hess + i, hess_sh[i]);
+      hess_quartet<LA, LB, LC, LD, false, Tab>(a, tid, pq, P, Q);
+    const int at[4] = {P.atom_a, P.atom_b, Q.atom_a, Q.atom_b};
+    hess_add_block(h45, at, o.hess, 3 * o.natoms, 0, 1);
   }
 }
 
@@ -247,7 +311,8 @@ __global__ void __launch_bounds__(128) hess_kernel(GradArgs<double> a, HessOut o
 // or on global scratch round trips rather than on the few dozen ops of a level.
 // ---------------------------------------------------------------------------
 constexpr int kHessLineThreads = 128;
-constexpr int kHessLineH45Bytes = 45 * kHessLineThreads * (int)sizeof(double);
+constexpr int kHessLineStride = kHessLineThreads + 1;  // odd: the lanes of hess_add_warp read one column
+constexpr int kHessLineH45Bytes = 45 * kHessLineStride * (int)sizeof(double);
 
 // grad_weights with every loop over the block unrolled, so that W stays in registers
 template <int NA, int NB, int NC, int ND>
@@ -276,11 +341,9 @@ __device__ __forceinline__ void hess_line_weights(const double* __restrict__ DJ,
 }
 
 template <int LA, int LB, int LC, int LD, bool PURE, typename Line>
-__device__ __forceinline__ void hess_line_quartet(const GradArgs<double>& a, const int2 pq, Strided<double> h45,
-                                                  double* hout, int n3) {
+__device__ __forceinline__ void hess_line_quartet(const GradArgs<double>& a, const int2 pq, const PairInfo& P,
+                                                  const PairInfo& Q, Strided<double> h45) {
   using Dm = BlockDims<LA, LB, LC, LD, PURE>;
-  const PairInfo P = a.pairs[pq.x];
-  const PairInfo Q = a.pairs[pq.y];
   double s = 8.0;
   if (P.sa == P.sb) s *= 0.5;
   if (Q.sa == Q.sb) s *= 0.5;
@@ -302,38 +365,34 @@ __device__ __forceinline__ void hess_line_quartet(const GradArgs<double>& a, con
   Line::template run<double>(a.prims + P.prim_off, a.alpha_a + P.prim_off, a.alpha_b + P.prim_off, P.nprim,
                              a.prims + Q.prim_off, a.alpha_a + Q.prim_off, Q.nprim, P.ABx, P.ABy, P.ABz, Q.ABx,
                              Q.ABy, Q.ABz, a.boys, weights, h45);
-  const int at[4] = {P.atom_a, P.atom_b, Q.atom_a, Q.atom_b};
-  hess_add_block(h45, at, hout, n3);
 }
 
-// dynamic shared memory: [the block's Hessian, 9 natoms^2 doubles, when o.smem | h45 slices]
+// dynamic shared memory: the h45 slices
 template <int LA, int LB, int LC, int LD, typename Line>
 __global__ void __launch_bounds__(kHessLineThreads) hess_line_kernel(GradArgs<double> a, HessOut o, int pure,
                                                                      const int2* __restrict__ quartets, int nq) {
   extern __shared__ double hess_sh[];
   const int tid = blockIdx.x * blockDim.x + threadIdx.x;
   const int nthr = gridDim.x * blockDim.x;
-  const int n3 = 3 * o.natoms;
-  double* hout = o.hess;
-  double* h45_base = hess_sh;
-  if (o.smem) {
-    for (int i = threadIdx.x; i < n3 * n3; i += blockDim.x) hess_sh[i] = 0.0;
-    __syncthreads();
-    hout = hess_sh;
-    h45_base = hess_sh + n3 * n3;
-  }
-  const Strided<double> h45{h45_base + threadIdx.x, kHessLineThreads};
+  const Strided<double> h45{hess_sh + threadIdx.x, kHessLineStride};
   const int np = a.nparts > 1 ? a.nparts : 1, p0 = np > 1 ? a.part : 0;
-  for (int t = tid; t < nq; t += nthr) {
-    const int2 pq = quartets[(size_t)t * np + p0];
-    if (pure)
-      hess_line_quartet<LA, LB, LC, LD, true, Line>(a, pq, h45, hout, n3);
-    else
-      hess_line_quartet<LA, LB, LC, LD, false, Line>(a, pq, h45, hout, n3);
-  }
-  if (o.smem) {
-    __syncthreads();
-    for (int i = threadIdx.x; i < n3 * n3; i += blockDim.x)
-      if (hess_sh[i] != 0.0) atomicAdd(o.hess + i, hess_sh[i]);
+  // whole warps stay in the loop together (lanes past the end add nothing), for hess_add_warp
+  for (int t = tid; t - (int)(threadIdx.x & 31) < nq; t += nthr) {
+    const bool valid = t < nq;
+    int at[4] = {0, 0, 0, 0};
+    if (valid) {
+      const int2 pq = quartets[(size_t)t * np + p0];
+      const PairInfo P = a.pairs[pq.x];
+      const PairInfo Q = a.pairs[pq.y];
+      at[0] = P.atom_a;
+      at[1] = P.atom_b;
+      at[2] = Q.atom_a;
+      at[3] = Q.atom_b;
+      if (pure)
+        hess_line_quartet<LA, LB, LC, LD, true, Line>(a, pq, P, Q, h45);
+      else
+        hess_line_quartet<LA, LB, LC, LD, false, Line>(a, pq, P, Q, h45);
+    }
+    hess_add_warp(valid, hess_sh + (threadIdx.x & ~31), kHessLineStride, 1, at, o.hess, 3 * o.natoms);
   }
 }

@@ -11,16 +11,13 @@ namespace hfgpu {
 
 struct HessLaunchers {
   int la, lb, lc, ld;
-  // hess_kernel over quartets q[0, nq) with grid blocks of 128 threads and smem bytes of
-  // dynamic shared memory (0: atomics straight into the output)
-  void (*launch)(const GradArgs<double>&, const HessOut&, int pure, const int2* q, int nq, int grid, int smem,
-                 cudaStream_t);
+  // hess_kernel over quartets q[0, nq) with grid blocks of 128 threads
+  void (*launch)(const GradArgs<double>&, const HessOut&, int pure, const int2* q, int nq, int grid, cudaStream_t);
   int (*scratch_slots)(int pure);  // doubles of scratch per thread
   // straight-line form (hess_line_kernel, one thread per quartet on register code, grid blocks of
-  // 128 threads; smem as for launch, to which the launcher adds the threads' 45-entry slices);
-  // false when the class has none
+  // 128 threads); false when the class has none
   bool has_line;
-  bool (*launch_line)(const GradArgs<double>&, const HessOut&, int pure, const int2* q, int nq, int grid, int smem,
+  bool (*launch_line)(const GradArgs<double>&, const HessOut&, int pure, const int2* q, int nq, int grid,
                       cudaStream_t);
 };
 

@@ -167,6 +167,7 @@ struct hfgpu_handle {
   // the Boys table in the plane layout of the staged kernels, and the device status word
   DevBuf d_boys_pd, d_boys_pf, d_status, d_abort;
   DevBuf d_purify;  // workspace of hfgpu_purify_device
+  DevBuf d_hess;    // half Hessian of hess_device_impl
   const double* rys_tab = nullptr;  // quadrature tables of the Rys kernels on this device
   cudaStream_t ctl_stream = nullptr;  // non-blocking stream of hfgpu_request_abort
   int status_host = 0;  // the status word as the last host-pointer entry point read it
@@ -1337,11 +1338,14 @@ constexpr int kGradForms = 7;
 static bool grad_has_forms(int c) { return hfgpu::kClassLaunchers[c]->grad_scratch_slots(0) > 0; }
 
 // Form of a gradient launch of class c: the one hfgpu_autotune_grad or hfgpu_set_grad_forms
-// chose, else the class's default: kGradForms + 1 + v for Rys quadrature in group size v, 0 for one
+// chose, else the class's default: kGradForms + 1 + v for Rys quadrature in variant v, 0 for one
 // thread per quartet on straight-line code; opts.grad_warp_max_waves <= 0 asks for the thread form
 // of the op-table classes instead.
-static int grad_form_of(const hfgpu_handle* h, int c) {
-  const int v = hfgpu::kRysLaunchers[c]->grad_variant;
+static int grad_form_of(const hfgpu_handle* h, int c, bool fp32) {
+  const hfgpu::RysLaunchers* Y = hfgpu::kRysLaunchers[c];
+  int v = Y->grad_variant;
+  const long long limit = fp32 ? 0 : Y->three_prims;
+  if (limit > 0 && h->q_prims[c] <= limit * (h->q_end[c] - h->q_beg[c])) v = hfgpu::kRysThree;
   if (grad_has_forms(c)) {
     if (h->grad_form[c] >= 0) return h->grad_form[c];
     if (h->opts.grad_warp_max_waves <= 0) return 0;
@@ -1407,7 +1411,7 @@ static int grad_device_impl(hfgpu_handle* h, const double* DJ, double cJ, int nK
     const long long nq = h->q_end[c] - h->q_beg[c];
     slice_off[c] = slice_off_f[c] = need_total;
     if (slots <= 0 || nq <= 0) continue;
-    if (grad_form_of(h, c) >= 1) continue;  // no scratch
+    if (grad_form_of(h, c, false) >= 1) continue;  // no scratch (both precisions take the same form)
     const size_t one = (size_t)slots * sizeof(double) * (size_t)table_threads(slots, nq);
     need_total += (one + 255) / 256 * 256;
     if (precision == HFGPU_MIXED) {
@@ -1429,7 +1433,7 @@ static int grad_device_impl(hfgpu_handle* h, const double* DJ, double cJ, int nK
     auto run = [&](bool fp32, long long lo, long long hi) -> int {
       const int nq = (int)part_share(h, hi - lo);
       if (nq <= 0) return HFGPU_OK;
-      const int form = grad_form_of(h, c);
+      const int form = grad_form_of(h, c, fp32);
       if (form >= 1) {
         const hfgpu::RysLaunchers* Y = hfgpu::kRysLaunchers[c];
         const int v = form > kGradForms ? form - kGradForms - 1 : (form - 1) / 2;
@@ -1686,7 +1690,7 @@ int hfgpu_destroy(hfgpu_handle* h) {
   for (DevBuf* d : {&h->d_onee, &h->d_pairs, &h->d_prim_d, &h->d_prim_f, &h->d_alpha_d, &h->d_alpha_f, &h->d_boys_d, &h->d_boys_f,
                     &h->d_quart, &h->d_mats, &h->d_half, &h->d_dmax, &h->d_counters, &h->d_grad, &h->d_scratch,
                     &h->d_eri, &h->d_eriq, &h->d_launch, &h->d_dyn, &h->d_first, &h->d_boys_pd,
-                    &h->d_boys_pf, &h->d_status, &h->d_abort, &h->d_purify})
+                    &h->d_boys_pf, &h->d_status, &h->d_abort, &h->d_purify, &h->d_hess})
     d->release();
   h->d_mol.release();
   if (h->ev[0])
@@ -1970,7 +1974,6 @@ int hfgpu_grad2e_uhf_backward(hfgpu_handle* h, const double* Da, const double* D
 // another; a class gets as many threads (whole 128-thread blocks) as kHessScratchBudget holds
 // (enough to fill the GPU for the largest tables), at most one per quartet, and loops over the rest.
 constexpr size_t kHessScratchBudget = (size_t)2 << 30;
-constexpr size_t kHessSmemBytes = 96 * 1024;  // per-block Hessian in shared memory up to 36 atoms
 constexpr long long kHessLineGrid = 4 * 148;     // straight-line form: at most four blocks per SM, grid-stride
 
 static int hess_device_impl(hfgpu_handle* h, const double* DJ, double cJ, int nK, const double* DK, double cK,
@@ -1990,9 +1993,12 @@ static int hess_device_impl(hfgpu_handle* h, const double* DJ, double cJ, int nK
   gd.part = h->part;
   gd.nparts = h->nparts;
   const size_t n3 = 3 * (size_t)h->natoms;
-  const size_t smem = sizeof(double) * n3 * n3;
-  HessOut o{hess, h->natoms, smem <= kHessSmemBytes ? 1 : 0};
-  RysOut ro{h->rys_tab, hess, h->natoms, 0};
+  // the classes add into U, hess += U + U^T at the end
+  HF_CUDA(h, h->d_hess.ensure(sizeof(double) * n3 * n3));
+  double* U = h->d_hess.as<double>();
+  HF_CUDA(h, cudaMemsetAsync(U, 0, sizeof(double) * n3 * n3, h->stream));
+  HessOut o{U, h->natoms};
+  RysOut ro{h->rys_tab, U, h->natoms, 0};
   const int2* q = h->d_quart.as<int2>();
   auto threads_of = [&](int slots, long long nq) -> long long {
     long long thr = (long long)(kHessScratchBudget / ((size_t)slots * sizeof(double)));
@@ -2044,7 +2050,7 @@ static int hess_device_impl(hfgpu_handle* h, const double* DJ, double cJ, int nK
     const long long nq = part_share(h, h->q_end[c] - h->q_beg[c]);
     if (form_of(c) == 3) {
       const long long grid = std::min<long long>((nq + 127) / 128, kHessLineGrid);
-      if (!L->launch_line(gd, o, h->pure, q + h->q_beg[c], (int)nq, (int)grid, o.smem ? (int)smem : 0,
+      if (!L->launch_line(gd, o, h->pure, q + h->q_beg[c], (int)nq, (int)grid,
                           h->aux[stream_of[c]]))
         return fail(h, HFGPU_ERR_STATE, "class without a Hessian straight-line form");
       HF_CHECK_LAUNCH(h, "hess line kernel");
@@ -2052,7 +2058,7 @@ static int hess_device_impl(hfgpu_handle* h, const double* DJ, double cJ, int nK
     }
     if (form_of(c) != 0) {
       const hfgpu::RysLaunchers* Y = hfgpu::kRysLaunchers[c];
-      const int v = form_of(c) == 1 ? hfgpu::kRysVariants - 1 : (form_of(c) == 2 ? 0 : Y->hess_variant);
+      const int v = form_of(c) == 1 ? 2 : (form_of(c) == 2 ? 0 : Y->hess_variant);
       if (!Y->hess[v](gd, ro, h->pure, q + h->q_beg[c], (int)nq, 0, h->aux[stream_of[c]]))
         return fail(h, HFGPU_ERR_CUDA, "Hessian launch: shared memory");
       HF_CHECK_LAUNCH(h, "hess kernel");
@@ -2065,10 +2071,13 @@ static int hess_device_impl(hfgpu_handle* h, const double* DJ, double cJ, int nK
       return fail(h, HFGPU_ERR_NOMEM, "Hessian scratch too small");
     gd.scratch = reinterpret_cast<double*>(h->d_scratch.as<unsigned char>() + off[st]);
     gd.scratch_threads = (int)thr;
-    L->launch(gd, o, h->pure, q + h->q_beg[c], (int)nq, (int)(thr / 128), o.smem ? (int)smem : 0, h->aux[st]);
+    L->launch(gd, o, h->pure, q + h->q_beg[c], (int)nq, (int)(thr / 128), h->aux[st]);
     HF_CHECK_LAUNCH(h, "hess kernel");
   }
-  return join_streams(h);
+  if ((rc = join_streams(h))) return rc;
+  hess_finish_kernel<<<(unsigned)((n3 * n3 + 255) / 256), 256, 0, h->stream>>>(U, hess, (int)n3);
+  HF_CHECK_LAUNCH(h, "hess finish kernel");
+  return HFGPU_OK;
 }
 
 int hfgpu_set_hess_form(hfgpu_handle* h, int form) {

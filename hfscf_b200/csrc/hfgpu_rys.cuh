@@ -15,7 +15,7 @@
 // op tables; here the state of a root is a few hundred table entries whatever the class, the code
 // is compact, and the inner loop is register arithmetic on broadcast-friendly shared-memory loads.
 #pragma once
-#include "hfgpu_kernels.cuh"
+#include "hfgpu_hess_kernels.cuh"
 #include "hfgpu_rys_math.cuh"
 
 // Synchronises the threads of a group: G <= 32 the whole warp (its groups run in step), else the
@@ -93,7 +93,8 @@ __device__ __forceinline__ void rys_weights(const GradArgs<R>& a, int pure, cons
   }
 }
 
-// Output of a launch: order 1 GradArgs::grad; order 2 hess, 3 natoms x 3 natoms row-major.
+// Output of a launch: order 1 GradArgs::grad; order 2 hess, 3 natoms x 3 natoms row-major, half of it
+// (HessEntry).
 struct RysOut {
   const double* __restrict__ tab;  // quadrature tables
   double* __restrict__ hess;
@@ -102,7 +103,7 @@ struct RysOut {
 };
 
 // G threads per quartet, BLOCK threads per block (BLOCK = G when G > 32), grid-stride over quartets.
-// Dynamic shared memory: [BLOCK / G groups of RysDims::kGroup values | NCART packed 2-D indexes of
+// Dynamic shared memory: [BLOCK / G groups of RysDims::group(G) values | NCART packed 2-D indexes of
 // the integrals | order 1: 3 smem_atoms doubles].
 template <int LA, int LB, int LC, int LD, int ORD, typename R, int G, int BLOCK>
 __global__ void __launch_bounds__(BLOCK) rys_deriv_kernel(GradArgs<R> a, RysOut o, int pure,
@@ -113,12 +114,12 @@ __global__ void __launch_bounds__(BLOCK) rys_deriv_kernel(GradArgs<R> a, RysOut 
   constexpr int GROUPS = BLOCK / G;
   const int lane = threadIdx.x % G, grp = threadIdx.x / G;
   double* gsum = reinterpret_cast<double*>(rys_sm);
-  R* rw = reinterpret_cast<R*>(gsum + (ORD == 1 ? 3 * o.smem_atoms : 0)) + (size_t)grp * D::kGroup;
+  R* rw = reinterpret_cast<R*>(gsum + (ORD == 1 ? 3 * o.smem_atoms : 0)) + (size_t)grp * D::group(G);
   R* g2 = rw + D::kRW;
   R* bv = g2 + D::kG2;
   R* vt = bv + D::kBV;
   R* W = rw + D::kWork;
-  int* tab = reinterpret_cast<int*>(rw + (size_t)(GROUPS - grp) * D::kGroup);
+  int* tab = reinterpret_cast<int*>(rw + (size_t)(GROUPS - grp) * D::group(G));
   for (int e = threadIdx.x; e < D::NCART; e += BLOCK) tab[e] = rys_index<LA, LB, LC, LD>(e);
   if (ORD == 1)
     for (int i = threadIdx.x; i < 3 * o.smem_atoms; i += BLOCK) gsum[i] = 0.0;
@@ -174,21 +175,21 @@ __global__ void __launch_bounds__(BLOCK) rys_deriv_kernel(GradArgs<R> a, RysOut 
         const R PA = d == 0 ? bp[ib].PAx : (d == 1 ? bp[ib].PAy : bp[ib].PAz);
         const R QC = d == 0 ? kp[ik].PAx : (d == 1 ? kp[ik].PAy : kp[ik].PAz);
         const R u = R(2) * B00 * PQd;
-        rys_vrr<D::E, D::F>(d == 2 ? rw[D::NR + r] : R(1), PA - q * u, QC + p * u, B00, B10, B01,
-                            g2 + it * (D::E + 1) * (D::F + 1));
+        rys_vrr<D::E, D::F, D::FS>(d == 2 ? rw[D::NR + r] : R(1), PA - q * u, QC + p * u, B00, B10, B01,
+                                   g2 + it * D::GS);
       }
       rys_sync<G>();
       for (int r = 0; r < D::NR; ++r) {
         for (int it = lane; it < 3 * (D::F + 1); it += G) {
           const int d = it / (D::F + 1), f = it - d * (D::F + 1);
-          rys_bra<LA, LB, ORD, D::F>(g2 + (r * 3 + d) * (D::E + 1) * (D::F + 1) + f, d == 0 ? ABx : (d == 1 ? ABy : ABz),
-                                     wa, wb, bv + d * D::NBV * D::NB * (D::F + 1) + f);
+          rys_bra<LA, LB, ORD, D::FS>(g2 + (r * 3 + d) * D::GS + f, d == 0 ? ABx : (d == 1 ? ABy : ABz), wa, wb,
+                                      bv + d * D::BS + f);
         }
         rys_sync<G>();  // also: every thread is done with the previous root's variant tables
         for (int it = lane; it < 3 * D::NB; it += G) {
           const int d = it / D::NB, ij = it - d * D::NB;
-          rys_ket<LC, LD, ORD, D::NB, 3 * D::NX>(bv + (d * D::NBV * D::NB + ij) * (D::F + 1),
-                                                 d == 0 ? CDx : (d == 1 ? CDy : CDz), wc, vt + d * D::NX + ij);
+          rys_ket<LC, LD, ORD, D::NB, D::FS, 3 * D::NX>(bv + d * D::BS + ij * D::FS,
+                                                        d == 0 ? CDx : (d == 1 ? CDy : CDz), wc, vt + d * D::NX + ij);
         }
         rys_sync<G>();
         for (int e = lane; e < D::NCART; e += G) {
@@ -246,22 +247,8 @@ __global__ void __launch_bounds__(BLOCK) rys_deriv_kernel(GradArgs<R> a, RysOut 
 #pragma unroll
         for (int x = 0; x < 45; ++x) h45[x] = acc[x];
       rys_sync<G>();
-      // the 12 x 12 block over centres A, B, C, D, a thread per entry; D rows and columns are minus
-      // the sums of the others
       const int at[4] = {P.atom_a, P.atom_b, Q.atom_a, Q.atom_b};
-      if (live)
-        for (int t = lane; t < 144; t += G) {
-          const int r = t / 12, s = t - 12 * r;
-          const int X = r / 3, i = r - 3 * X, Y = s / 3, j = s - 3 * Y;
-          double v = 0.0;
-          for (int u = X < 3 ? X : 0; u < (X < 3 ? X + 1 : 3); ++u)
-            for (int w = Y < 3 ? Y : 0; w < (Y < 3 ? Y + 1 : 3); ++w) {
-              const int m = 3 * u + i, n = 3 * w + j;
-              v += double(h45[m < n ? rys_tri(m, n) : rys_tri(n, m)]);
-            }
-          if ((X == 3) != (Y == 3)) v = -v;
-          if (v != 0.0) atomicAdd(o.hess + (size_t)(3 * at[X] + i) * (3 * o.natoms) + 3 * at[Y] + j, v);
-        }
+      if (live) hess_add_block(h45, at, o.hess, 3 * o.natoms, lane, G);
     }
     rys_sync<G>();
   }
@@ -277,9 +264,9 @@ __global__ void __launch_bounds__(BLOCK) rys_deriv_kernel(GradArgs<R> a, RysOut 
 template <typename D, typename R, int G>
 constexpr int rys_block() {
   return G > 32 ? G
-                : (128 / G * D::kGroup * (int)sizeof(R) <= 72 * 1024
+                : (128 / G * D::group(G) * (int)sizeof(R) <= 72 * 1024
                        ? 128
-                       : (64 / G * D::kGroup * (int)sizeof(R) <= 72 * 1024 ? 64 : 32));
+                       : (64 / G * D::group(G) * (int)sizeof(R) <= 72 * 1024 ? 64 : 32));
 }
 
 // Launches class (LA LB|LC LD) at derivative order ORD with G threads per quartet over quartets
@@ -290,7 +277,7 @@ static bool launch_rys(const GradArgs<R>& a, const RysOut& o, int pure, const in
   if (nq <= 0) return true;
   using D = RysDims<LA, LB, LC, LD, ORD>;
   constexpr int BLOCK = rys_block<D, R, G>(), GROUPS = BLOCK / G;
-  const size_t bytes = (size_t)GROUPS * D::kGroup * sizeof(R) + (size_t)D::NCART * sizeof(int) +
+  const size_t bytes = (size_t)GROUPS * D::group(G) * sizeof(R) + (size_t)D::NCART * sizeof(int) +
                        (ORD == 1 ? 3 * sizeof(double) * (size_t)o.smem_atoms : 0);
   auto k = rys_deriv_kernel<LA, LB, LC, LD, ORD, R, G, BLOCK>;
   if (bytes > 48 * 1024 && cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes) != cudaSuccess)

@@ -9,12 +9,15 @@ struct RysOut;
 
 namespace hfgpu {
 
-constexpr int kRysVariants = 3;  // threads per quartet: fewest, middle, most
+// Variants: groups of threads over shared-memory tables, fewest, middle and most threads per quartet,
+// and (kRysThree, null for the larger classes) three threads per quartet, one per direction.
+constexpr int kRysVariants = 4, kRysThree = 3;
 
 struct RysLaunchers {
   int la, lb, lc, ld;
-  int group[kRysVariants];  // threads per quartet of each variant
-  int grad_variant, hess_variant;  // default variants (grad_variant -1: straight-line code instead)
+  // defaults, -1: straight-line code instead.  A gradient class of at most three_prims primitive quartets
+  // per quartet on average runs three threads per quartet in FP64.
+  int grad_variant, three_prims, hess_variant;
   // quartets q[0, nq) on at most max_blocks blocks (0: no limit); false when the launch's shared
   // memory could not be had
   bool (*grad_d[kRysVariants])(const GradArgs<double>&, const RysOut&, int pure, const int2* q, int nq, int max_blocks,

@@ -49,13 +49,20 @@ struct RysDims {
   static constexpr int NOUT = ORD == 2 ? 45 : 9;
   static constexpr int CB = ncart_of(LB), CC = ncart_of(LC), CD = ncart_of(LD);
   static constexpr int NCART = ncart_of(LA) * CB * CC * CD;
+  // Strides are odd, so that threads on consecutive columns (f) or rows (ij) use different banks.
+  static constexpr int FS = (F + 1) | 1;              // column stride of the 2-D tables
+  static constexpr int GS = ((E + 1) * FS) | 1;       // 2-D integrals of one root and direction
+  static constexpr int BS = (NBV * NB * FS) | 1;      // bra variants of one direction
   static constexpr int kRW = 2 * NR;
-  static constexpr int kG2 = NR * 3 * (E + 1) * (F + 1);
-  static constexpr int kBV = 3 * NBV * NB * (F + 1);
+  static constexpr int kG2 = NR * 3 * GS;
+  static constexpr int kBV = 3 * BS;
   static constexpr int kVT = NV * 3 * NX;
   static constexpr int kMain = kRW + kG2 + kBV + kVT;
   static constexpr int kWork = kMain > 2 * NCART ? kMain : 2 * NCART;
-  static constexpr int kGroup = kWork + NCART + (ORD == 2 ? 46 : 0);
+  static constexpr int kUsed = kWork + NCART + (ORD == 2 ? 46 : 0);
+  // values per group of G threads: G above a multiple of 32, so that the groups of a warp working on
+  // the same place of their tables use different banks (4-byte and 8-byte values alike)
+  static constexpr int group(int G) { return kUsed + ((G - kUsed) % 32 + 32) % 32; }
 };
 
 // The packed 2-D table positions (x | y << 8 | z << 16) of Cartesian integral e of a class: ket tuple
@@ -69,15 +76,15 @@ __device__ __forceinline__ int rys_index(int e) {
   return at(a.x, b.x, c.x, d.x) | at(a.y, b.y, c.y, d.y) << 8 | at(a.z, b.z, c.z, d.z) << 16;
 }
 
-// Vertical recurrence of the 2-D integrals of one root and direction: g[e (F+1) + f].
-template <int E, int F, typename R>
+// Vertical recurrence of the 2-D integrals of one root and direction: g[e FS + f].
+template <int E, int F, int FS, typename R>
 __device__ __forceinline__ void rys_vrr(R i00, R C, R Cp, R B00, R B10, R B01, R* __restrict__ g) {
   R prev2[E + 1], prev[E + 1], cur[E + 1];
   cur[0] = i00;
 #pragma unroll
   for (int e = 1; e <= E; ++e) cur[e] = C * cur[e - 1] + (e > 1 ? R(e - 1) * B10 * cur[e - 2] : R(0));
 #pragma unroll
-  for (int e = 0; e <= E; ++e) g[e * (F + 1)] = cur[e];
+  for (int e = 0; e <= E; ++e) g[e * FS] = cur[e];
 #pragma unroll
   for (int f = 1; f <= F; ++f) {
 #pragma unroll
@@ -91,7 +98,7 @@ __device__ __forceinline__ void rys_vrr(R i00, R C, R Cp, R B00, R B10, R B01, R
       if (f > 1) v += R(f - 1) * B01 * prev2[e];
       if (e > 0) v += R(e) * B00 * prev[e - 1];
       cur[e] = v;
-      g[e * (F + 1) + f] = v;
+      g[e * FS + f] = v;
     }
   }
 }
@@ -108,20 +115,20 @@ __device__ __forceinline__ void rys_hrr(const R (&s)[N + 1], R d, R (&h)[N + 1][
       if (i + j <= N) h[i][j] = h[i + 1][j - 1] + d * h[i][j - 1];
 }
 
-// Bra variants of one (direction, f): bv[(v NB + ij) (F+1)], from the column g[e (F+1)].
-template <int LA, int LB, int ORD, int F, typename R>
+// Bra variants of one (direction, f): bv[(v NB + ij) FS], from the column g[e FS].
+template <int LA, int LB, int ORD, int FS, typename R>
 __device__ __forceinline__ void rys_bra(const R* __restrict__ g, R AB, R wa, R wb, R* __restrict__ bv) {
   constexpr int E = LA + LB + ORD, J = LB + ORD, NB = (LA + 1) * (LB + 1);
   R s[E + 1], h[E + 1][J + 1];
 #pragma unroll
-  for (int e = 0; e <= E; ++e) s[e] = g[e * (F + 1)];
+  for (int e = 0; e <= E; ++e) s[e] = g[e * FS];
   rys_hrr<E, E, J>(s, AB, h);
 #pragma unroll
   for (int i = 0; i <= LA; ++i)
 #pragma unroll
     for (int j = 0; j <= LB; ++j) {
-      const int at = (i * (LB + 1) + j) * (F + 1);
-      auto put = [&](int v, R x) { bv[v * NB * (F + 1) + at] = x; };
+      const int at = (i * (LB + 1) + j) * FS;
+      auto put = [&](int v, R x) { bv[v * NB * FS + at] = x; };
       put(0, h[i][j]);
       R A = wa * h[i + 1][j], B = wb * h[i][j + 1];
       if (i > 0) A -= R(i) * h[i - 1][j];
@@ -150,15 +157,14 @@ __device__ __forceinline__ void rys_bra(const R* __restrict__ g, R AB, R wa, R w
 
 // Ket transfer and C derivatives of one (direction, bra tuple): variant v of ket tuple kl into
 // vt[v VS + kl NB].  Variants: 0 1, 1 A, 2 B, 3 C; second order 4 AA, 5 BB, 6 CC, 7 AB, 8 AC, 9 BC.
-template <int LC, int LD, int ORD, int NB, int VS, typename R>
+template <int LC, int LD, int ORD, int NB, int FS, int VS, typename R>
 __device__ __forceinline__ void rys_ket(const R* __restrict__ bv, R CD, R wc, R* __restrict__ vt) {
-  constexpr int F = LC + LD + ORD;
   auto transfer = [&](auto cord, int v, auto out) {
     constexpr int CO = decltype(cord)::value;  // C derivatives this bra variant still takes
     constexpr int N = LC + LD + CO;
     R s[N + 1], h[N + 1][LD + 1];
 #pragma unroll
-    for (int f = 0; f <= N; ++f) s[f] = bv[v * NB * (F + 1) + f];
+    for (int f = 0; f <= N; ++f) s[f] = bv[v * NB * FS + f];
     rys_hrr<N, N, LD>(s, CD, h);
 #pragma unroll
     for (int k = 0; k <= LC; ++k)
@@ -242,3 +248,178 @@ __device__ __forceinline__ void rys_accumulate(R w, const R (&X)[NV], const R (&
   }
 }
 
+
+// ---------------------------------------------------------------------------
+// One thread per direction (hfgpu_rys3.cuh): thread d of a quartet's three owns direction d, calls it
+// x, the next one y and the previous one z.  By cyclic symmetry every thread runs the same code on
+// the Cartesian integrals with their components renamed.
+// ---------------------------------------------------------------------------
+// Index of component (lx, ly, lz = l - lx - ly) of a shell (order of gen_eri.py cart()).
+__host__ __device__ constexpr int rys_cart(int l, int lx, int ly) {
+  return (l - lx) * (l - lx + 1) / 2 + (l - lx - ly);
+}
+
+template <int LA, int LB, int LC, int LD, int ORD>
+struct Rys3Dims {
+  static constexpr int NR = (LA + LB + LC + LD + ORD) / 2 + 1;
+  static constexpr int E = LA + LB + ORD, F = LC + LD + ORD;
+  static constexpr int NB = (LA + 1) * (LB + 1), NK = (LC + 1) * (LD + 1), NX = NB * NK;
+  static constexpr int CB = ncart_of(LB), CC = ncart_of(LC), CD = ncart_of(LD);
+  static constexpr int NCART = ncart_of(LA) * CB * CC * CD;
+  static constexpr int NSH = ORD == 2 ? 4 : 1;    // variants the other two directions read: 1 (A, B, C)
+  static constexpr int NACC = ORD == 2 ? 15 : 3;  // sums of one thread
+  static constexpr int at(int i, int j, int k, int l) { return ((i * (LB + 1) + j) * (LC + 1) + k) * (LD + 1) + l; }
+  // shared memory of a warp's quartet: [roots and weights | the three directions' shared variants |
+  // three renamed copies of W]; direction strides are 1 and the quartet's stride 3 above a
+  // multiple of 16, so that consecutive threads (quartet, direction) use consecutive banks
+  static constexpr int up(int n, int r) { return n + ((r - n) % 16 + 16) % 16; }
+  static constexpr int DV = up(NSH * NX, 1), DW = up(NCART, 1);
+  static constexpr int kV = 2 * NR, kW = kV + 3 * DV;
+  static constexpr int kQuartet = up(kW + 3 * DW, 3);
+};
+
+// h[i][j] of the horizontal transfer from the column s[e] = h[e][0], j <= 4 (binomial form).
+template <typename S, typename R>
+__device__ __forceinline__ R rys_h(const S& s, R d, int i, int j) {
+  R v = s(i);
+  R c = R(1);
+#pragma unroll
+  for (int m = 1; m <= 4; ++m)
+    if (m <= j) {
+      c = c * R(j - m + 1) / R(m);
+      v = c * s(i + m) + d * v;
+    }
+  return v;
+}
+
+// Variants (numbered as in rys_ket) of one direction for bra tuple (i, j) and every ket tuple:
+// o[v][k (LD+1) + l], from the 2-D integrals g[e][f].  SECOND: all ten, else the first four.
+template <int LA, int LB, int LC, int LD, int ORD, bool SECOND, typename R>
+__device__ __forceinline__ void rys3_variants(const R (&g)[LA + LB + ORD + 1][LC + LD + ORD + 1], R AB, R CD, R wa, R wb,
+                                              R wc, int i, int j,
+                                              R (&o)[SECOND ? 10 : 4][(LC + 1) * (LD + 1)]) {
+  constexpr int F = LC + LD + ORD;
+  R u[SECOND ? 6 : 3][F + 1];
+#pragma unroll
+  for (int f = 0; f <= F; ++f) {
+    auto s = [&](int e) { return g[e][f]; };
+    auto h = [&](int a, int b) { return rys_h(s, AB, a, b); };
+    u[0][f] = h(i, j);
+    if (f <= F - 1) {
+      R A = wa * h(i + 1, j), B = wb * h(i, j + 1);
+      if (i > 0) A -= R(i) * h(i - 1, j);
+      if (j > 0) B -= R(j) * h(i, j - 1);
+      u[1][f] = A;
+      u[2][f] = B;
+    }
+    if constexpr (SECOND) {
+      if (f <= F - 2) {
+        R AA = wa * (wa * h(i + 2, j) - R(2 * i + 1) * h(i, j)), BB = wb * (wb * h(i, j + 2) - R(2 * j + 1) * h(i, j));
+        if (i > 1) AA += R(i * (i - 1)) * h(i - 2, j);
+        if (j > 1) BB += R(j * (j - 1)) * h(i, j - 2);
+        R x = wb * h(i + 1, j + 1);
+        if (j > 0) x -= R(j) * h(i + 1, j - 1);
+        R ab = wa * x;
+        if (i > 0) {
+          R y = wb * h(i - 1, j + 1);
+          if (j > 0) y -= R(j) * h(i - 1, j - 1);
+          ab -= R(i) * y;
+        }
+        u[3][f] = AA;
+        u[4][f] = BB;
+        u[5][f] = ab;
+      }
+    }
+  }
+#pragma unroll
+  for (int k = 0; k <= LC; ++k)
+#pragma unroll
+    for (int l = 0; l <= LD; ++l) {
+      const int x = k * (LD + 1) + l;
+      auto h = [&](int v, int c, int d) {
+        auto s = [&](int f) { return u[v][f]; };
+        return rys_h(s, CD, c, d);
+      };
+      auto C = [&](int v) {
+        R c = wc * h(v, k + 1, l);
+        if (k > 0) c -= R(k) * h(v, k - 1, l);
+        return c;
+      };
+      o[0][x] = h(0, k, l);
+      o[1][x] = h(1, k, l);
+      o[2][x] = h(2, k, l);
+      o[3][x] = C(0);
+      if constexpr (SECOND) {
+        o[4][x] = h(3, k, l);
+        o[5][x] = h(4, k, l);
+        R cc = wc * (wc * h(0, k + 2, l) - R(2 * k + 1) * h(0, k, l));
+        if (k > 1) cc += R(k * (k - 1)) * h(0, k - 2, l);
+        o[6][x] = cc;
+        o[7][x] = h(5, k, l);
+        o[8][x] = C(1);
+        o[9][x] = C(2);
+      }
+    }
+}
+
+// Adds the integrals whose own-direction exponents are (i, j) on the bra: o their own variants, n and
+// m the next and previous direction's shared variants by tuple, W the renamed weights.  acc: order 1
+// dA, dB, dC of the own direction; order 2 AA BB CC AB AC BC of the own direction, then (P own, Q next).
+template <int LA, int LB, int LC, int LD, int ORD, typename R>
+__device__ __forceinline__ void rys3_accumulate(const R (&o)[ORD == 2 ? 10 : 4][(LC + 1) * (LD + 1)], int i, int j,
+                                                const R* n, const R* m, const R* W, R* acc) {
+  using D = Rys3Dims<LA, LB, LC, LD, ORD>;
+#pragma unroll
+  for (int k = 0; k <= LC; ++k)
+#pragma unroll
+    for (int l = 0; l <= LD; ++l) {
+      R S0 = R(0), S1[3] = {R(0), R(0), R(0)};
+#pragma unroll
+      for (int i2 = 0; i2 <= LA; ++i2)
+#pragma unroll
+        for (int j2 = 0; j2 <= LB; ++j2)
+#pragma unroll
+          for (int k2 = 0; k2 <= LC; ++k2)
+#pragma unroll
+            for (int l2 = 0; l2 <= LD; ++l2)
+              if (i2 <= LA - i && j2 <= LB - j && k2 <= LC - k && l2 <= LD - l) {
+                const int e = ((rys_cart(LA, i, i2) * D::CB + rys_cart(LB, j, j2)) * D::CC + rys_cart(LC, k, k2)) * D::CD +
+                              rys_cart(LD, l, l2);
+                const R wm = W[e] * m[D::at(LA - i - i2, LB - j - j2, LC - k - k2, LD - l - l2)];
+                const int t = D::at(i2, j2, k2, l2);
+                S0 += n[t] * wm;
+                if constexpr (ORD == 2)
+#pragma unroll
+                  for (int Q = 0; Q < 3; ++Q) S1[Q] += n[(1 + Q) * D::NX + t] * wm;
+              }
+      const int x = k * (LD + 1) + l;
+      if constexpr (ORD == 1) {
+#pragma unroll
+        for (int P = 0; P < 3; ++P) acc[P] += o[1 + P][x] * S0;
+      } else {
+#pragma unroll
+        for (int v = 0; v < 6; ++v) acc[v] += o[4 + v][x] * S0;
+#pragma unroll
+        for (int P = 0; P < 3; ++P)
+#pragma unroll
+          for (int Q = 0; Q < 3; ++Q) acc[6 + 3 * P + Q] += o[1 + P][x] * S1[Q];
+      }
+    }
+}
+
+// Vertical recurrence of one root and direction into registers, g[e][f].
+template <int E, int F, typename R>
+__device__ __forceinline__ void rys3_vrr(R i00, R C, R Cp, R B00, R B10, R B01, R (&g)[E + 1][F + 1]) {
+  g[0][0] = i00;
+#pragma unroll
+  for (int e = 1; e <= E; ++e) g[e][0] = C * g[e - 1][0] + (e > 1 ? R(e - 1) * B10 * g[e > 1 ? e - 2 : 0][0] : R(0));
+#pragma unroll
+  for (int f = 1; f <= F; ++f)
+#pragma unroll
+    for (int e = 0; e <= E; ++e) {
+      R v = Cp * g[e][f - 1];
+      if (f > 1) v += R(f - 1) * B01 * g[e][f > 1 ? f - 2 : 0];
+      if (e > 0) v += R(e) * B00 * g[e > 0 ? e - 1 : 0][f - 1];
+      g[e][f] = v;
+    }
+}

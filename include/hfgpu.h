@@ -138,9 +138,9 @@ int hfgpu_grad2e_uhf_backward(hfgpu_handle* h, const double* Da, const double* D
  * FP64 only; single-molecule handles (HFGPU_ERR_UNSUPPORTED for a batched handle). */
 int hfgpu_hess2e(hfgpu_handle* h, const double* D, double scale, double* hess);
 int hfgpu_hess2e_uhf(hfgpu_handle* h, const double* Da, const double* Db, double scale, double* hess);
-/* Launch form of the Hessian classes: -1 (default) the faster one measured per class, a group of
- * threads per quartet by Rys quadrature for most and one thread per quartet on straight-line
- * register code for (ss|ss), (ps|ss) and (ds|ss); 0 one thread per quartet on global scratch
+/* Launch form of the Hessian classes: -1 (default) the fastest one measured per class, Rys quadrature
+ * with three threads per quartet, or a group of threads for the larger classes, and one thread per
+ * quartet on straight-line register code for (ss|ss); 0 one thread per quartet on global scratch
  * everywhere, 1 Rys quadrature with the class's largest group of threads per quartet everywhere,
  * 2 with its smallest group, 3 the straight-line form wherever the class has it ((ss|ss), (ps|ss),
  * (ps|ps), (pp|ss), (pp|ps), (ds|ss), (ds|ps), (dp|ss); the default elsewhere).  The results agree

@@ -6,7 +6,8 @@ large T, contracted, A = B) the 45 second-derivative entries equal the one-threa
 same class (gen_eri.gen_hess_table, themselves pinned to the reference by the GPU tests).  Both
 sums are of a few thousand products of values up to ~10 times their result, so 1e-11 of the largest
 entry bounds their rounding.  The gradient is checked against the Hessian by central differences
-(h = 1e-4: truncation and rounding both near 1e-8 of the largest entry; 1e-6 is asked).
+(h = 1e-4: truncation and rounding both near 1e-8 of the largest entry; 1e-6 is asked).  The form with
+one thread per direction (csrc/hfgpu_rys3.cuh) equals the group form to 1e-11 in both orders.
 """
 import importlib.util
 import os
@@ -62,19 +63,19 @@ void rys_run(const Shells& s, const double* W, double* out) {
       for (int it = 0; it < 3 * D::NR; ++it) {
         const int r = it / 3, d = it % 3;
         const double B00 = 0.5 * rw[r] * ipq, u = 2 * B00 * PQ[d];
-        rys_vrr<D::E, D::F>(d == 2 ? rw[D::NR + r] : 1.0, PA[d] - q * u, QC[d] + p * u, B00, P.ip * (0.5 - B00 * q),
-                            Q.ip * (0.5 - B00 * p), g2.data() + it * (D::E + 1) * (D::F + 1));
+        rys_vrr<D::E, D::F, D::FS>(d == 2 ? rw[D::NR + r] : 1.0, PA[d] - q * u, QC[d] + p * u, B00, P.ip * (0.5 - B00 * q),
+                            Q.ip * (0.5 - B00 * p), g2.data() + it * D::GS);
       }
       for (int r = 0; r < D::NR; ++r) {
         for (int it = 0; it < 3 * (D::F + 1); ++it) {
           const int d = it / (D::F + 1), f = it % (D::F + 1);
-          rys_bra<LA, LB, ORD, D::F>(g2.data() + (r * 3 + d) * (D::E + 1) * (D::F + 1) + f, s.A[d] - s.B[d],
-                                     2 * s.a[ib], 2 * s.b[ib], bv.data() + d * D::NBV * D::NB * (D::F + 1) + f);
+          rys_bra<LA, LB, ORD, D::FS>(g2.data() + (r * 3 + d) * D::GS + f, s.A[d] - s.B[d], 2 * s.a[ib], 2 * s.b[ib],
+                                      bv.data() + d * D::BS + f);
         }
         for (int it = 0; it < 3 * D::NB; ++it) {
           const int d = it / D::NB, ij = it % D::NB;
-          rys_ket<LC, LD, ORD, D::NB, 3 * D::NX>(bv.data() + (d * D::NBV * D::NB + ij) * (D::F + 1),
-                                                 s.C[d] - s.D[d], 2 * s.c[ik], vt.data() + d * D::NX + ij);
+          rys_ket<LC, LD, ORD, D::NB, D::FS, 3 * D::NX>(bv.data() + d * D::BS + ij * D::FS, s.C[d] - s.D[d], 2 * s.c[ik],
+                                                        vt.data() + d * D::NX + ij);
         }
         for (int e = 0; e < D::NCART; ++e) {
           const int t = rys_index<LA, LB, LC, LD>(e);
@@ -89,6 +90,71 @@ void rys_run(const Shells& s, const double* W, double* out) {
       }
     }
   for (int x = 0; x < D::NOUT; ++x) out[x] = acc[x];
+}
+
+// the same by the three threads, one per direction, of hfgpu_rys3.cuh
+template <int LA, int LB, int LC, int LD, int ORD>
+void rys3_run(const Shells& s, const double* W, double* out) {
+  using D = Rys3Dims<LA, LB, LC, LD, ORD>;
+  std::vector<double> rw(2 * D::NR);
+  double acc[3][D::NACC] = {{0.0}};
+  auto renamed = [&](int d, int e) {  // weight of the integral whose exponents along d, d+1, d+2 are e's
+    auto back = [&](int l, int c) {
+      const int3 v = rys_comp(l, c);
+      return d == 0 ? c : (d == 1 ? rys_cart(l, v.z, v.x) : rys_cart(l, v.y, v.z));
+    };
+    return W[((back(LA, e / (D::CB * D::CC * D::CD)) * D::CB + back(LB, e / (D::CC * D::CD) % D::CB)) * D::CC +
+              back(LC, e / D::CD % D::CC)) * D::CD + back(LD, e % D::CD)];
+  };
+  std::vector<double> Wd[3];
+  for (int d = 0; d < 3; ++d)
+    for (int e = 0; e < D::NCART; ++e) Wd[d].push_back(renamed(d, e));
+  for (int ib = 0; ib < 2; ++ib)
+    for (int ik = 0; ik < 2; ++ik) {
+      PrimPair<double> P, Q;
+      make(P, s.a[ib], s.b[ib], s.A, s.B);
+      make(Q, s.c[ik], s.d[ik], s.C, s.D);
+      const double p = P.p, q = Q.p, ipq = 1.0 / (p + q);
+      const double PQ[3] = {P.Px - Q.Px, P.Py - Q.Py, P.Pz - Q.Pz};
+      const double PA[3] = {P.PAx, P.PAy, P.PAz}, QC[3] = {Q.PAx, Q.PAy, Q.PAz};
+      const double T = p * q * ipq * (PQ[0] * PQ[0] + PQ[1] * PQ[1] + PQ[2] * PQ[2]);
+      const double pre = P.Kp * Q.Kp * std::sqrt(ipq), wa = 2 * s.a[ib], wb = 2 * s.b[ib], wc = 2 * s.c[ik];
+      for (int v = 0; v < 2 * D::NR; ++v) rw[v] = rys_value<D::NR>(rys_data, T, v) * (v < D::NR ? 1.0 : pre);
+      for (int r = 0; r < D::NR; ++r) {
+        std::vector<double> V(3 * D::DV);
+        double g[3][D::E + 1][D::F + 1];
+        for (int d = 0; d < 3; ++d) {
+          const double B00 = 0.5 * rw[r] * ipq, u = 2 * B00 * PQ[d];
+          rys3_vrr<D::E, D::F>(d == 2 ? rw[D::NR + r] : 1.0, PA[d] - q * u, QC[d] + p * u, B00,
+                               P.ip * (0.5 - B00 * q), Q.ip * (0.5 - B00 * p), g[d]);
+          for (int i = 0; i <= LA; ++i)
+            for (int j = 0; j <= LB; ++j) {
+              double w[4][D::NK];
+              rys3_variants<LA, LB, LC, LD, ORD, false>(g[d], s.A[d] - s.B[d], s.C[d] - s.D[d], wa, wb, wc, i, j, w);
+              for (int v = 0; v < D::NSH; ++v)
+                for (int kl = 0; kl < D::NK; ++kl) V.at(d * D::DV + v * D::NX + (i * (LB + 1) + j) * D::NK + kl) = w[v][kl];
+            }
+        }
+        for (int d = 0; d < 3; ++d)
+          for (int i = 0; i <= LA; ++i)
+            for (int j = 0; j <= LB; ++j) {
+              double w[ORD == 2 ? 10 : 4][D::NK];
+              rys3_variants<LA, LB, LC, LD, ORD, ORD == 2>(g[d], s.A[d] - s.B[d], s.C[d] - s.D[d], wa, wb, wc, i, j, w);
+              rys3_accumulate<LA, LB, LC, LD, ORD>(w, i, j, V.data() + (d + 1) % 3 * D::DV, V.data() + (d + 2) % 3 * D::DV,
+                                                   Wd[d].data(), acc[d]);
+            }
+      }
+    }
+  for (int d = 0; d < 3; ++d)
+    for (int A = 0; A < 3; ++A)
+      for (int B = 0; B < 3; ++B)
+        if (ORD == 1) {
+          out[3 * A + d] = acc[d][A];
+        } else {
+          const int r = 3 * A + d, c = 3 * B + (d + 1) % 3;
+          if (A <= B) out[rys_tri(r, 3 * B + d)] = acc[d][rys_second(A, B) - 4];
+          out[r < c ? rys_tri(r, c) : rys_tri(c, r)] = acc[d][6 + 3 * A + B];
+        }
 }
 
 // largest difference of the Hessian from the op tables, and of the gradient's central differences
@@ -121,6 +187,15 @@ void rys_check(unsigned seed, double far, bool same, double* worst) {
   rys_run<LA, LB, LC, LD, 2>(s, W.data(), hr);
   for (int x = 0; x < 45; ++x) mx = std::max(mx, std::fabs(ht[x]));
   for (int x = 0; x < 45; ++x) worst[0] = std::max(worst[0], std::fabs(ht[x] - hr[x]) / mx);
+  if constexpr (NC <= 81) {
+    rys3_run<LA, LB, LC, LD, 2>(s, W.data(), ht);
+    for (int x = 0; x < 45; ++x) worst[2] = std::max(worst[2], std::fabs(ht[x] - hr[x]) / mx);
+    rys_run<LA, LB, LC, LD, 1>(s, W.data(), gp);
+    rys3_run<LA, LB, LC, LD, 1>(s, W.data(), gm);
+    double gx = 0;
+    for (int x = 0; x < 9; ++x) gx = std::max(gx, std::fabs(gp[x]));
+    for (int x = 0; x < 9; ++x) worst[2] = std::max(worst[2], std::fabs(gp[x] - gm[x]) / gx);
+  }
   const double h = 1e-4;
   for (int r = 0; r < 9; ++r) {
     double* X[3] = {s.A, s.B, s.C};
@@ -140,7 +215,7 @@ void rys_check(unsigned seed, double far, bool same, double* worst) {
 """
 
 
-@pytest.mark.parametrize("cls", [(0, 0, 0, 0), (1, 0, 0, 0), (1, 1, 1, 0), (2, 0, 1, 1), (2, 1, 0, 0), (2, 1, 2, 0),
+@pytest.mark.parametrize("cls", [(0, 0, 0, 0), (1, 0, 0, 0), (1, 1, 1, 0), (1, 1, 1, 1), (2, 0, 1, 1), (2, 1, 0, 0), (2, 1, 2, 0),
                                  (2, 2, 1, 0), (2, 2, 2, 2)], ids=lambda c: "".join("spd"[x] for x in c))
 def test_rys_derivatives_match_the_op_tables(tmp_path, cls):
     gxx = shutil.which("g++")
@@ -158,15 +233,16 @@ def test_rys_derivatives_match_the_op_tables(tmp_path, cls):
     table, _ = _gen_eri().gen_hess_table(*cls)
     t = "".join(map(str, cls))
     args = ", ".join(map(str, cls))
-    main = ["int main() {", "  double w[2] = {0, 0};"]
+    main = ["int main() {", "  double w[3] = {0, 0, 0};"]
     for seed, far, same in ((1, 0.0, "false"), (2, 1.0, "true"), (3, 3.0, "false")):
         main.append(f"  rys_check<{args}, HessTable{t}>({seed}, {far}, {same}, w);")
-    main += ['  std::printf("%.3e %.3e\\n", w[0], w[1]);', "}"]
+    main += ['  std::printf("%.3e %.3e %.3e\\n", w[0], w[1], w[2]);', "}"]
     src = tmp_path / "rys.cpp"
     src.write_text("\n".join([STUB, "#include <vector>", table, EXEC, DRIVER] + main))
     exe = tmp_path / "rys"
     subprocess.run([gxx, "-std=c++17", "-O1", "-fsanitize=address", "-I", str(tmp_path), str(src), "-o", str(exe)],
                    check=True)
-    hess, grad = map(float, subprocess.run([str(exe)], check=True, capture_output=True, text=True).stdout.split())
+    hess, grad, three = map(float, subprocess.run([str(exe)], check=True, capture_output=True, text=True).stdout.split())
     assert hess < 1e-11, hess
     assert grad < 1e-6, grad
+    assert three < 1e-11, three
