@@ -79,8 +79,11 @@ __device__ __forceinline__ float rsqrt_t<float>(float x) { return rsqrtf(x); }
 //                  F_{m-1} = (2T F_m + e^-T) / (2m - 1), where (FP64) e^-T = e^-T_k e^(T_k - T)
 //                  with e^-T_k tabulated and e^d, |d| <= h/2, from its degree-8 Taylor
 //                  polynomial (remainder below (h/2)^9 / 9! = 5e-18 relative);
-//   T >= BOYS_TMAX: F_0 = sqrt(pi/T)/2 (erf(sqrt T) = 1 to double precision there)
-//                  and the upward recursion F_{m+1} = ((2m+1) F_m - e^-T) / (2T).
+//   T >= BOYS_TMAX: F_0 = sqrt(pi/T)/2 (erf(sqrt T) = 1 to double precision there); FP64
+//                  F_M = (2M-1)!!/2^(M+1) sqrt(pi) T^-(M+1/2) and the same downward recursion with
+//                  e^-T = 0, so that the lanes of a warp on both sides part only for F_M (a library
+//                  exponential on the far side made the anthracene J/K classes up to (pp|ps) 6-10% slower); FP32 the
+//                  upward recursion F_{m+1} = ((2m+1) F_m - e^-T) / (2T).
 // Table layout: one row of 8 values per (order M, grid point k), rows of one order
 // contiguous.  FP64 row: F_{M+j}(T_k) / j!, j = 0..6, then e^-T_k (64 bytes, four 16-byte
 // loads give the whole expansion); FP32 row: F_{M+j}(T_k) / j!, j = 0..3, then e^-T_k and
@@ -88,37 +91,39 @@ __device__ __forceinline__ float rsqrt_t<float>(float x) { return rsqrtf(x); }
 // series F_m(T) = e^-T sum_i (2T)^i / ((2m+1)(2m+3)...(2m+2i+1)) in long double.
 // ---------------------------------------------------------------------------
 #define BOYS_H 0.1
-#define BOYS_NGRID 361           // T_k = 0 .. 36
-#define BOYS_TMAX 36.0
+// Grid points (T_k = 0 .. 56 in FP64, 36 in FP32) and the end of the table's use.  FP64, order M: the T
+// from which e^-T / 2T is below 2e-14 of F_M (below 2e-15 up to M = 6), so that the asymptotic side
+// needs no exponential.
+#define BOYS_NGRID_D 561
+#define BOYS_NGRID_F 361
+#define BOYS_TMAX_F 36.0
+__host__ __device__ constexpr double boys_tmax_d(int M) {
+  return M == 0 ? 36.0 : (M == 1 ? 38.0 : (M == 2 ? 40.0 : (M <= 4 ? 45.0 : (M <= 6 ? 50.0 : (M <= 8 ? 53.0 : 56.0)))));
+}
+template <typename R>
+__host__ __device__ constexpr int boys_ngrid() {
+  return sizeof(R) == 8 ? BOYS_NGRID_D : BOYS_NGRID_F;
+}
 #define BOYS_MMAX 10             // orders M = 0 .. 10 have rows
 #define BOYS_NM 18               // m = 0 .. 17 computed on the host (M <= 10 plus 7 Taylor terms)
 #define BOYS_ROW 8               // values per row
 
 template <typename R>
 struct BoysTable {
-  const R* __restrict__ tab;  // [BOYS_MMAX + 1][BOYS_NGRID][BOYS_ROW]
+  const R* __restrict__ tab;  // [BOYS_MMAX + 1][boys_ngrid<R>()][BOYS_ROW]
 
   template <int M>
   __device__ __forceinline__ void eval(R T, R pre, R* F) const {
     static_assert(M <= BOYS_MMAX, "Boys order beyond the table");
-    if (T < R(BOYS_TMAX)) {
-      int k;
-      R d;  // -(T - T_k)
-      if constexpr (sizeof(R) == 8) {
+    if constexpr (sizeof(R) == 8) {
+      double f, e;
+      if (T < boys_tmax_d(M)) {
         // nearest grid index without int/float conversions (they go through the narrow XU
         // pipe): adding 1.5 * 2^52 leaves round(T / h) in the low mantissa bits
         const double sh = T * 10.0 + 6755399441055744.0;
-        k = __double2loint(sh);
-        d = (sh - 6755399441055744.0) * BOYS_H - T;
-      } else {
-        k = __float2int_rn(T * R(10));
-        d = R(k) * R(BOYS_H) - T;
-      }
-      const R* row = tab + ((size_t)M * BOYS_NGRID + k) * BOYS_ROW;
-      R f;
-      R ek;  // e^-T_k
-      if constexpr (sizeof(R) == 8) {
-        const double2* r = reinterpret_cast<const double2*>(row);
+        const int k = __double2loint(sh);
+        const double d = (sh - 6755399441055744.0) * BOYS_H - T;  // -(T - T_k)
+        const double2* r = reinterpret_cast<const double2*>(tab + ((size_t)M * BOYS_NGRID_D + k) * BOYS_ROW);
         const double2 r0 = r[0], r1 = r[1], r2 = r[2], r3 = r[3];
         f = r3.x;
         f = r2.y + f * d;
@@ -127,42 +132,49 @@ struct BoysTable {
         f = r1.x + f * d;
         f = r0.y + f * d;
         f = r0.x + f * d;
-        ek = r3.y;
+        if constexpr (M > 0) {
+          double x = 1.0 / 40320.0;
+          x = 1.0 / 5040.0 + d * x;
+          x = 1.0 / 720.0 + d * x;
+          x = 1.0 / 120.0 + d * x;
+          x = 1.0 / 24.0 + d * x;
+          x = 1.0 / 6.0 + d * x;
+          x = 0.5 + d * x;
+          x = 1.0 + d * x;
+          x = 1.0 + d * x;
+          e = r3.y * x;
+        }
       } else {
-        const float4* r = reinterpret_cast<const float4*>(row);
-        const float4 r0 = r[0];
-        f = r0.w;
-        f = r0.z + f * d;
-        f = r0.y + f * d;
-        f = r0.x + f * d;
-        ek = R(0);
+        const double rt = rsqrt(T), it = rt * rt;
+        f = 0.88622692545275801365 * rt;  // sqrt(pi)/2 / sqrt(T)
+#pragma unroll
+        for (int m = 0; m < M; ++m) f *= (m + 0.5) * it;
+        e = 0.0;
       }
       F[M] = f;
       if constexpr (M > 0) {
-        R e;
-        if constexpr (sizeof(R) == 8) {
-          R x = R(1.0 / 40320.0);
-          x = R(1.0 / 5040.0) + d * x;
-          x = R(1.0 / 720.0) + d * x;
-          x = R(1.0 / 120.0) + d * x;
-          x = R(1.0 / 24.0) + d * x;
-          x = R(1.0 / 6.0) + d * x;
-          x = R(0.5) + d * x;
-          x = R(1.0) + d * x;
-          x = R(1.0) + d * x;
-          e = ek * x;
-        } else {
-          (void)ek;
-          e = exp_t<R>(-T);
-        }
-        const R t2 = T + T;
+        const double t2 = T + T;
+#pragma unroll
+        for (int m = M; m > 0; --m) F[m - 1] = (t2 * F[m] + e) * (1.0 / (2 * m - 1));
+      }
+    } else if (T < R(BOYS_TMAX_F)) {
+      const int k = __float2int_rn(T * R(10));
+      const R d = R(k) * R(BOYS_H) - T;
+      const float4 r0 = *reinterpret_cast<const float4*>(tab + ((size_t)M * BOYS_NGRID_F + k) * BOYS_ROW);
+      R f = r0.w;
+      f = r0.z + f * d;
+      f = r0.y + f * d;
+      f = r0.x + f * d;
+      F[M] = f;
+      if constexpr (M > 0) {
+        const R e = exp_t<R>(-T), t2 = T + T;
 #pragma unroll
         for (int m = M; m > 0; --m) F[m - 1] = (t2 * F[m] + e) * R(1.0 / (2 * m - 1));
       }
     } else {
       const R rt = rsqrt_t<R>(T);
       const R it = rt * rt;
-      F[0] = R(0.88622692545275801365) * rt;  // sqrt(pi)/2 / sqrt(T)
+      F[0] = R(0.88622692545275801365) * rt;
       if constexpr (M > 0) {
         const R e = exp_t<R>(-T);
         const R h = R(0.5) * it;
@@ -190,8 +202,8 @@ __host__ __device__ constexpr int npure_of(int L) { return 2 * L + 1; }
 // 0..3).  Global layout: per order, the planes back to back (BOYS_PLANE_BYTES(R) bytes).
 // ---------------------------------------------------------------------------
 #define BOYS_PLANES_D 4
-#define BOYS_PLANE_BYTES_D (BOYS_PLANES_D * BOYS_NGRID * 16)  // 23104 bytes per FP64 order
-#define BOYS_PLANE_BYTES_F (BOYS_NGRID * 16)                  // 5776 bytes per FP32 order
+#define BOYS_PLANE_BYTES_D (BOYS_PLANES_D * BOYS_NGRID_D * 16)  // 35904 bytes per FP64 order
+#define BOYS_PLANE_BYTES_F (BOYS_NGRID_F * 16)                // 5776 bytes per FP32 order
 
 template <typename R>
 __host__ __device__ constexpr int boys_plane_bytes() {
@@ -205,21 +217,16 @@ struct BoysShared {
   template <int M>
   __device__ __forceinline__ void eval(R T, R pre, R* F) const {
     static_assert(M == MS, "the staged table holds one order");
-    if (T < R(BOYS_TMAX)) {
-      int k;
-      R d;
-      if constexpr (sizeof(R) == 8) {
+    if constexpr (sizeof(R) == 8) {
+      double f, e;
+      if (T < boys_tmax_d(M)) {
+        // nearest grid index without int/float conversions (they go through the narrow XU
+        // pipe): adding 1.5 * 2^52 leaves round(T / h) in the low mantissa bits
         const double sh = T * 10.0 + 6755399441055744.0;
-        k = __double2loint(sh);
-        d = (sh - 6755399441055744.0) * BOYS_H - T;
-      } else {
-        k = __float2int_rn(T * R(10));
-        d = R(k) * R(BOYS_H) - T;
-      }
-      R f, ek;
-      if constexpr (sizeof(R) == 8) {
+        const int k = __double2loint(sh);
+        const double d = (sh - 6755399441055744.0) * BOYS_H - T;  // -(T - T_k)
         const double2* P = reinterpret_cast<const double2*>(tab);
-        const double2 r0 = P[k], r1 = P[BOYS_NGRID + k], r2 = P[2 * BOYS_NGRID + k], r3 = P[3 * BOYS_NGRID + k];
+        const double2 r0 = P[k], r1 = P[BOYS_NGRID_D + k], r2 = P[2 * BOYS_NGRID_D + k], r3 = P[3 * BOYS_NGRID_D + k];
         f = r3.x;
         f = r2.y + f * d;
         f = r2.x + f * d;
@@ -227,34 +234,42 @@ struct BoysShared {
         f = r1.x + f * d;
         f = r0.y + f * d;
         f = r0.x + f * d;
-        ek = r3.y;
+        if constexpr (M > 0) {
+          double x = 1.0 / 40320.0;
+          x = 1.0 / 5040.0 + d * x;
+          x = 1.0 / 720.0 + d * x;
+          x = 1.0 / 120.0 + d * x;
+          x = 1.0 / 24.0 + d * x;
+          x = 1.0 / 6.0 + d * x;
+          x = 0.5 + d * x;
+          x = 1.0 + d * x;
+          x = 1.0 + d * x;
+          e = r3.y * x;
+        }
       } else {
-        const float4 r0 = reinterpret_cast<const float4*>(tab)[k];
-        f = r0.w;
-        f = r0.z + f * d;
-        f = r0.y + f * d;
-        f = r0.x + f * d;
-        ek = R(0);
+        const double rt = rsqrt(T), it = rt * rt;
+        f = 0.88622692545275801365 * rt;  // sqrt(pi)/2 / sqrt(T)
+#pragma unroll
+        for (int m = 0; m < M; ++m) f *= (m + 0.5) * it;
+        e = 0.0;
       }
       F[M] = f;
       if constexpr (M > 0) {
-        R e;
-        if constexpr (sizeof(R) == 8) {
-          R x = R(1.0 / 40320.0);
-          x = R(1.0 / 5040.0) + d * x;
-          x = R(1.0 / 720.0) + d * x;
-          x = R(1.0 / 120.0) + d * x;
-          x = R(1.0 / 24.0) + d * x;
-          x = R(1.0 / 6.0) + d * x;
-          x = R(0.5) + d * x;
-          x = R(1.0) + d * x;
-          x = R(1.0) + d * x;
-          e = ek * x;
-        } else {
-          (void)ek;
-          e = exp_t<R>(-T);
-        }
-        const R t2 = T + T;
+        const double t2 = T + T;
+#pragma unroll
+        for (int m = M; m > 0; --m) F[m - 1] = (t2 * F[m] + e) * (1.0 / (2 * m - 1));
+      }
+    } else if (T < R(BOYS_TMAX_F)) {
+      const int k = __float2int_rn(T * R(10));
+      const R d = R(k) * R(BOYS_H) - T;
+      const float4 r0 = reinterpret_cast<const float4*>(tab)[k];
+      R f = r0.w;
+      f = r0.z + f * d;
+      f = r0.y + f * d;
+      f = r0.x + f * d;
+      F[M] = f;
+      if constexpr (M > 0) {
+        const R e = exp_t<R>(-T), t2 = T + T;
 #pragma unroll
         for (int m = M; m > 0; --m) F[m - 1] = (t2 * F[m] + e) * R(1.0 / (2 * m - 1));
       }

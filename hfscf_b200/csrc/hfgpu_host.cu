@@ -42,8 +42,9 @@ int quartet_class(int cp, int cq) { return cp * (cp + 1) / 2 + cq; }  // cp >= c
 // Taylor term, and e^-T_k.  `terms` = 7 (FP64 rows) or 4 (FP32 rows).
 template <typename R>
 std::vector<R> boys_table(int terms) {
-  std::vector<long double> F((size_t)BOYS_NGRID * BOYS_NM), ek(BOYS_NGRID);
-  for (int k = 0; k < BOYS_NGRID; ++k) {
+  constexpr int NGRID = boys_ngrid<R>();
+  std::vector<long double> F((size_t)NGRID * BOYS_NM), ek(NGRID);
+  for (int k = 0; k < NGRID; ++k) {
     const long double T = (long double)k * (long double)BOYS_H;
     for (int m = 0; m < BOYS_NM; ++m) {
       long double term = 1.0L / (2 * m + 1), sum = term;
@@ -56,10 +57,10 @@ std::vector<R> boys_table(int terms) {
     }
     ek[k] = expl(-T);
   }
-  std::vector<R> t((size_t)(BOYS_MMAX + 1) * BOYS_NGRID * BOYS_ROW, R(0));
+  std::vector<R> t((size_t)(BOYS_MMAX + 1) * NGRID * BOYS_ROW, R(0));
   for (int M = 0; M <= BOYS_MMAX; ++M)
-    for (int k = 0; k < BOYS_NGRID; ++k) {
-      R* row = &t[((size_t)M * BOYS_NGRID + k) * BOYS_ROW];
+    for (int k = 0; k < NGRID; ++k) {
+      R* row = &t[((size_t)M * NGRID + k) * BOYS_ROW];
       long double fact = 1.0L;
       for (int j = 0; j < terms; ++j) {
         if (j > 0) fact *= j;
@@ -74,16 +75,17 @@ std::vector<R> boys_table(int terms) {
 // j = 0..3 of (row[2j], row[2j+1]) over the grid points; FP32 one plane of row[0..3].
 template <typename R>
 std::vector<R> boys_planes(const std::vector<R>& rows) {
+  constexpr int NGRID = boys_ngrid<R>();
   const int per = boys_plane_bytes<R>() / (int)sizeof(R);  // values per order
   std::vector<R> t((size_t)(BOYS_MMAX + 1) * per, R(0));
   for (int M = 0; M <= BOYS_MMAX; ++M)
-    for (int k = 0; k < BOYS_NGRID; ++k) {
-      const R* row = &rows[((size_t)M * BOYS_NGRID + k) * BOYS_ROW];
+    for (int k = 0; k < NGRID; ++k) {
+      const R* row = &rows[((size_t)M * NGRID + k) * BOYS_ROW];
       R* o = &t[(size_t)M * per];
       if (sizeof(R) == 8) {
         for (int j = 0; j < BOYS_PLANES_D; ++j) {
-          o[((size_t)j * BOYS_NGRID + k) * 2 + 0] = row[2 * j];
-          o[((size_t)j * BOYS_NGRID + k) * 2 + 1] = row[2 * j + 1];
+          o[((size_t)j * NGRID + k) * 2 + 0] = row[2 * j];
+          o[((size_t)j * NGRID + k) * 2 + 1] = row[2 * j + 1];
         }
       } else {
         for (int j = 0; j < 4; ++j) o[(size_t)k * 4 + j] = row[j];
