@@ -59,7 +59,8 @@ def _compile(src, verbose):
                  os.path.join(CSRC, "hfgpu_hess_kernels.cuh"), os.path.join(CSRC, "hfgpu_hess_launch.h")]
     elif base.startswith("rys_"):
         deps += [os.path.join(GEN, "rys_layout.cuh"), os.path.join(CSRC, "hfgpu_rys.cuh"),
-                 os.path.join(CSRC, "hfgpu_rys3.cuh"), os.path.join(CSRC, "hfgpu_hess_kernels.cuh"),
+                 os.path.join(CSRC, "hfgpu_rys3.cuh"), os.path.join(CSRC, "hfgpu_rys_jk.cuh"),
+                 os.path.join(CSRC, "hfgpu_hess_kernels.cuh"),
                  os.path.join(CSRC, "hfgpu_rys_math.cuh"),
                  os.path.join(CSRC, "hfgpu_rys_launch.h")]
     else:  # hand-written sources: every hand-written header counts

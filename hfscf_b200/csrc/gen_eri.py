@@ -777,6 +777,15 @@ def cap_blocks(vrr_values):
     return 0
 
 
+def block_default(c):
+    """Threads per block of the thread-per-quartet form: 128, but smaller blocks for the few quartets of
+    the spilling classes (n-octane, us at 32 / 64 / 128: (dp|dp) 194 / 218 / 226, (dd|pp) 143 / 165 / 180,
+    (dd|ps) 70 / 73 / 75, (dd|ds) 63 / 59 / 98; (ps|ps) 281 / 276 / 263, (ds|ds) 74 / 72 / 61)."""
+    if c in ((2, 1, 2, 1), (2, 2, 1, 1), (2, 2, 1, 0)):
+        return 32
+    return 64 if c[:2] == (2, 2) and c[2] == 2 else 128
+
+
 STAGED_MAX_L = 4          # classes that also get the persistent form with the Boys table in shared memory
 LOWRES_MIN_VRR = 250      # classes that also get the low-residency thread variant (their registers spill)
 WARP_MIN_VRR = 250        # classes that also get a warp-per-quartet form (hfgpu_autotune picks)
@@ -897,8 +906,10 @@ static void launch_quartet_impl(const QuartetArgs<R>& a, const int2* q, int nq, 
       return;
     }}
   }}
+  // FP64: the Rys-quadrature form instead (hfgpu_rys_jk.cuh)
+  constexpr bool kWarp = CC::kWarp && sizeof(R) == 4;
   bool warp = false;
-  if constexpr (CC::kWarp) warp = nq <= a.warp_max;
+  if constexpr (kWarp) warp = nq <= a.warp_max;
   if (!warp && a.capped == 3) {{
     // low residency: the launch reserves (unused) shared memory so that at most two blocks share
     // an SM; the spilled stacks of the large-register classes then stay inside L2
@@ -920,7 +931,7 @@ static void launch_quartet_impl(const QuartetArgs<R>& a, const int2* q, int nq, 
     quartet_kernel<{la}, {lb}, {lc}, {ld}, R><<<(nq + bs - 1) / bs, bs, 0, s>>>(a, q, nq);
     return;
   }}
-  if constexpr (CC::kWarp) {{
+  if constexpr (kWarp) {{
     using Tab = typename CC::WarpTab;
     constexpr int per = warp_slots<Tab, R>();
     if (a.warp_threads == 128) {{
@@ -1000,7 +1011,7 @@ const ClassLaunchers launchers_{t} = {{{la}, {lb}, {lc}, {ld}, &launch_quartet<d
                                       ClassCode<{la}, {lb}, {lc}, {ld}>::kWarp,
                                       ClassCode<{la}, {lb}, {lc}, {ld}>::kWarpDefault,
                                       ClassCode<{la}, {lb}, {lc}, {ld}>::kCapBlocks > 0,
-                                      ClassCode<{la}, {lb}, {lc}, {ld}>::kStaged,
+                                      ClassCode<{la}, {lb}, {lc}, {ld}>::kStaged, {block},
                                       ClassCode<{la}, {lb}, {lc}, {ld}>::kLowRes}};
 }}  // namespace hfgpu
 """
@@ -1044,6 +1055,7 @@ static bool launch_hess_line(const GradArgs<double>&, const HessOut&, int, const
 
 RYS_INST_TEMPLATE = """// GENERATED by gen_eri.py -- do not edit.
 #include "../hfgpu_rys3.cuh"
+#include "../hfgpu_rys_jk.cuh"
 #include "../hfgpu_rys_launch.h"
 
 namespace hfgpu {{
@@ -1051,12 +1063,22 @@ extern const RysLaunchers rys_launchers_{t};
 const RysLaunchers rys_launchers_{t} = {{{la}, {lb}, {lc}, {ld}, {gv}, {p64}, {hv},
     {{{gd}}},
     {{{gf}}},
-    {{{hd}}}}};
+    {{{hd}}}, {qp}, {qf}}};
 }}  // namespace hfgpu
 """
 
 # Cartesian block of the classes that have the form of three threads per quartet, by order and precision
 RYS_THREE_MAX_CART = {(1, "double"): 162, (1, "float"): 0, (2, "double"): 81}
+
+
+# Undifferentiated integrals by Rys quadrature, one warp per quartet: the classes that have it and the
+# average number of primitive quartets per quartet up to which it is the default (0: only when the
+# schedule asks).  Against the fastest thread form, us: n-octane (dd|dd) 34 against 293, (dd|dp) 57
+# against 183, (dd|pp) 75 against 139, (dp|dp) 145 against 193, but (dd|ds) 72 against 57 and (dp|pp) 348
+# against 178; anthracene, with longer contractions, (dd|pp) 600 against 510 at 4.0 primitive quartets
+# and (dp|dp) 1360 against 720 at 4.1, (dd|dp) 537 against 800 at 2.0.
+RYS_QUARTET_PRIMS = {(2, 1, 1, 1): 0, (2, 1, 2, 0): 0, (2, 1, 2, 1): 3, (2, 2, 1, 1): 3, (2, 2, 2, 0): 0,
+                     (2, 2, 2, 1): 1000, (2, 2, 2, 2): 1000}
 
 
 def rys_inst(c, t):
@@ -1071,7 +1093,8 @@ def rys_inst(c, t):
 
     gv, p64, hv = rys_defaults(c)
     return RYS_INST_TEMPLATE.format(t=t, la=c[0], lb=c[1], lc=c[2], ld=c[3], gv=gv, p64=p64, hv=hv, gd=row(1, "double"),
-                                    gf=row(1, "float"), hd=row(2, "double"))
+                                    gf=row(1, "float"), hd=row(2, "double"), qp=RYS_QUARTET_PRIMS.get(c, 0),
+                                    qf=f"&launch_rys_quartet<{cl}>" if c in RYS_QUARTET_PRIMS else "nullptr")
 
 
 def rys_groups(la, lb, lc, ld):
@@ -1143,7 +1166,8 @@ def main(outdir):
         meta["grad"].append(mg)
         write_if_changed(os.path.join(outdir, f"class_{t}.cuh"), text)
         la, lb, lc, ld = c
-        write_if_changed(os.path.join(outdir, f"inst_{t}.cu"), INST_TEMPLATE.format(t=t, la=la, lb=lb, lc=lc, ld=ld))
+        write_if_changed(os.path.join(outdir, f"inst_{t}.cu"), INST_TEMPLATE.format(t=t, la=la, lb=lb, lc=lc, ld=ld,
+                                                                                          block=block_default(c)))
         names.append(t)
     # the adjoint Hessian: one table header and one launcher unit per class
     hnames = []

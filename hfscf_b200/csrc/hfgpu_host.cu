@@ -152,6 +152,7 @@ struct hfgpu_handle {
   // [beg, hik1) and [mid, hik2) run the warp-over-primitives kernel where the class has one
   std::vector<long long> q_beg, q_mid, q_end, q_hik1, q_hik2;
   std::vector<long long> q_prims;  // per class: primitive quartets of the Schwarz-screened quartets
+  int q_maxprims[21 * 4] = {0};    // per class and list segment: most primitive quartets of one quartet
   int part = 0, nparts = 1;        // partition of every quartet list (hfgpu_set_partition)
   // classes of a J/K build / a gradient on the auxiliary streams concurrently (0) or one after
   // another on one of them (1); chosen by the autotuners on whole builds
@@ -209,9 +210,9 @@ struct hfgpu_handle {
 
   hfgpu_handle() : q_beg(21), q_mid(21), q_end(21), q_hik1(21), q_hik2(21), q_prims(21) {
     for (int c = 0; c < 21; ++c) {
-      sched_block[c] = 64;
-      sched_primwarp[c] = 0;
-      sched_warp[c] = c < hfgpu::kNumClasses && hfgpu::kClassLaunchers[c]->warp_default ? -1 : 0;
+      sched_block[c] = c < hfgpu::kNumClasses ? hfgpu::kClassLaunchers[c]->block_default : 64;
+      sched_primwarp[c] = -1;
+      sched_warp[c] = c < hfgpu::kNumClasses && hfgpu::kClassLaunchers[c]->has_warp ? -1 : 0;
       sched_cap[c] = 0;
       grad_form[c] = -1;
       hess_cls_form[c] = -1;
@@ -226,14 +227,70 @@ int fail(hfgpu_handle* h, int code, const std::string& msg) {
   return code;
 }
 
-// warp_max of QuartetArgs for class c under the handle's schedule
+// warp_max of QuartetArgs (the FP32 op-table forms) for class c under the handle's schedule
 int class_warp_max(const hfgpu_handle* h, int c) {
   const int w = h->sched_warp[c];
-  return w < 0 ? h->opts.warp_max_quartets : (w ? INT_MAX : -1);
+  if (w < 0) return hfgpu::kClassLaunchers[c]->warp_default ? h->opts.warp_max_quartets : -1;
+  return w ? INT_MAX : -1;
 }
 
 // threads per quartet of that form: schedule entry 2 = one block of 128 threads per quartet
 int class_warp_threads(const hfgpu_handle* h, int c) { return h->sched_warp[c] == 2 ? 128 : 32; }
+
+// Whether an FP64 launch of nq quartets of class c runs one warp per quartet by Rys quadrature:
+// schedule entry 1 or 2; by default the classes and average primitive-quartet counts where it measured
+// faster than one thread per quartet (rys_jk_prims in gen_eri.py), up to opts.warp_max_quartets.
+bool use_rys_quartet(const hfgpu_handle* h, int c, long long nq) {
+  const hfgpu::RysLaunchers* Y = hfgpu::kRysLaunchers[c];
+  if (!Y->quartet) return false;
+  const int w = h->sched_warp[c];
+  if (w >= 0) return w > 0;
+  return nq <= h->opts.warp_max_quartets &&
+         h->q_prims[c] <= Y->quartet_prims * std::max<double>(1.0, double(h->q_end[c] - h->q_beg[c]));
+}
+
+// FP64 launch of class c over quartets q[0, nq); false when its shared memory could not be had.
+bool launch_quartet_d(const hfgpu_handle* h, int c, const QuartetArgs<double>& qa, const int2* q, int nq,
+                      cudaStream_t st) {
+  if (use_rys_quartet(h, c, nq)) return hfgpu::kRysLaunchers[c]->quartet(qa, h->rys_tab, q, nq, st);
+  hfgpu::kClassLaunchers[c]->quartet_d(qa, q, nq, st);
+  return true;
+}
+
+// Lanes per quartet for a launch of nq quartets of class c's list segment seg (one of the
+// many-primitive segments): the schedule's, or, by default (-1), 0 (one thread) or 4 ... 32 lanes in
+// FP64 where the longest quartet's primitive loop would outlast the rest of a small launch: water in
+// cc-pVDZ, whose (ss|ss) loop runs 2025 primitive quartets, 1.59 -> 0.3 ms per build, propane in
+// 6-31G** (ps|ps) 117 -> 82 us.  Model, in us, fitted to builds of eight molecules from water to hexane:
+// one thread takes kStep per primitive quartet; G lanes take the G-th part of that, kBase, and per quartet
+// G times kLane, growing with the contracted targets that the lanes sum (digestion runs on one lane).
+// FP32 keeps one thread: another order of its sums shows in mixed-precision results.
+int primwarp_group(const hfgpu_handle* h, int c, int seg, long long nq, bool fp32) {
+  const hfgpu::ClassLaunchers* L = hfgpu::kClassLaunchers[c];
+  if (!L->has_primwarp) return 0;
+  const int w = h->sched_primwarp[c];
+  if (w >= 0) return w == 1 ? 32 : w;
+  constexpr double kStep = 0.4, kBase = 30.0, kLane = 0.06e-3;
+  constexpr long long kMostQuartets = 60000;  // one thread per quartet fills the GPU from here
+  if (fp32 || nq > kMostQuartets) return 0;
+  auto targets = [](int la, int lb) {
+    int n = 0;
+    for (int l = la; l <= la + lb; ++l) n += ncart_of(l);
+    return n;
+  };
+  const double thread = kStep * h->q_maxprims[4 * c + seg];
+  const double lane = kLane * nq * (1.0 + targets(L->la, L->lb) * targets(L->lc, L->ld) / 8.0);
+  int best = 0;
+  double t = 0.8 * thread;  // only where it clearly pays
+  for (int g = 4; g <= 32; g *= 2) {
+    const double tg = kBase + thread / g + lane * g;
+    if (tg < t) {
+      t = tg;
+      best = g;
+    }
+  }
+  return best;
+}
 
 int cuda_fail(hfgpu_handle* h, cudaError_t e, const char* where) {
   return fail(h, e == cudaErrorMemoryAllocation ? HFGPU_ERR_NOMEM : HFGPU_ERR_CUDA,
@@ -533,8 +590,8 @@ int compute_schwarz(hfgpu_handle* h) {
     qa.warp_threads = class_warp_threads(h, quartet_class(c, c));
     qa.block = h->sched_block[quartet_class(c, c)];
     qa.capped = h->sched_cap[quartet_class(c, c)];
-    const hfgpu::ClassLaunchers* L = hfgpu::kClassLaunchers[quartet_class(c, c)];
-    L->quartet_d(qa, h->d_quart.as<int2>() + b, e - b, h->stream);
+    if (!launch_quartet_d(h, quartet_class(c, c), qa, h->d_quart.as<int2>() + b, e - b, h->stream))
+      return fail(h, HFGPU_ERR_CUDA, "schwarz launch: shared memory");
     HF_CHECK_LAUNCH(h, "schwarz kernel");
   }
   HF_CUDA(h, cudaMemcpyAsync(h->pairs.data(), h->d_pairs.p, sizeof(PairInfo) * npairs, cudaMemcpyDeviceToHost, h->stream));
@@ -582,6 +639,7 @@ struct ListChunk {
   std::vector<int2> q[4];       // survivors per segment, in list order
   std::vector<int> key[4];      // bound decade * kProdSpan + primitive shape
   int maxprod[4] = {0, 0, 0, 0};
+  int maxprims[4] = {0, 0, 0, 0};  // most primitive quartets of one survivor, per segment
   long long prims = 0;          // primitive quartets of the survivors
 };
 
@@ -661,6 +719,7 @@ int build_quartets(hfgpu_handle* h) {
         c.q[sg].push_back(make_int2(P, Q));
         c.key[sg].push_back(bound_decade(b) * kProdSpan + shape);
         c.maxprod[sg] = std::max(c.maxprod[sg], shape);
+        c.maxprims[sg] = std::max(c.maxprims[sg], prod);
       }
     }
   });
@@ -737,6 +796,11 @@ int build_quartets(hfgpu_handle* h) {
     h->q_hik2[qc] = seg_base[(size_t)i * 5 + 3];
     h->q_end[qc] = seg_base[(size_t)i * 5 + 4];
     h->q_prims[qc] = 0;
+    for (int sg = 0; sg < 4; ++sg) {
+      h->q_maxprims[4 * qc + sg] = 0;
+      for (int ci = cls_chunk0[i]; ci < cls_chunk0[i + 1]; ++ci)
+        h->q_maxprims[4 * qc + sg] = std::max(h->q_maxprims[4 * qc + sg], chunks[ci].maxprims[sg]);
+    }
     for (int ci = cls_chunk0[i]; ci < cls_chunk0[i + 1]; ++ci) h->q_prims[qc] += chunks[ci].prims;
   }
   h->nquartets = total;
@@ -1235,7 +1299,6 @@ static int jk_device_impl(hfgpu_handle* h, const double* DJ, int nK, const doubl
     qf.jk.counters = cnt + 3 * c;
     qd.block = qf.block = h->sched_block[c];
     qd.capped = qf.capped = h->sched_cap[c];
-    qd.group = qf.group = h->sched_primwarp[c] == 1 ? 32 : h->sched_primwarp[c];
     qd.warp_max = qf.warp_max = class_warp_max(h, c);
     qd.warp_threads = qf.warp_threads = class_warp_threads(h, c);
     qd.staged = qf.staged = (h->sched_cap[c] == 2 && L->has_staged) ? 1 : 0;
@@ -1248,20 +1311,21 @@ static int jk_device_impl(hfgpu_handle* h, const double* DJ, int nK, const doubl
     // keeps the device-computed prefix of its bound decades: the launch gets the parts' offsets
     // and their slots of the device counts (consecutive, one per part).
     const long long pstart[5] = {b, h->q_hik1[c], m, h->q_hik2[c], e};
-    struct Range { long long lo, hi; bool fp32, many; int part0, nseg; long long off[4]; };
+    struct Range { long long lo, hi; bool fp32; int group, part0, nseg; long long off[4]; };
     Range rg[4];
     int nr = 0;
     for (int part = 0; part < 4; ++part) {
       const long long lo = pstart[part], hi = pstart[part + 1];
       const bool fp32 = precision == HFGPU_MIXED && part >= 2;
-      const bool many = (part % 2) == 0 && L->has_primwarp && h->sched_primwarp[c];
-      if (nr > 0 && rg[nr - 1].hi == lo && rg[nr - 1].fp32 == fp32 && rg[nr - 1].many == many) {
+      const int group =
+          part % 2 == 0 ? primwarp_group(h, c, part, (hi - lo + h->nparts - 1) / h->nparts, fp32) : 0;
+      if (nr > 0 && rg[nr - 1].hi == lo && rg[nr - 1].fp32 == fp32 && rg[nr - 1].group == group) {
         Range& r = rg[nr - 1];  // contiguous and the same kernel: extend
         r.off[r.nseg++] = lo - r.lo;
         r.hi = hi;
       } else {
         Range& r = rg[nr++];
-        r = Range{lo, hi, fp32, many, part, 1, {0, 0, 0, 0}};
+        r = Range{lo, hi, fp32, group, part, 1, {0, 0, 0, 0}};
       }
     }
     for (int r = 0; r < nr; ++r) {
@@ -1276,13 +1340,16 @@ static int jk_device_impl(hfgpu_handle* h, const double* DJ, int nK, const doubl
         qf.nseg = rg[r].nseg;
         qf.full_nq = nq_all;
         for (int k = 0; k < 4; ++k) qf.seg_off[k] = (int)rg[r].off[k];
-        if (!(rg[r].many && L->primwarp_f(qf, qs, nq_max, st))) L->quartet_f(qf, qs, nq_max, st);
+        qf.group = rg[r].group;
+        if (!(rg[r].group && L->primwarp_f(qf, qs, nq_max, st))) L->quartet_f(qf, qs, nq_max, st);
       } else {
         qd.dyn_nq = dyn;
         qd.nseg = rg[r].nseg;
         qd.full_nq = nq_all;
         for (int k = 0; k < 4; ++k) qd.seg_off[k] = (int)rg[r].off[k];
-        if (!(rg[r].many && L->primwarp_d(qd, qs, nq_max, st))) L->quartet_d(qd, qs, nq_max, st);
+        qd.group = rg[r].group;
+        if (!(rg[r].group && L->primwarp_d(qd, qs, nq_max, st)) && !launch_quartet_d(h, c, qd, qs, nq_max, st))
+          return fail(h, HFGPU_ERR_CUDA, "quartet launch: shared memory");
       }
       ++kernels;
     }
@@ -1785,7 +1852,8 @@ int hfgpu_eri_packed(hfgpu_handle* h, double* eri_out, long long eri_len) {
       qa.warp_threads = class_warp_threads(h, quartet_class(cp, cq));
       qa.block = h->sched_block[quartet_class(cp, cq)];
       qa.capped = h->sched_cap[quartet_class(cp, cq)];
-      hfgpu::kClassLaunchers[quartet_class(cp, cq)]->quartet_d(qa, h->d_eriq.as<int2>(), (int)list.size(), h->stream);
+      if (!launch_quartet_d(h, quartet_class(cp, cq), qa, h->d_eriq.as<int2>(), (int)list.size(), h->stream))
+        return fail(h, HFGPU_ERR_CUDA, "packed eri launch: shared memory");
       HF_CHECK_LAUNCH(h, "packed eri kernel");
       HF_CUDA(h, cudaStreamSynchronize(h->stream));
     }
@@ -2378,7 +2446,7 @@ int hfgpu_set_schedule(hfgpu_handle* h, const int* schedule) {
   if (!h || !schedule) return HFGPU_ERR_INVALID;
   for (int c = 0; c < hfgpu::kNumClasses; ++c) {
     const int bs = schedule[4 * c], pw = schedule[4 * c + 1], wp = schedule[4 * c + 2], cp = schedule[4 * c + 3];
-    if ((bs != 32 && bs != 64 && bs != 128) || (pw != 0 && pw != 1 && pw != 4 && pw != 8 && pw != 16 && pw != 32) ||
+    if ((bs != 32 && bs != 64 && bs != 128) || (pw != -1 && pw != 0 && pw != 1 && pw != 4 && pw != 8 && pw != 16 && pw != 32) ||
         wp < -1 || wp > 2 || cp < 0 || cp > 3)
       return fail(h, HFGPU_ERR_INVALID, "schedule entry out of range");
   }

@@ -859,6 +859,55 @@ __device__ __forceinline__ void warp_digest(const R* V, int NA, int NB, int NC, 
   }
 }
 
+// What a group of NT threads (a warp, or a block) does with its quartet's Cartesian block A in shared
+// memory, by mode (see use_block); Bb: scratch of the same size for the pure transform, wred: one
+// double per warp.
+template <int LA, int LB, int LC, int LD, typename R, int NT>
+__device__ __forceinline__ void group_finish(const QuartetArgs<R>& qa, const int2 pq, const PairInfo& P,
+                                             const PairInfo& Q, R* A, R* Bb, double* wred, int lane) {
+  const JKArgs<R>& a = qa.jk;
+  const R* V = A;
+  int NA = ncart_of(LA), NB = ncart_of(LB), NC = ncart_of(LC), ND = ncart_of(LD);
+  if (qa.pure) {
+    const int Ls[4] = {LA, LB, LC, LD};
+    warp_to_pure<R, NT>(A, Bb, A, Ls, lane, &V);
+    NA = npure_of(LA);
+    NB = npure_of(LB);
+    NC = npure_of(LC);
+    ND = npure_of(LD);
+  }
+  double s = 1.0;
+  if (P.sa == P.sb) s *= 0.5;
+  if (Q.sa == Q.sb) s *= 0.5;
+  if (pq.x == pq.y) s *= 0.5;
+  if (qa.mode == QMODE_JK) {
+    long long blk;
+    int nm;
+    mol_block(a.mol_off, a.mol_n, P.mol, a.n, blk, nm);
+    warp_digest<R, NT>(V, NA, NB, NC, ND, P.fa, P.fb, Q.fa, Q.fb, s, off_ptr(a.DJ, blk), a.nK, off_ptr(a.DK, blk),
+                   off_ptr(a.Jh, blk), off_ptr(a.Kh, blk), nm, lane);
+  } else if (qa.mode == QMODE_PACKED) {
+    for (int e = lane; e < NA * NB * NC * ND; e += NT) {
+      const int l = e % ND, k = (e / ND) % NC, j = (e / (ND * NC)) % NB, i = e / (ND * NC * NB);
+      qa.eri[packed_index(P.fa + i, P.fb + j, Q.fa + k, Q.fb + l)] = double(V[e]);
+    }
+  } else {
+    double m = 0.0;
+    for (int x = lane; x < NA * NB; x += NT) {
+      const int i = x / NB, j = x % NB;
+      m = fmax(m, fabs(double(V[((i * NB + j) * NC + i) * ND + j])));
+    }
+    for (int off = 16; off > 0; off >>= 1) m = fmax(m, __shfl_xor_sync(0xffffffffu, m, off));
+    if constexpr (NT > 32) {  // the block's warps through shared memory
+      if ((lane & 31) == 0) wred[lane >> 5] = m;
+      __syncthreads();
+      if (lane == 0)
+        for (int k = 1; k < NT / 32; ++k) m = fmax(m, wred[k]);
+    }
+    if (lane == 0) qa.pairs_rw[pq.x].schwarz = sqrt(m);
+  }
+}
+
 template <typename Tab, typename R>
 constexpr int warp_slots() {
   return Tab::NVSLOT + 1 + Tab::NHSLOT + 1 + 2 * Tab::NCART;
@@ -985,44 +1034,5 @@ __global__ void __launch_bounds__(128) quartet_warp_kernel(QuartetArgs<R> qa, co
   const int* outs = Tab::out();
   for (int o = lane; o < Tab::NCART; o += NT) A[o] = hs[__ldg(outs + o)];
   group_sync<NT>();
-  const R* V = A;
-  int NA = ncart_of(LA), NB = ncart_of(LB), NC = ncart_of(LC), ND = ncart_of(LD);
-  if (qa.pure) {
-    const int Ls[4] = {LA, LB, LC, LD};
-    warp_to_pure<R, NT>(A, Bb, A, Ls, lane, &V);
-    NA = npure_of(LA);
-    NB = npure_of(LB);
-    NC = npure_of(LC);
-    ND = npure_of(LD);
-  }
-  double s = 1.0;
-  if (P.sa == P.sb) s *= 0.5;
-  if (Q.sa == Q.sb) s *= 0.5;
-  if (pq.x == pq.y) s *= 0.5;
-  if (qa.mode == QMODE_JK) {
-    long long blk;
-    int nm;
-    mol_block(a.mol_off, a.mol_n, P.mol, a.n, blk, nm);
-    warp_digest<R, NT>(V, NA, NB, NC, ND, P.fa, P.fb, Q.fa, Q.fb, s, off_ptr(a.DJ, blk), a.nK, off_ptr(a.DK, blk),
-                   off_ptr(a.Jh, blk), off_ptr(a.Kh, blk), nm, lane);
-  } else if (qa.mode == QMODE_PACKED) {
-    for (int e = lane; e < NA * NB * NC * ND; e += NT) {
-      const int l = e % ND, k = (e / ND) % NC, j = (e / (ND * NC)) % NB, i = e / (ND * NC * NB);
-      qa.eri[packed_index(P.fa + i, P.fb + j, Q.fa + k, Q.fb + l)] = double(V[e]);
-    }
-  } else {
-    double m = 0.0;
-    for (int x = lane; x < NA * NB; x += NT) {
-      const int i = x / NB, j = x % NB;
-      m = fmax(m, fabs(double(V[((i * NB + j) * NC + i) * ND + j])));
-    }
-    for (int off = 16; off > 0; off >>= 1) m = fmax(m, __shfl_xor_sync(0xffffffffu, m, off));
-    if constexpr (NT > 32) {  // the block's warps through shared memory
-      if ((lane & 31) == 0) wred[lane >> 5] = m;
-      __syncthreads();
-      if (lane == 0)
-        for (int k = 1; k < NT / 32; ++k) m = fmax(m, wred[k]);
-    }
-    if (lane == 0) qa.pairs_rw[pq.x].schwarz = sqrt(m);
-  }
+  group_finish<LA, LB, LC, LD, R, NT>(qa, pq, P, Q, A, Bb, wred, lane);
 }

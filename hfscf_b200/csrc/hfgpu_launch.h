@@ -23,6 +23,7 @@ struct ClassLaunchers {
   bool warp_default;                     // ... used unless the schedule or opts say otherwise
   bool has_capped;                       // register-capped variant of the thread-per-quartet form
   bool has_staged;                       // persistent thread form with the Boys table in shared memory
+  int block_default;                     // threads per block of the thread-per-quartet form
   bool has_lowres;                       // low-residency variant of the thread form (classes that spill)
 };
 

@@ -423,3 +423,75 @@ __device__ __forceinline__ void rys3_vrr(R i00, R C, R Cp, R B00, R B10, R B01, 
       g[e][f] = v;
     }
 }
+
+// ---------------------------------------------------------------------------
+// Undifferentiated integrals (rys_quartet_kernel): a thread takes (a, c, d) component triples and all
+// components of b, whose 2-D integrals lie next to each other in the tables.
+// ---------------------------------------------------------------------------
+template <int LA, int LB, int LC, int LD>
+struct RysJKDims {
+  static constexpr int NR = (LA + LB + LC + LD) / 2 + 1, E = LA + LB, F = LC + LD;
+  static constexpr int NB = (LA + 1) * (LB + 1), NK = (LC + 1) * (LD + 1), NX = NB * NK;
+  static constexpr int CA = ncart_of(LA), CB = ncart_of(LB), CC = ncart_of(LC), CD = ncart_of(LD);
+  static constexpr int NCART = CA * CB * CC * CD, NT = CA * CC * CD;  // integrals, triples
+  static constexpr int FS = (F + 1) | 1, GS = ((E + 1) * FS) | 1, BS = (NB * FS) | 1;
+  // shared memory of a group: [roots and weights | 2-D integrals | bra-transferred | transferred], all
+  // roots at once; afterwards the Cartesian block and its transform's scratch
+  static constexpr int kRW = 2 * NR, kG2 = NR * 3 * GS, kBV = NR * 3 * BS, kVT = NR * 3 * NX;
+  static constexpr int kUsed = kRW + kG2 + kBV + kVT > 2 * NCART ? kRW + kG2 + kBV + kVT : 2 * NCART;
+  static constexpr int kGroup = kUsed | 1;
+};
+
+// Table positions (x | y << 10 | z << 20) of triple t = (a CC + c) CD + d, for b = s.
+template <int LA, int LB, int LC, int LD>
+__device__ __forceinline__ int rys_triple(int t) {
+  constexpr int CC = ncart_of(LC), CD = ncart_of(LD), NB = (LA + 1) * (LB + 1);
+  const int3 a = rys_comp(LA, t / (CC * CD)), c = rys_comp(LC, t / CD % CC), d = rys_comp(LD, t % CD);
+  auto at = [](int i, int k, int l) { return (k * (LD + 1) + l) * NB + i * (LB + 1); };
+  return at(a.x, c.x, d.x) | at(a.y, c.y, d.y) << 10 | at(a.z, c.z, d.z) << 20;
+}
+
+// Bra transfer of one column: bv[(i (LB+1) + j) FS] = h[i][j] from g[e FS].
+template <int LA, int LB, int FS, typename R>
+__device__ __forceinline__ void rys_jk_bra(const R* __restrict__ g, R AB, R* __restrict__ bv) {
+  constexpr int E = LA + LB;
+  R s[E + 1], h[E + 1][LB + 1];
+#pragma unroll
+  for (int e = 0; e <= E; ++e) s[e] = g[e * FS];
+  rys_hrr<E, E, LB>(s, AB, h);
+#pragma unroll
+  for (int i = 0; i <= LA; ++i)
+#pragma unroll
+    for (int j = 0; j <= LB; ++j) bv[(i * (LB + 1) + j) * FS] = h[i][j];
+}
+
+// Ket transfer of one bra tuple: vt[(k (LD+1) + l) NB] from the row bv[f].
+template <int LC, int LD, int NB, typename R>
+__device__ __forceinline__ void rys_jk_ket(const R* __restrict__ bv, R CD, R* __restrict__ vt) {
+  constexpr int F = LC + LD;
+  R s[F + 1], h[F + 1][LD + 1];
+#pragma unroll
+  for (int f = 0; f <= F; ++f) s[f] = bv[f];
+  rys_hrr<F, F, LD>(s, CD, h);
+#pragma unroll
+  for (int k = 0; k <= LC; ++k)
+#pragma unroll
+    for (int l = 0; l <= LD; ++l) vt[(k * (LD + 1) + l) * NB] = h[k][l];
+}
+
+// Adds one root's contribution to the CB integrals of a triple: x, y, z its rows of the tables.
+template <int LB, typename R, int CB>
+__device__ __forceinline__ void rys_jk_triple(const R* __restrict__ x, const R* __restrict__ y,
+                                              const R* __restrict__ z, R (&acc)[CB]) {
+  R X[LB + 1], Y[LB + 1], Z[LB + 1];
+#pragma unroll
+  for (int j = 0; j <= LB; ++j) {
+    X[j] = x[j];
+    Y[j] = y[j];
+    Z[j] = z[j];
+  }
+#pragma unroll
+  for (int i = 0; i <= LB; ++i)
+#pragma unroll
+    for (int j = 0; j <= i; ++j) acc[i * (i + 1) / 2 + j] += X[LB - i] * Y[i - j] * Z[j];
+}

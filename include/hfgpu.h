@@ -65,8 +65,8 @@ typedef struct {
                               with HFGPU_MIXED; default 1e-12 as for full builds: a looser 1e-10 made the
                               incremental SCF of n-octane take 44 iterations instead of 24) */
   int device;              /* CUDA device ordinal (default 0) */
-  int warp_max_quartets;   /* (dd|dp), (dd|dd): one warp per quartet when the class has at most this many
-                              quartets, one thread per quartet otherwise (default 2^30 = always; -1 = never) */
+  int warp_max_quartets;   /* classes whose default is one warp per quartet: so when the class has at most this
+                              many quartets, one thread per quartet otherwise (default 2^30 = always; -1 = never) */
   int grad_warp_max_waves;    /* gradient of (dp|dp) (dd|pp) (dd|ds) (dd|dp) (dd|dd) before any
                                  hfgpu_autotune_grad / hfgpu_set_grad_forms: > 0 (default 48) a group of
                                  threads per quartet by Rys quadrature, 0 = one thread per quartet on
@@ -302,19 +302,22 @@ int hfgpu_setup_times(const hfgpu_handle* h, double* ms);
  * hfgpu_class_stats:
  *   [0] threads per block of the thread-per-quartet form (32, 64, 128);
  *   [1] lanes per quartet of the primitive-split form used for quartets with at least 16
- *       primitive quartets (4, 8, 16, 32; 1 = 32; 0 = thread form; classes without that
- *       form ignore it);
- *   [2] 2/1/0/-1 = block-per-quartet form (128 threads per quartet) / warp-per-quartet form
- *       (four quartets per 128-thread block) for the classes that have one, (dp|pp) (dp|ds)
- *       (dp|dp) (dd|pp) (dd|ds) (dd|dp) (dd|dd) / thread forms (-1 = follow
- *       opts.warp_max_quartets with the warp form);
+ *       primitive quartets (4, 8, 16, 32; 1 = 32; 0 = thread form; -1 = by the launch's size, FP64
+ *       only; classes without that form ignore it);
+ *   [2] form of the classes (dp|pp) (dp|ds) (dp|dp) (dd|pp) (dd|ds) (dd|dp) (dd|dd): 2/1 = one warp
+ *       per quartet by Rys quadrature in FP64, and in FP32 the block-per-quartet form (128 threads per
+ *       quartet) / warp-per-quartet form (four quartets per 128-thread block) over op tables; 0 =
+ *       thread forms; -1 = the measured default: FP64 the Rys form for (dd|dp), (dd|dd) and, with few
+ *       primitive quartets per quartet, (dp|dp) and (dd|pp), FP32 the warp form for (dd|dp) and (dd|dd),
+ *       both up to opts.warp_max_quartets quartets, thread forms otherwise;
  *   [3] variant of the thread-per-quartet form: 0 plain; 1 register-capped, for more warps
  *       per SM (the small classes (ps|ss) ... (dp|ss) have one); 2 persistent, with the
  *       class's Boys table staged into shared memory by one bulk (TMA) copy per block (the
  *       classes of total angular momentum <= 4 have one); 3 at most two blocks per SM, so that
  *       the spilled registers of the large classes stay in L2 (classes with 250 or more VRR
  *       values have one); classes without the variant ignore it.
- * Default: 64, 0, -1 for (dd|dp) and (dd|dd) else 0, 0.
+ * Default: 128, -1, -1, 0, but blocks of 32 for (dp|dp) (dd|ps) (dd|pp) and of 64 for (dd|ds) (dd|dp)
+ * (dd|dd).
  * autotune: times every form of every class on the current geometry with device density D
  * (n x n; `repeats` builds per candidate, one class at a time on the handle's stream),
  * keeps the fastest; then, on whole builds, tries per class the best candidate of each other
