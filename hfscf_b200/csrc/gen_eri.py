@@ -1088,7 +1088,9 @@ def rys_inst(c, t):
 
     def row(order, real):
         fns = [f"&launch_rys<{cl}, {order}, {real}, {g}>" for g in rys_groups(*c)]
-        fns.append(f"&launch_rys3<{cl}, {order}, {real}>" if n <= RYS_THREE_MAX_CART[order, real] else "nullptr")
+        for split in (1, 10):
+            fns.append(f"&launch_rys3<{cl}, {order}, {real}, {split}>" if n <= RYS_THREE_MAX_CART[order, real]
+                       else "nullptr")
         return ", ".join(fns)
 
     gv, p64, hv = rys_defaults(c)

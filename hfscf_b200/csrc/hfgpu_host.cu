@@ -162,7 +162,7 @@ struct hfgpu_handle {
   // bucket_end[(c * 4 + seg) * kBuckets + e] is the
   // end of decade e (bound in [10^-e, 10^(1-e)), e = 0 collects bounds >= 1)
   std::vector<long long> bucket_end;
-  DevBuf d_gmax;
+  unsigned long long* counters = nullptr;  // three per class, at the head of d_half (last J/K build)
   // per geometry, for density-screened builds without a host round trip: d_launch holds per
   // (class, list segment) the segment's [lo, hi) and its decade ends (2 + kBuckets longs),
   // d_dyn the counts a build's launches process, d_first the first function of every shell
@@ -178,7 +178,7 @@ struct hfgpu_handle {
 
   DevBuf d_pairs, d_prim_d, d_prim_f, d_alpha_d, d_alpha_f, d_boys_d, d_boys_f, d_quart;
   DevBuf d_onee;  // one-electron kernels: atoms (x, y, z, Z), molecule atom ranges, Cartesian -> pure tables
-  DevBuf d_mats, d_half, d_dmax, d_counters, d_grad, d_scratch, d_eri, d_eriq;
+  DevBuf d_mats, d_half, d_dmax, d_grad, d_scratch, d_eri, d_eriq;
   long long last_launched = 0, last_skipped = 0;
   int last_kernels = 0;                 // kernel launches of the last J/K build
   double setup_ms[4] = {0, 0, 0, 0};    // last set_geometry: pairs, Schwarz, quartet lists (host), list upload
@@ -245,8 +245,12 @@ bool use_rys_quartet(const hfgpu_handle* h, int c, long long nq) {
   if (!Y->quartet) return false;
   const int w = h->sched_warp[c];
   if (w >= 0) return w > 0;
+  // few primitive quartets in all: one warp per quartet finishes first in every class ((dp|ds) of propane
+  // 36 against 55 us, of (H2O)3/cc-pVDZ 55 against 92, but 155 against 80 for the 110,000 of (H2O)8)
+  constexpr long long kFewPrims = 30000;
   return nq <= h->opts.warp_max_quartets &&
-         h->q_prims[c] <= Y->quartet_prims * std::max<double>(1.0, double(h->q_end[c] - h->q_beg[c]));
+         (h->q_prims[c] <= kFewPrims ||
+          h->q_prims[c] <= Y->quartet_prims * std::max<double>(1.0, double(h->q_end[c] - h->q_beg[c])));
 }
 
 // FP64 launch of class c over quartets q[0, nq); false when its shared memory could not be had.
@@ -262,8 +266,9 @@ bool launch_quartet_d(const hfgpu_handle* h, int c, const QuartetArgs<double>& q
 // FP64 where the longest quartet's primitive loop would outlast the rest of a small launch: water in
 // cc-pVDZ, whose (ss|ss) loop runs 2025 primitive quartets, 1.59 -> 0.3 ms per build, propane in
 // 6-31G** (ps|ps) 117 -> 82 us.  Model, in us, fitted to builds of eight molecules from water to hexane:
-// one thread takes kStep per primitive quartet; G lanes take the G-th part of that, kBase, and per quartet
-// G times kLane, growing with the contracted targets that the lanes sum (digestion runs on one lane).
+// one thread takes kStep per primitive quartet; G lanes take the G-th part of that and per quartet
+// G times kLane, growing with the contracted targets that the lanes sum (digestion runs on one lane);
+// kBase when the class also has quartets of few primitives, which then need a launch of their own.
 // FP32 keeps one thread: another order of its sums shows in mixed-precision results.
 int primwarp_group(const hfgpu_handle* h, int c, int seg, long long nq, bool fp32) {
   const hfgpu::ClassLaunchers* L = hfgpu::kClassLaunchers[c];
@@ -279,11 +284,12 @@ int primwarp_group(const hfgpu_handle* h, int c, int seg, long long nq, bool fp3
     return n;
   };
   const double thread = kStep * h->q_maxprims[4 * c + seg];
+  const bool alone = h->q_mid[c] == h->q_hik1[c] && h->q_end[c] == h->q_hik2[c];
   const double lane = kLane * nq * (1.0 + targets(L->la, L->lb) * targets(L->lc, L->ld) / 8.0);
   int best = 0;
   double t = 0.8 * thread;  // only where it clearly pays
   for (int g = 4; g <= 32; g *= 2) {
-    const double tg = kBase + thread / g + lane * g;
+    const double tg = (alone ? 0.0 : kBase) + thread / g + lane * g;
     if (tg < t) {
       t = tg;
       best = g;
@@ -837,30 +843,6 @@ int build_quartets(hfgpu_handle* h) {
   return HFGPU_OK;
 }
 
-__global__ void dmax_kernel(const int* __restrict__ first, int nshell, int n, const double* __restrict__ DJ, int nK,
-                            const double* __restrict__ DK, float* __restrict__ out) {
-  const int idx = blockIdx.x * blockDim.x + threadIdx.x;
-  if (idx >= nshell * nshell) return;
-  const int s = idx / nshell, t = idx % nshell;
-  double m = 0.0;
-  for (int i = first[s]; i < first[s + 1]; ++i)
-    for (int j = first[t]; j < first[t + 1]; ++j) {
-      if (DJ) m = fmax(m, fabs(DJ[(size_t)i * n + j]));
-      for (int k = 0; k < nK; ++k) m = fmax(m, fabs(DK[(size_t)k * n * n + (size_t)i * n + j]));
-    }
-  out[idx] = (float)m;
-}
-
-// J = Jh + Jh^T, K = Kh + Kh^T (in place into J/K outputs).
-// Largest entry of the shell-pair density maxima (non-negative floats compare as ints).
-__global__ void gmax_kernel(const float* __restrict__ dmax, int n, unsigned int* out) {
-  unsigned int m = 0;
-  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x)
-    m = max(m, __float_as_uint(dmax[i]));
-  for (int off = 16; off > 0; off >>= 1) m = max(m, __shfl_xor_sync(0xffffffffu, m, off));
-  if ((threadIdx.x & 31) == 0) atomicMax(out, m);
-}
-
 // Per launch of a density-screened build: how many quartets of its list segment can pass the
 // per-quartet test.  A segment is ordered by Schwarz-bound decade, largest first; decade e holds
 // bounds below kDecadeUpper[e], so with 4 max|D| = dm4 only the decades with
@@ -869,19 +851,52 @@ __global__ void gmax_kernel(const float* __restrict__ dmax, int n, unsigned int*
 // last such decade.  Runs on the device, so the build needs no host round trip.
 __constant__ double kDecadeUpper[18] = {1e300, 1.0,   1e-1,  1e-2,  1e-3,  1e-4,  1e-5,  1e-6,  1e-7,
                                         1e-8,  1e-9,  1e-10, 1e-11, 1e-12, 1e-13, 1e-14, 1e-15, 1e-16};
-__global__ void launch_counts_kernel(const unsigned int* __restrict__ gmax_bits, double dtol,
-                                     const long long* __restrict__ table, int nslot, int nbuckets,
-                                     int* __restrict__ dyn) {
-  const int s = blockIdx.x * blockDim.x + threadIdx.x;
-  if (s >= nslot) return;
-  const double dm4 = 4.0 * (double)__uint_as_float(*gmax_bits);
+//
+// One launch makes the table of max |D| over every shell pair (four lanes per pair), its largest entry
+// (non-negative floats compare as ints) and, in the block that finishes last, the counts: on a small
+// molecule the three launches this replaces took as long as a class kernel.  gmax and done are zero at
+// the start.
+__global__ void __launch_bounds__(128) density_bounds_kernel(const int* __restrict__ first, int nshell, int n,
+                                                             const double* __restrict__ DJ, int nK,
+                                                             const double* __restrict__ DK, float* __restrict__ out,
+                                                             unsigned int* gmax, unsigned int* done, double dtol,
+                                                             const long long* __restrict__ table, int nslot,
+                                                             int nbuckets, int* __restrict__ dyn) {
+  const long long idx = ((long long)blockIdx.x * 128 + threadIdx.x) / 4, npair = (long long)nshell * nshell;
+  const int sub = threadIdx.x & 3;
+  double m = 0.0;
+  if (idx < npair) {
+    const int s = (int)(idx / nshell), t = (int)(idx - (long long)s * nshell);
+    const int i0 = first[s], j0 = first[t], nb = first[t + 1] - j0, ne = (first[s + 1] - i0) * nb;
+    for (int e = sub; e < ne; e += 4) {
+      const size_t at = (size_t)(i0 + e / nb) * n + j0 + e % nb;
+      if (DJ) m = fmax(m, fabs(DJ[at]));
+      for (int k = 0; k < nK; ++k) m = fmax(m, fabs(DK[(size_t)k * n * n + at]));
+    }
+  }
+  unsigned int v = __float_as_uint((float)m);
+  v = max(v, __shfl_xor_sync(0xffffffffu, v, 1));
+  v = max(v, __shfl_xor_sync(0xffffffffu, v, 2));
+  if (sub == 0 && idx < npair) out[idx] = __uint_as_float(v);
+  for (int off = 4; off < 32; off <<= 1) v = max(v, __shfl_xor_sync(0xffffffffu, v, off));
+  if ((threadIdx.x & 31) == 0) atomicMax(gmax, v);
+  __shared__ bool last;
+  __threadfence();
+  __syncthreads();
+  if (threadIdx.x == 0) last = atomicAdd(done, 1u) == gridDim.x - 1;
+  __syncthreads();
+  if (!last) return;
+  __threadfence();
+  const double dm4 = 4.0 * (double)__uint_as_float(__ldcg(gmax));
   int keep = 0;
   for (int e = 0; e < nbuckets; ++e)
     if (kDecadeUpper[e] * dm4 >= dtol) keep = e + 1;
-  const long long* row = table + (size_t)s * (2 + nbuckets);
-  const long long lo = row[0], hi = row[1];
-  const long long end = keep > 0 ? min(hi, row[2 + keep - 1]) : lo;
-  dyn[s] = (int)max(0LL, end - lo);
+  for (int s = threadIdx.x; s < nslot; s += 128) {
+    const long long* row = table + (size_t)s * (2 + nbuckets);
+    const long long lo = row[0], hi = row[1];
+    const long long end = keep > 0 ? min(hi, row[2 + keep - 1]) : lo;
+    dyn[s] = (int)max(0LL, end - lo);
+  }
 }
 
 // J = Jh + Jh^T inside every molecule's block of a batched handle.
@@ -902,13 +917,16 @@ __global__ void batch_symmetrise_kernel(const double* __restrict__ h, double* __
   out[e] = h[e] + h[b + j * nm + i];
 }
 
-__global__ void symmetrise_kernel(const double* __restrict__ h, double* __restrict__ out, int n, int nmat) {
-  const int idx = blockIdx.x * blockDim.x + threadIdx.x;
-  const int tot = n * n;
-  if (idx >= tot * nmat) return;
-  const int m = idx / tot, e = idx % tot;
-  const int i = e / n, j = e % n;
-  out[idx] = h[(size_t)m * tot + i * n + j] + h[(size_t)m * tot + j * n + i];
+// J = Jh + Jh^T (skipped when J is null) and K = Kh + Kh^T of nK matrices, h = [Jh | Kh].
+__global__ void symmetrise_kernel(const double* __restrict__ h, double* __restrict__ J, double* __restrict__ K, int n,
+                                  int nK) {
+  const long long idx = (long long)blockIdx.x * blockDim.x + threadIdx.x, tot = (long long)n * n;
+  if (idx >= tot * (1 + nK)) return;
+  const int m = (int)(idx / tot), e = (int)(idx - m * tot);
+  double* out = m == 0 ? J : K + (size_t)(m - 1) * tot;
+  if (m == 0 && J == nullptr) return;
+  const int i = e / n, j = e - i * n;
+  out[e] = h[(size_t)m * tot + e] + h[(size_t)m * tot + (size_t)j * n + i];
 }
 
 // F = H + 2J - K (F may alias J).
@@ -1158,37 +1176,27 @@ static int ensure_aux(hfgpu_handle* h) {
   return HFGPU_OK;
 }
 
-// Fork: every auxiliary stream waits for the work already queued on the handle's stream.
-static int fork_streams(hfgpu_handle* h) {
+// Fork: the first `used` auxiliary streams wait for the work already queued on the handle's stream.
+static int fork_streams(hfgpu_handle* h, int used = hfgpu_handle::kAux) {
   int rc = ensure_aux(h);
   if (rc) return rc;
   HF_CUDA(h, cudaEventRecord(h->fork_ev, h->stream));
-  for (int i = 0; i < hfgpu_handle::kAux; ++i) HF_CUDA(h, cudaStreamWaitEvent(h->aux[i], h->fork_ev, 0));
+  for (int i = 0; i < used; ++i) HF_CUDA(h, cudaStreamWaitEvent(h->aux[i], h->fork_ev, 0));
   return HFGPU_OK;
 }
 
-// Join: the handle's stream waits for all auxiliary streams.
-static int join_streams(hfgpu_handle* h) {
-  for (int i = 0; i < hfgpu_handle::kAux; ++i) {
+// Join: the handle's stream waits for them.
+static int join_streams(hfgpu_handle* h, int used = hfgpu_handle::kAux) {
+  for (int i = 0; i < used; ++i) {
     HF_CUDA(h, cudaEventRecord(h->join_ev[i], h->aux[i]));
     HF_CUDA(h, cudaStreamWaitEvent(h->stream, h->join_ev[i], 0));
   }
   return HFGPU_OK;
 }
 
-// Largest classes first, each of the first kAux on its own stream, the rest
-// round-robin: the few-quartet, long-latency d classes then overlap the
-// many-quartet s/p classes instead of running alone on a handful of SMs.
-static void class_schedule(int* order, int* stream_of) {
-  for (int i = 0; i < hfgpu::kNumClasses; ++i) {
-    order[i] = hfgpu::kNumClasses - 1 - i;
-    stream_of[i] = i % hfgpu_handle::kAux;
-  }
-}
-
 static int read_counters(hfgpu_handle* h, long long* computed, long long* skipped) {
   std::vector<unsigned long long> c(3 * hfgpu::kNumClasses);
-  HF_CUDA(h, cudaMemcpy(c.data(), h->d_counters.p, sizeof(unsigned long long) * c.size(), cudaMemcpyDeviceToHost));
+  HF_CUDA(h, cudaMemcpy(c.data(), h->counters, sizeof(unsigned long long) * c.size(), cudaMemcpyDeviceToHost));
   long long a = 0, b = 0;
   for (int k = 0; k < hfgpu::kNumClasses; ++k) {
     a += (long long)c[3 * k];
@@ -1223,39 +1231,33 @@ static int jk_device_impl(hfgpu_handle* h, const double* DJ, int nK, const doubl
   const int n = h->n, ns = h->nshell;
   const size_t nn = (size_t)h->mat_total;  // n*n, or the block storage of a batched handle
   if (h->batched && nK > 1) return fail(h, HFGPU_ERR_UNSUPPORTED, "batched handles build RHF J/K (one density)");
-  HF_CUDA(h, h->d_half.ensure(sizeof(double) * nn * (1 + std::max(nK, 1))));
-  HF_CUDA(h, h->d_counters.ensure(sizeof(unsigned long long) * 3 * hfgpu::kNumClasses));
-  double* Jh = h->d_half.as<double>();
+  // one block of zeroed memory: the per-class counters, the largest density entry, the half matrices
+  constexpr size_t kHead = 3 * 21 + 1;
+  h->counters = nullptr;
+  HF_CUDA(h, h->d_half.ensure(sizeof(double) * (kHead + nn * (1 + std::max(nK, 1)))));
+  unsigned long long* cnt = h->d_half.as<unsigned long long>();
+  h->counters = cnt;
+  unsigned int* gmax = reinterpret_cast<unsigned int*>(cnt + 3 * 21);
+  double* Jh = h->d_half.as<double>() + kHead;
   double* Kh = Jh + nn;
-  HF_CUDA(h, cudaMemsetAsync(Jh, 0, sizeof(double) * nn * (1 + nK), h->stream));
-  HF_CUDA(h, cudaMemsetAsync(h->d_counters.p, 0, sizeof(unsigned long long) * 3 * hfgpu::kNumClasses, h->stream));
+  HF_CUDA(h, cudaMemsetAsync(cnt, 0, sizeof(double) * (kHead + nn * (1 + nK)), h->stream));
   int kernels = 0;
   // mixed-precision Delta-D builds screen at their own (looser) threshold; full builds never do
   const double dtol = delta && precision == HFGPU_MIXED ? h->opts.mixed_density_tol : h->opts.density_tol;
   const float* dmax = nullptr;
   if (dtol > 0.0 && !h->batched) {
     HF_CUDA(h, h->d_dmax.ensure(sizeof(float) * ns * ns));
-    dmax_kernel<<<(ns * ns + 127) / 128, 128, 0, h->stream>>>(h->d_first.as<int>(), ns, n, DJ, nK, DK,
-                                                              h->d_dmax.as<float>());
-    HF_CHECK_LAUNCH(h, "dmax kernel");
-    ++kernels;
     dmax = h->d_dmax.as<float>();
-  }
-  // Quartets whose Schwarz bound times 4 max|D| is below the threshold cannot survive the
-  // per-quartet density test: with the lists ordered by bound decade, only a prefix of every
-  // segment can.  The prefix lengths are computed on the device (launch_counts_kernel) and read
-  // by the class kernels, so a density-screened build never waits for the host.
-  const int nslot = hfgpu::kNumClasses * 4;
-  if (dmax != nullptr) {
-    static_assert(kBuckets == 18, "launch_counts_kernel's decade table");
-    HF_CUDA(h, h->d_gmax.ensure(sizeof(unsigned int)));
-    HF_CUDA(h, cudaMemsetAsync(h->d_gmax.p, 0, sizeof(unsigned int), h->stream));
-    gmax_kernel<<<std::min((ns * ns + 255) / 256, 1024), 256, 0, h->stream>>>(h->d_dmax.as<float>(), ns * ns,
-                                                                            h->d_gmax.as<unsigned int>());
-    launch_counts_kernel<<<1, 128, 0, h->stream>>>(h->d_gmax.as<unsigned int>(), dtol, h->d_launch.as<long long>(),
-                                                   nslot, kBuckets, h->d_dyn.as<int>());
-    HF_CHECK_LAUNCH(h, "launch counts");
-    kernels += 2;
+    // Quartets whose Schwarz bound times 4 max|D| is below the threshold cannot survive the
+    // per-quartet density test: with the lists ordered by bound decade, only a prefix of every
+    // segment can.  The prefix lengths are computed on the device and read by the class kernels, so a
+    // density-screened build never waits for the host.
+    static_assert(kBuckets == 18, "kDecadeUpper");
+    density_bounds_kernel<<<(unsigned)(((long long)ns * ns + 31) / 32), 128, 0, h->stream>>>(
+        h->d_first.as<int>(), ns, n, DJ, nK, DK, h->d_dmax.as<float>(), gmax, gmax + 1, dtol,
+        h->d_launch.as<long long>(), hfgpu::kNumClasses * 4, kBuckets, h->d_dyn.as<int>());
+    HF_CHECK_LAUNCH(h, "density bounds kernel");
+    ++kernels;
   }
   QuartetArgs<double> qd{};
   qd.jk = jk_args_d(h);
@@ -1263,10 +1265,10 @@ static int jk_device_impl(hfgpu_handle* h, const double* DJ, int nK, const doubl
   qf.jk = jk_args_f(h);
   for (JKArgs<double>* a : {&qd.jk}) {
     a->DJ = DJ; a->nK = nK; a->DK = DK; a->Jh = Jh; a->Kh = Kh; a->dmax = dmax; a->dtol = dtol;
-    a->counters = h->d_counters.as<unsigned long long>();
+    a->counters = h->counters;
   }
   qf.jk.DJ = DJ; qf.jk.nK = nK; qf.jk.DK = DK; qf.jk.Jh = Jh; qf.jk.Kh = Kh; qf.jk.dmax = dmax;
-  qf.jk.dtol = dtol; qf.jk.counters = h->d_counters.as<unsigned long long>();
+  qf.jk.dtol = dtol; qf.jk.counters = h->counters;
   if (h->batched) {
     const long long* mo = h->d_mol.as<long long>();
     const int* mn = reinterpret_cast<const int*>(mo + h->nmol);
@@ -1284,15 +1286,19 @@ static int jk_device_impl(hfgpu_handle* h, const double* DJ, int nK, const doubl
   qd.nparts = qf.nparts = h->nparts;
   const int2* q = h->d_quart.as<int2>();
   long long launched = 0;
-  // largest classes first so that they overlap the tail of the smaller ones
-  unsigned long long* cnt = h->d_counters.as<unsigned long long>();
-  int rc0 = fork_streams(h);
+  // Largest classes first, each of the first kAux on its own stream, the rest round-robin: the
+  // few-quartet, long-latency d classes then overlap the many-quartet s/p classes instead of running
+  // alone on a handful of SMs.
+  auto runs = [&](int c) { return h->q_end[c] > h->q_beg[c] && ((h->class_mask >> c) & 1u); };
+  int nrun = 0, turn = 0;
+  for (int c = 0; c < hfgpu::kNumClasses; ++c) nrun += runs(c);
+  const int used = h->jk_serial ? 1 : std::min(nrun, hfgpu_handle::kAux);
+  int rc0 = fork_streams(h, used);
   if (rc0) return rc0;
-  int order[32], sidx[32];
-  class_schedule(order, sidx);
-  for (int i = 0; i < hfgpu::kNumClasses; ++i) {
-    const int c = order[i];
-    cudaStream_t st = h->aux[h->jk_serial ? 0 : sidx[i]];
+  for (int c = hfgpu::kNumClasses - 1; c >= 0; --c) {
+    h->ev_used[c] = false;
+    if (!runs(c)) continue;
+    cudaStream_t st = h->aux[turn++ % used];
     const hfgpu::ClassLaunchers* L = hfgpu::kClassLaunchers[c];
     const long long b = h->q_beg[c], m = h->q_mid[c], e = h->q_end[c];
     qd.jk.counters = cnt + 3 * c;
@@ -1302,8 +1308,6 @@ static int jk_device_impl(hfgpu_handle* h, const double* DJ, int nK, const doubl
     qd.warp_max = qf.warp_max = class_warp_max(h, c);
     qd.warp_threads = qf.warp_threads = class_warp_threads(h, c);
     qd.staged = qf.staged = (h->sched_cap[c] == 2 && L->has_staged) ? 1 : 0;
-    h->ev_used[c] = false;
-    if (e <= b || !((h->class_mask >> c) & 1u)) continue;
     if (h->timing) HF_CUDA(h, cudaEventRecord(h->ev[2 * c], st));
     // Four parts in list order: [beg,hik1) many-primitive / [hik1,mid) few-primitive (high
     // bound, FP64), [mid,hik2) / [hik2,end) (low bound, FP32 in mixed mode).  Adjacent parts
@@ -1360,10 +1364,11 @@ static int jk_device_impl(hfgpu_handle* h, const double* DJ, int nK, const doubl
     }
     launched += e - b;
   }
-  if ((rc0 = join_streams(h))) return rc0;
+  if ((rc0 = join_streams(h, used))) return rc0;
   h->last_launched = launched;
   const int tot = (int)nn;
-  h->last_kernels = kernels + ((Jout && DJ) ? 1 : 0) + ((Kout && nK > 0) ? 1 : 0);
+  const bool out_j = Jout && DJ, out_k = Kout && nK > 0;
+  h->last_kernels = kernels + (h->batched ? int(out_j) + int(out_k) : int(out_j || out_k));
   if (h->batched) {
     const long long* mo = h->d_mol.as<long long>();
     const int* mn = reinterpret_cast<const int*>(mo + h->nmol);
@@ -1372,13 +1377,10 @@ static int jk_device_impl(hfgpu_handle* h, const double* DJ, int nK, const doubl
     if (Kout && nK > 0) batch_symmetrise_kernel<<<nb, 256, 0, h->stream>>>(Kh, Kout, (long long)nn, mo, mn, h->nmol);
     HF_CHECK_LAUNCH(h, "symmetrise blocks");
   } else {
-    if (Jout && DJ) {
-      symmetrise_kernel<<<(tot + 255) / 256, 256, 0, h->stream>>>(Jh, Jout, n, 1);
-      HF_CHECK_LAUNCH(h, "symmetrise J");
-    }
-    if (Kout && nK > 0) {
-      symmetrise_kernel<<<(tot * nK + 255) / 256, 256, 0, h->stream>>>(Kh, Kout, n, nK);
-      HF_CHECK_LAUNCH(h, "symmetrise K");
+    if (out_j || out_k) {
+      const int nk = out_k ? nK : 0;
+      symmetrise_kernel<<<(unsigned)(((long long)tot * (1 + nk) + 255) / 256), 256, 0, h->stream>>>(Jh, out_j ? Jout : nullptr, Kout, n, nk);
+      HF_CHECK_LAUNCH(h, "symmetrise");
     }
   }
   return HFGPU_OK;
@@ -1406,27 +1408,52 @@ constexpr int kGradForms = 7;
 // The op-table classes have a choice of forms.
 static bool grad_has_forms(int c) { return hfgpu::kClassLaunchers[c]->grad_scratch_slots(0) > 0; }
 
-// Form of a gradient launch of class c: the one hfgpu_autotune_grad or hfgpu_set_grad_forms
-// chose, else the class's default: kGradForms + 1 + v for Rys quadrature in variant v, 0 for one
-// thread per quartet on straight-line code; opts.grad_warp_max_waves <= 0 asks for the thread form
-// of the op-table classes instead.
-static int grad_form_of(const hfgpu_handle* h, int c, bool fp32) {
-  const hfgpu::RysLaunchers* Y = hfgpu::kRysLaunchers[c];
-  int v = Y->grad_variant;
-  const long long limit = fp32 ? 0 : Y->three_prims;
-  if (limit > 0 && h->q_prims[c] <= limit * (h->q_end[c] - h->q_beg[c])) v = hfgpu::kRysThree;
-  if (grad_has_forms(c)) {
-    if (h->grad_form[c] >= 0) return h->grad_form[c];
-    if (h->opts.grad_warp_max_waves <= 0) return 0;
-  }
-  return v >= 0 ? kGradForms + 1 + v : 0;
-}
-
 // Quartets of a list range of n that this handle's partition processes (every nparts-th,
 // starting at number part).
 static long long part_share(const hfgpu_handle* h, long long n) {
   if (h->nparts <= 1) return n;
   return n > h->part ? (n - h->part + h->nparts - 1) / h->nparts : 0;
+}
+
+// Whether a class runs faster with ten thread triples of Rys quadrature per quartet (kRysSplit) than in
+// a form that walks a quartet's primitive quartets one after another: when few quartets leave the GPU to
+// the longest of those walks (441 steps for water in 6-31G*, whose gradient went from 736 to 150 us).
+// In steps of a triple, which costs about three of them around its own; kWarps quartets run at a time.
+// Against the straight-line gradient a step of which costs more in the larger classes, up to the whole
+// of the longest walk is allowed; else a quarter of it, because the classes of a call share the GPU
+// (with 0.8 the (H2O)4 Hessian took 2.5 ms instead of 2.2).
+static bool rys_split_pays(const hfgpu_handle* h, int c, double share) {
+  constexpr double kWarps = 148 * 8;
+  const double nq = (double)part_share(h, h->q_end[c] - h->q_beg[c]);
+  if (nq <= 0) return false;
+  const double avg = double(h->q_prims[c]) / double(h->q_end[c] - h->q_beg[c]);
+  int longest = 0;
+  for (int sg = 0; sg < 4; ++sg) longest = std::max(longest, h->q_maxprims[4 * c + sg]);
+  const double split = std::max(std::ceil(nq / kWarps) * (std::ceil(avg / 10) + 3), std::ceil(longest / 10.0) + 3);
+  return split < share * longest;
+}
+
+// Form of a gradient launch of class c: the one hfgpu_autotune_grad or hfgpu_set_grad_forms
+// chose, else the class's default: kGradForms + 1 + v for Rys quadrature in variant v, 0 for one
+// thread per quartet on straight-line code; opts.grad_warp_max_waves <= 0 asks for the thread form
+// of the op-table classes instead.
+static int grad_form_of(const hfgpu_handle* h, int c, bool fp32) {
+  // few quartets with long primitive loops: ten thread triples per quartet, FP64 only (as the rest of the
+  // three-thread form)
+  const hfgpu::ClassLaunchers* L = hfgpu::kClassLaunchers[c];
+  const int ncart = ncart_of(L->la) * ncart_of(L->lb) * ncart_of(L->lc) * ncart_of(L->ld);
+  const bool split = !fp32 && hfgpu::kRysLaunchers[c]->grad_d[hfgpu::kRysSplit] != nullptr &&
+                     rys_split_pays(h, c, ncart >= 54 ? 1.0 : (ncart > 27 ? 0.5 : 0.25));
+  const hfgpu::RysLaunchers* Y = hfgpu::kRysLaunchers[c];
+  int v = Y->grad_variant;
+  const long long limit = fp32 ? 0 : Y->three_prims;
+  if (limit > 0 && h->q_prims[c] <= limit * (h->q_end[c] - h->q_beg[c])) v = hfgpu::kRysThree;
+  if (split) v = hfgpu::kRysSplit;
+  if (grad_has_forms(c)) {
+    if (h->grad_form[c] >= 0) return h->grad_form[c];
+    if (h->opts.grad_warp_max_waves <= 0) return 0;
+  }
+  return v >= 0 ? kGradForms + 1 + v : 0;
 }
 
 static int grad_device_impl(hfgpu_handle* h, const double* DJ, double cJ, int nK, const double* DK, double cK,
@@ -1757,7 +1784,7 @@ int hfgpu_destroy(hfgpu_handle* h) {
     DeviceGuard dev_guard(h);
     if (h->stream) cudaStreamSynchronize(h->stream);
   for (DevBuf* d : {&h->d_onee, &h->d_pairs, &h->d_prim_d, &h->d_prim_f, &h->d_alpha_d, &h->d_alpha_f, &h->d_boys_d, &h->d_boys_f,
-                    &h->d_quart, &h->d_mats, &h->d_half, &h->d_dmax, &h->d_counters, &h->d_grad, &h->d_scratch,
+                    &h->d_quart, &h->d_mats, &h->d_half, &h->d_dmax, &h->d_grad, &h->d_scratch,
                     &h->d_eri, &h->d_eriq, &h->d_launch, &h->d_dyn, &h->d_first, &h->d_boys_pd,
                     &h->d_boys_pf, &h->d_status, &h->d_abort, &h->d_purify, &h->d_hess})
     d->release();
@@ -2083,7 +2110,7 @@ static int hess_device_impl(hfgpu_handle* h, const double* DJ, double cJ, int nK
   auto form_of = [&](int c) -> int {
     int f = h->hess_cls_form[c] >= 0 ? h->hess_cls_form[c] : h->hess_form;
     if (f == 3 && !hfgpu::kHessLaunchers[c]->has_line) f = -1;
-    return f < 0 && hfgpu::kRysLaunchers[c]->hess_variant < 0 ? 3 : f;
+    return f < 0 && hfgpu::kRysLaunchers[c]->hess_variant < 0 && !rys_split_pays(h, c, 0.25) ? 3 : f;
   };
   // classes largest first, round-robin over the auxiliary streams; each stream's slice is the
   // largest need of its classes
@@ -2128,7 +2155,8 @@ static int hess_device_impl(hfgpu_handle* h, const double* DJ, double cJ, int nK
     }
     if (form_of(c) != 0) {
       const hfgpu::RysLaunchers* Y = hfgpu::kRysLaunchers[c];
-      const int v = form_of(c) == 1 ? 2 : (form_of(c) == 2 ? 0 : Y->hess_variant);
+      int v = form_of(c) == 1 ? 2 : (form_of(c) == 2 ? 0 : Y->hess_variant);
+      if (form_of(c) < 0 && Y->hess[hfgpu::kRysSplit] && rys_split_pays(h, c, 0.25)) v = hfgpu::kRysSplit;
       if (!Y->hess[v](gd, ro, h->pure, q + h->q_beg[c], (int)nq, 0, h->aux[stream_of[c]]))
         return fail(h, HFGPU_ERR_CUDA, "Hessian launch: shared memory");
       HF_CHECK_LAUNCH(h, "hess kernel");
@@ -2400,10 +2428,10 @@ int hfgpu_class_stats(hfgpu_handle* h, int cls, long long* out) {
   out[4] = h->q_end[cls] - h->q_beg[cls];
   out[5] = h->q_mid[cls] - h->q_beg[cls];
   out[6] = out[7] = out[8] = 0;
-  if (h->d_counters.p) {
+  if (h->counters) {
     unsigned long long c[3];
     HF_CUDA(h, cudaStreamSynchronize(h->stream));
-    HF_CUDA(h, cudaMemcpy(c, h->d_counters.as<unsigned long long>() + 3 * cls, sizeof(c), cudaMemcpyDeviceToHost));
+    HF_CUDA(h, cudaMemcpy(c, h->counters + 3 * cls, sizeof(c), cudaMemcpyDeviceToHost));
     out[6] = (long long)c[0];
     out[7] = (long long)c[1];
     out[8] = (long long)c[2];

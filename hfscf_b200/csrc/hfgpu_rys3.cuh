@@ -11,23 +11,26 @@
 #pragma once
 #include "hfgpu_rys.cuh"
 
-template <int LA, int LB, int LC, int LD, int ORD, typename R, int BLOCK>
+// SPLIT = 10: a warp takes one quartet, its ten thread triples every tenth primitive quartet, for launches
+// of few quartets, which would otherwise wait for the longest quartet's primitive loop.
+template <int LA, int LB, int LC, int LD, int ORD, typename R, int BLOCK, int SPLIT>
 __global__ void __launch_bounds__(BLOCK) rys3_kernel(GradArgs<R> a, RysOut o, int pure,
                                                      const int2* __restrict__ quartets, int nq) {
   using D = Rys3Dims<LA, LB, LC, LD, ORD>;
   extern __shared__ __align__(16) unsigned char rys_sm[];
-  constexpr int WARPS = BLOCK / 32, QW = 10;  // quartets per warp
+  static_assert(SPLIT == 1 || SPLIT == 10, "triples per quartet");
+  constexpr int WARPS = BLOCK / 32, SLOTS = 10, QW = SLOTS / SPLIT;  // thread triples and quartets per warp
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int slot = lane < 30 ? lane / 3 : 9, d = lane % 3, nd = (d + 1) % 3, pd = (d + 2) % 3;
   double* gsum = reinterpret_cast<double*>(rys_sm);
-  R* base = reinterpret_cast<R*>(gsum + (ORD == 1 ? 3 * o.smem_atoms : 0)) + (size_t)warp * QW * D::kQuartet;
+  R* base = reinterpret_cast<R*>(gsum + (ORD == 1 ? 3 * o.smem_atoms : 0)) + (size_t)warp * SLOTS * D::kQuartet;
   R* rw = base + (size_t)slot * D::kQuartet;
   R* V = rw + D::kV;
   R* W0 = rw + D::kW + 2 * D::DW;                       // d = 0: the weights as they are
   R* W = d == 0 ? W0 : rw + D::kW + (d - 1) * D::DW;    // renamed for this thread's direction
   // source of the renamed weights: integral e in own, next, previous order
   int* rot = reinterpret_cast<int*>(reinterpret_cast<R*>(gsum + (ORD == 1 ? 3 * o.smem_atoms : 0)) +
-                                    (size_t)WARPS * QW * D::kQuartet);
+                                    (size_t)WARPS * SLOTS * D::kQuartet);
   for (int x = threadIdx.x; x < 2 * D::NCART; x += BLOCK) {
     const int e = x % D::NCART, r = x < D::NCART ? 1 : 2;
     auto back = [&](int l, int c) {  // component with own, next, previous exponents at r, r + 1, r + 2
@@ -42,8 +45,9 @@ __global__ void __launch_bounds__(BLOCK) rys3_kernel(GradArgs<R> a, RysOut o, in
   __syncthreads();
   const int np = a.nparts > 1 ? a.nparts : 1, p0 = np > 1 ? a.part : 0;
   for (int q0 = (blockIdx.x * WARPS + warp) * QW; q0 < nq; q0 += gridDim.x * WARPS * QW) {
-    const bool live = q0 + slot < nq;
-    const int2 pq = quartets[(size_t)(live ? q0 + slot : nq - 1) * np + p0];
+    const int qi = q0 + slot / SPLIT;
+    const bool live = qi < nq;
+    const int2 pq = quartets[(size_t)(live ? qi : nq - 1) * np + p0];
     const PairInfo P = a.pairs[pq.x];
     const PairInfo Q = a.pairs[pq.y];
     double s8 = 8.0;
@@ -53,7 +57,9 @@ __global__ void __launch_bounds__(BLOCK) rys3_kernel(GradArgs<R> a, RysOut o, in
     rys_weights<LA, LB, LC, LD, 3, R>(a, pure, P, Q, s8, d, W0, rw);
     if (d > 0)
       for (int e = 0; e < D::NCART; ++e) W[e] = W0[rot[(d - 1) * D::NCART + e]];
-    const int mine = live ? P.nprim * Q.nprim : 0;
+    // this triple's primitive quartets: first, first + SPLIT, ...
+    const int all = live ? P.nprim * Q.nprim : 0, first = SPLIT > 1 ? slot : 0;
+    const int mine = SPLIT > 1 ? (all > first ? (all - first + SPLIT - 1) / SPLIT : 0) : all;
     const int bo = mine > 0 ? P.prim_off : 0, ko = mine > 0 ? Q.prim_off : 0;
     const PrimPair<R>* bp = a.prims + bo;
     const PrimPair<R>* kp = a.prims + ko;
@@ -65,6 +71,10 @@ __global__ void __launch_bounds__(BLOCK) rys3_kernel(GradArgs<R> a, RysOut o, in
 #pragma unroll
     for (int off = 16; off > 0; off >>= 1) most = max(most, __shfl_xor_sync(0xffffffffu, most, off));
     int ib = 0, ik = 0;
+    if (SPLIT > 1 && mine > 0) {
+      ib = first / Q.nprim;
+      ik = first - ib * Q.nprim;
+    }
     for (int x = 0; x < most; ++x) {
       const bool on = x < mine;  // quartets with fewer primitive quartets add zeros
       const R p = bp[ib].p, ip = bp[ib].ip, q = kp[ik].p, iq = kp[ik].ip;
@@ -120,13 +130,27 @@ __global__ void __launch_bounds__(BLOCK) rys3_kernel(GradArgs<R> a, RysOut o, in
           }
       }
       __syncwarp();  // the roots are read no more
-      if (x + 1 < mine && ++ik == Q.nprim) {
-        ik = 0;
-        ++ib;
+      if (x + 1 < mine) {
+        ik += SPLIT;
+        while (ik >= Q.nprim) {
+          ik -= Q.nprim;
+          ++ib;
+        }
       }
     }
+    if constexpr (SPLIT > 1) {  // sum over the triples into lanes 0-2 (lanes 30 and 31 repeat others)
+#pragma unroll
+      for (int x = 0; x < D::NACC; ++x) {
+        R v = acc[x];
+        v += __shfl_down_sync(0xffffffffu, v, 15);
+        const R v1 = __shfl_down_sync(0xffffffffu, v, 3), v2 = __shfl_down_sync(0xffffffffu, v, 6);
+        const R v3 = __shfl_down_sync(0xffffffffu, v, 9), v4 = __shfl_down_sync(0xffffffffu, v, 12);
+        acc[x] = v + v1 + v2 + v3 + v4;
+      }
+    }
+    const bool lead = lane < 30 && slot % SPLIT == 0;  // holds its quartet's sums
     if constexpr (ORD == 1) {
-      if (lane < 30 && live) {
+      if (lead && live) {
         double* gout = (o.smem_atoms > 0 ? gsum : a.grad) + d;
         const double gA = double(acc[0]), gB = double(acc[1]), gC = double(acc[2]);
         atomicAdd(gout + 3 * P.atom_a, gA);
@@ -137,6 +161,7 @@ __global__ void __launch_bounds__(BLOCK) rys3_kernel(GradArgs<R> a, RysOut o, in
     } else {
       // the 45 entries of each quartet to shared memory, then into the output warp-wide
       R* h45 = base + (size_t)slot * 45;
+      if (SPLIT == 1 || lead)
 #pragma unroll
       for (int A = 0; A < 3; ++A)
 #pragma unroll
@@ -146,7 +171,7 @@ __global__ void __launch_bounds__(BLOCK) rys3_kernel(GradArgs<R> a, RysOut o, in
           h45[r < c ? rys_tri(r, c) : rys_tri(c, r)] = acc[6 + 3 * A + B];
         }
       const int at[4] = {P.atom_a, P.atom_b, Q.atom_a, Q.atom_b};
-      hess_add_warp(lane < 30 && d == 0 && live, base, 1, 15, at, o.hess, 3 * o.natoms);
+      hess_add_warp(lead && d == 0 && live, base, 1, 15, at, o.hess, 3 * o.natoms);
     }
     __syncwarp();
   }
@@ -157,15 +182,15 @@ __global__ void __launch_bounds__(BLOCK) rys3_kernel(GradArgs<R> a, RysOut o, in
   }
 }
 
-template <int LA, int LB, int LC, int LD, int ORD, typename R>
+template <int LA, int LB, int LC, int LD, int ORD, typename R, int SPLIT>
 static bool launch_rys3(const GradArgs<R>& a, const RysOut& o, int pure, const int2* q, int nq, int max_blocks,
                         cudaStream_t s) {
   if (nq <= 0) return true;
   using D = Rys3Dims<LA, LB, LC, LD, ORD>;
-  constexpr int BLOCK = 64, QB = BLOCK / 32 * 10;
-  const size_t bytes = (size_t)QB * D::kQuartet * sizeof(R) + 2 * (size_t)D::NCART * sizeof(int) +
+  constexpr int BLOCK = 64, SLOTS = BLOCK / 32 * 10, QB = SLOTS / SPLIT;
+  const size_t bytes = (size_t)SLOTS * D::kQuartet * sizeof(R) + 2 * (size_t)D::NCART * sizeof(int) +
                        (ORD == 1 ? 3 * sizeof(double) * (size_t)o.smem_atoms : 0);
-  auto k = rys3_kernel<LA, LB, LC, LD, ORD, R, BLOCK>;
+  auto k = rys3_kernel<LA, LB, LC, LD, ORD, R, BLOCK, SPLIT>;
   if (bytes > 48 * 1024 && cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes) != cudaSuccess)
     return false;
   int grid = (nq + QB - 1) / QB;

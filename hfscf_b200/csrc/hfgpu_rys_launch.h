@@ -12,8 +12,9 @@ struct RysOut;
 namespace hfgpu {
 
 // Variants: groups of threads over shared-memory tables, fewest, middle and most threads per quartet,
-// and (kRysThree, null for the larger classes) three threads per quartet, one per direction.
-constexpr int kRysVariants = 4, kRysThree = 3;
+// and (null for the larger classes) three threads per quartet, one per direction (kRysThree), or ten such
+// triples per quartet (kRysSplit).
+constexpr int kRysVariants = 5, kRysThree = 3, kRysSplit = 4;
 
 struct RysLaunchers {
   int la, lb, lc, ld;
