@@ -73,117 +73,138 @@ __device__ __forceinline__ float rsqrt_t<float>(float x) { return rsqrtf(x); }
 //
 // Method (Gill, Johnson & Pople, Int. J. Quantum Chem. 40, 745 (1991); Helgaker,
 // Jorgensen & Olsen, "Molecular Electronic-Structure Theory", sec. 9.8.2):
-//   T <  BOYS_TMAX: Taylor expansion of F_M about the nearest grid point T_k = k h
-//                  (h = 0.1), F_M(T) = sum_j F_{M+j}(T_k) (-dT)^j / j!, j = 0..6 in FP64
-//                  (0..3 in FP32), then the stable downward recursion
-//                  F_{m-1} = (2T F_m + e^-T) / (2m - 1), where (FP64) e^-T = e^-T_k e^(T_k - T)
-//                  with e^-T_k tabulated and e^d, |d| <= h/2, from its degree-8 Taylor
-//                  polynomial (remainder below (h/2)^9 / 9! = 5e-18 relative);
-//   T >= BOYS_TMAX: F_0 = sqrt(pi/T)/2 (erf(sqrt T) = 1 to double precision there); FP64
-//                  F_M = (2M-1)!!/2^(M+1) sqrt(pi) T^-(M+1/2) and the same downward recursion with
-//                  e^-T = 0, so that the lanes of a warp on both sides part only for F_M (a library
-//                  exponential on the far side made the anthracene J/K classes up to (pp|ps) 6-10% slower); FP32 the
-//                  upward recursion F_{m+1} = ((2m+1) F_m - e^-T) / (2T).
-// Table layout: one row of 8 values per (order M, grid point k), rows of one order
-// contiguous.  FP64 row: F_{M+j}(T_k) / j!, j = 0..6, then e^-T_k (64 bytes, four 16-byte
-// loads give the whole expansion); FP32 row: F_{M+j}(T_k) / j!, j = 0..3, then e^-T_k and
-// padding (32 bytes).  The values F_m(T_k) are computed on the host from the convergent
-// series F_m(T) = e^-T sum_i (2T)^i / ((2m+1)(2m+3)...(2m+2i+1)) in long double.
+//   T <  tmax: F_M from a polynomial in d = T_k - T about the nearest grid point T_k = k h, then the
+//              stable downward recursion F_{m-1} = (2T F_m + e^-T) / (2m - 1).  FP64: h = 1/16 (so
+//              that T_k and d are exact), the degree-5 interpolation polynomial of the interval, and
+//              e^-T = e^-T_k e^d with e^-T_k tabulated and e^d, |d| <= h/2, from its degree-7 Taylor
+//              polynomial (remainder below (h/2)^8 / 8! = 3e-17).  FP32: h = 0.1, the Taylor
+//              expansion sum_j F_{M+j}(T_k) d^j / j!, j = 0..3, and the library's exponential;
+//   T >= tmax: F_0 = sqrt(pi/T)/2 (erf(sqrt T) = 1 to double precision there); FP64
+//              F_M = (2M-1)!!/2^(M+1) sqrt(pi) T^-(M+1/2) and the same downward recursion with
+//              e^-T = 0, so that the lanes of a warp on both sides part only for F_M (a library
+//              exponential on the far side made the anthracene J/K classes up to (pp|ps) 6-10% slower); FP32 the
+//              upward recursion F_{m+1} = ((2m+1) F_m - e^-T) / (2T).
+//
+// FP64 row of (order M, grid point k), rows of one order contiguous: 48 bytes, three 16-byte loads,
+// since the low classes wait for the L1 wavefronts of these rows (one per lane and load).  Values
+// c0, c1, c2, c3 in full; the fifth 8 bytes hold the upper halves of c4 (in the low word) and of
+// c5 (in the high word): read as one double they are c5, and c4 is the low word over a zero one;
+// then e^-T_k.  c0..c3 are fitted to what c4 and c5 leave as rounded, so that the rounding of c4
+// and c5 costs only its share beyond degree 3, 2^-21 (h/2)^4 / 8 of c4.  Against 80-bit values the
+// largest relative error of F_M is 6e-15 (M = 0) to 5e-14 (M = 10), T's own rounding of the argument
+// T - T_k gone: 1.5 to 1.8 times below that of a 64-byte row of seven Taylor terms at h = 0.1.
+// @MEASURED@
+// FP32 row: F_{M+j}(T_k) / j!, j = 0..3, then e^-T_k and padding (32 bytes).
 // ---------------------------------------------------------------------------
-#define BOYS_H 0.1
+#define BOYS_H_D 0.0625
+#define BOYS_H_F 0.1
 // Grid points (T_k = 0 .. 56 in FP64, 36 in FP32) and the end of the table's use.  FP64, order M: the T
 // from which e^-T / 2T is below 2e-14 of F_M (below 2e-15 up to M = 6), so that the asymptotic side
 // needs no exponential.
-#define BOYS_NGRID_D 561
+#define BOYS_NGRID_D 897
 #define BOYS_NGRID_F 361
 #define BOYS_TMAX_F 36.0
 __host__ __device__ constexpr double boys_tmax_d(int M) {
   return M == 0 ? 36.0 : (M == 1 ? 38.0 : (M == 2 ? 40.0 : (M <= 4 ? 45.0 : (M <= 6 ? 50.0 : (M <= 8 ? 53.0 : 56.0)))));
 }
-template <typename R>
-__host__ __device__ constexpr int boys_ngrid() {
-  return sizeof(R) == 8 ? BOYS_NGRID_D : BOYS_NGRID_F;
-}
 #define BOYS_MMAX 10             // orders M = 0 .. 10 have rows
-#define BOYS_NM 18               // m = 0 .. 17 computed on the host (M <= 10 plus 7 Taylor terms)
-#define BOYS_ROW 8               // values per row
+#define BOYS_ROW_D 6             // values per FP64 row
+#define BOYS_ROW_F 8             // values per FP32 row
+
+// The FP64 evaluation; row(k, r0, r1, r2) reads the row of grid point k of order M.
+template <int M, class Row>
+__device__ __forceinline__ void boys_eval_d(double T, double pre, const Row& row, double* F) {
+  double f, e;
+  if (T < boys_tmax_d(M)) {
+    // nearest grid index without int/float conversions (they go through the narrow XU
+    // pipe): adding 1.5 * 2^52 leaves round(T / h) in the low mantissa bits
+    const double sh = T * 16.0 + 6755399441055744.0;
+    const double d = (sh - 6755399441055744.0) * BOYS_H_D - T;  // T_k - T, exact
+    double2 r0, r1, r2;
+    row(__double2loint(sh), r0, r1, r2);
+    f = r2.x;
+    f = __hiloint2double(__double2loint(r2.x), 0) + f * d;
+    f = r1.y + f * d;
+    f = r1.x + f * d;
+    f = r0.y + f * d;
+    f = r0.x + f * d;
+    if constexpr (M > 0) {
+      double x = 1.0 / 5040.0;
+      x = 1.0 / 720.0 + d * x;
+      x = 1.0 / 120.0 + d * x;
+      x = 1.0 / 24.0 + d * x;
+      x = 1.0 / 6.0 + d * x;
+      x = 0.5 + d * x;
+      x = 1.0 + d * x;
+      x = 1.0 + d * x;
+      e = r2.y * x;
+    }
+  } else {
+    const double rt = rsqrt(T), it = rt * rt;
+    f = 0.88622692545275801365 * rt;  // sqrt(pi)/2 / sqrt(T)
+#pragma unroll
+    for (int m = 0; m < M; ++m) f *= (m + 0.5) * it;
+    e = 0.0;
+  }
+  F[M] = f;
+  if constexpr (M > 0) {
+    const double t2 = T + T;
+#pragma unroll
+    for (int m = M; m > 0; --m) F[m - 1] = (t2 * F[m] + e) * (1.0 / (2 * m - 1));
+  }
+#pragma unroll
+  for (int m = 0; m <= M; ++m) F[m] *= pre;
+}
+
+// The FP32 evaluation; row(k) returns the four Taylor terms of grid point k of order M.
+template <int M, class Row>
+__device__ __forceinline__ void boys_eval_f(float T, float pre, const Row& row, float* F) {
+  if (T < float(BOYS_TMAX_F)) {
+    const int k = __float2int_rn(T * 10.0f);
+    const float d = float(k) * float(BOYS_H_F) - T;
+    const float4 r0 = row(k);
+    float f = r0.w;
+    f = r0.z + f * d;
+    f = r0.y + f * d;
+    f = r0.x + f * d;
+    F[M] = f;
+    if constexpr (M > 0) {
+      const float e = exp_t<float>(-T), t2 = T + T;
+#pragma unroll
+      for (int m = M; m > 0; --m) F[m - 1] = (t2 * F[m] + e) * float(1.0 / (2 * m - 1));
+    }
+  } else {
+    const float rt = rsqrt_t<float>(T);
+    const float it = rt * rt;
+    F[0] = 0.88622692545275801365f * rt;
+    if constexpr (M > 0) {
+      const float e = exp_t<float>(-T);
+      const float h = 0.5f * it;
+#pragma unroll
+      for (int m = 0; m < M; ++m) F[m + 1] = (float(2 * m + 1) * F[m] - e) * h;
+    }
+  }
+#pragma unroll
+  for (int m = 0; m <= M; ++m) F[m] *= pre;
+}
 
 template <typename R>
 struct BoysTable {
-  const R* __restrict__ tab;  // [BOYS_MMAX + 1][boys_ngrid<R>()][BOYS_ROW]
+  const R* __restrict__ tab;  // [BOYS_MMAX + 1][BOYS_NGRID_D or _F][BOYS_ROW_D or _F]
 
   template <int M>
   __device__ __forceinline__ void eval(R T, R pre, R* F) const {
     static_assert(M <= BOYS_MMAX, "Boys order beyond the table");
     if constexpr (sizeof(R) == 8) {
-      double f, e;
-      if (T < boys_tmax_d(M)) {
-        // nearest grid index without int/float conversions (they go through the narrow XU
-        // pipe): adding 1.5 * 2^52 leaves round(T / h) in the low mantissa bits
-        const double sh = T * 10.0 + 6755399441055744.0;
-        const int k = __double2loint(sh);
-        const double d = (sh - 6755399441055744.0) * BOYS_H - T;  // -(T - T_k)
-        const double2* r = reinterpret_cast<const double2*>(tab + ((size_t)M * BOYS_NGRID_D + k) * BOYS_ROW);
-        const double2 r0 = r[0], r1 = r[1], r2 = r[2], r3 = r[3];
-        f = r3.x;
-        f = r2.y + f * d;
-        f = r2.x + f * d;
-        f = r1.y + f * d;
-        f = r1.x + f * d;
-        f = r0.y + f * d;
-        f = r0.x + f * d;
-        if constexpr (M > 0) {
-          double x = 1.0 / 40320.0;
-          x = 1.0 / 5040.0 + d * x;
-          x = 1.0 / 720.0 + d * x;
-          x = 1.0 / 120.0 + d * x;
-          x = 1.0 / 24.0 + d * x;
-          x = 1.0 / 6.0 + d * x;
-          x = 0.5 + d * x;
-          x = 1.0 + d * x;
-          x = 1.0 + d * x;
-          e = r3.y * x;
-        }
-      } else {
-        const double rt = rsqrt(T), it = rt * rt;
-        f = 0.88622692545275801365 * rt;  // sqrt(pi)/2 / sqrt(T)
-#pragma unroll
-        for (int m = 0; m < M; ++m) f *= (m + 0.5) * it;
-        e = 0.0;
-      }
-      F[M] = f;
-      if constexpr (M > 0) {
-        const double t2 = T + T;
-#pragma unroll
-        for (int m = M; m > 0; --m) F[m - 1] = (t2 * F[m] + e) * (1.0 / (2 * m - 1));
-      }
-    } else if (T < R(BOYS_TMAX_F)) {
-      const int k = __float2int_rn(T * R(10));
-      const R d = R(k) * R(BOYS_H) - T;
-      const float4 r0 = *reinterpret_cast<const float4*>(tab + ((size_t)M * BOYS_NGRID_F + k) * BOYS_ROW);
-      R f = r0.w;
-      f = r0.z + f * d;
-      f = r0.y + f * d;
-      f = r0.x + f * d;
-      F[M] = f;
-      if constexpr (M > 0) {
-        const R e = exp_t<R>(-T), t2 = T + T;
-#pragma unroll
-        for (int m = M; m > 0; --m) F[m - 1] = (t2 * F[m] + e) * R(1.0 / (2 * m - 1));
-      }
+      boys_eval_d<M>(T, pre, [&](int k, double2& r0, double2& r1, double2& r2) {
+        const double2* r = reinterpret_cast<const double2*>(tab + (size_t)M * BOYS_NGRID_D * BOYS_ROW_D) + 3 * k;
+        r0 = r[0], r1 = r[1], r2 = r[2];
+      }, F);
     } else {
-      const R rt = rsqrt_t<R>(T);
-      const R it = rt * rt;
-      F[0] = R(0.88622692545275801365) * rt;
-      if constexpr (M > 0) {
-        const R e = exp_t<R>(-T);
-        const R h = R(0.5) * it;
-#pragma unroll
-        for (int m = 0; m < M; ++m) F[m + 1] = (R(2 * m + 1) * F[m] - e) * h;
-      }
+      boys_eval_f<M>(T, pre, [&](int k) {
+        return *reinterpret_cast<const float4*>(tab + ((size_t)M * BOYS_NGRID_F + k) * BOYS_ROW_F);
+      }, F);
     }
-#pragma unroll
-    for (int m = 0; m <= M; ++m) F[m] *= pre;
   }
 };
 
@@ -193,21 +214,26 @@ __host__ __device__ constexpr int npure_of(int L) { return 2 * L + 1; }
 // ---------------------------------------------------------------------------
 // Boys table of one order staged in shared memory.
 //
-// The same expansion as BoysTable::eval, reading the table of the kernel's single order MS
-// from shared memory, where a block puts it once with one bulk copy (stage_boys_table).  The
-// rows are stored as planes: FP64 plane j (j = 0..3) holds the 16-byte pair (value 2j, value
-// 2j+1) of every grid point, so the four 16-byte loads of one evaluation go to four planes and
-// the lanes of a warp, holding different T, spread over the banks by grid point instead of all
-// hitting the same four banks of their 64-byte rows; FP32 has one plane of float4 (values
-// 0..3).  Global layout: per order, the planes back to back (BOYS_PLANE_BYTES(R) bytes).
+// The same evaluation, reading the table of the kernel's single order MS from shared memory,
+// where a block puts it once with one bulk copy (stage_to_shared).  The
+// rows are stored as planes: FP64 plane j (j = 0..2) holds the j-th 16 bytes of every grid
+// point's row, so the three loads of one evaluation go to three planes and the lanes of a warp,
+// holding different T, spread over the banks by grid point; FP32 has one plane of float4 (values
+// 0..3).  Global layout: per order, boys_plane_stride<R>() bytes from the last, its planes back to
+// back: boys_plane_bytes<R>(M) bytes.
 // ---------------------------------------------------------------------------
-#define BOYS_PLANES_D 4
-#define BOYS_PLANE_BYTES_D (BOYS_PLANES_D * BOYS_NGRID_D * 16)  // 35904 bytes per FP64 order
-#define BOYS_PLANE_BYTES_F (BOYS_NGRID_F * 16)                // 5776 bytes per FP32 order
+#define BOYS_PLANES_D 3
+
+// Grid points of order M that an FP64 evaluation can reach.
+__host__ __device__ constexpr int boys_points_d(int M) { return (int)(boys_tmax_d(M) * 16.0) + 1; }
 
 template <typename R>
-__host__ __device__ constexpr int boys_plane_bytes() {
-  return sizeof(R) == 8 ? BOYS_PLANE_BYTES_D : BOYS_PLANE_BYTES_F;
+__host__ __device__ constexpr int boys_plane_bytes(int M) {  // 27.7 kB (M = 0) to 34.6 kB (M = 4) in FP64, 5.8 kB in FP32
+  return 16 * (sizeof(R) == 8 ? BOYS_PLANES_D * boys_points_d(M) : BOYS_NGRID_F);
+}
+template <typename R>
+__host__ __device__ constexpr int boys_plane_stride() {
+  return 16 * (sizeof(R) == 8 ? BOYS_PLANES_D * BOYS_NGRID_D : BOYS_NGRID_F);
 }
 
 template <typename R, int MS>
@@ -218,74 +244,13 @@ struct BoysShared {
   __device__ __forceinline__ void eval(R T, R pre, R* F) const {
     static_assert(M == MS, "the staged table holds one order");
     if constexpr (sizeof(R) == 8) {
-      double f, e;
-      if (T < boys_tmax_d(M)) {
-        // nearest grid index without int/float conversions (they go through the narrow XU
-        // pipe): adding 1.5 * 2^52 leaves round(T / h) in the low mantissa bits
-        const double sh = T * 10.0 + 6755399441055744.0;
-        const int k = __double2loint(sh);
-        const double d = (sh - 6755399441055744.0) * BOYS_H - T;  // -(T - T_k)
-        const double2* P = reinterpret_cast<const double2*>(tab);
-        const double2 r0 = P[k], r1 = P[BOYS_NGRID_D + k], r2 = P[2 * BOYS_NGRID_D + k], r3 = P[3 * BOYS_NGRID_D + k];
-        f = r3.x;
-        f = r2.y + f * d;
-        f = r2.x + f * d;
-        f = r1.y + f * d;
-        f = r1.x + f * d;
-        f = r0.y + f * d;
-        f = r0.x + f * d;
-        if constexpr (M > 0) {
-          double x = 1.0 / 40320.0;
-          x = 1.0 / 5040.0 + d * x;
-          x = 1.0 / 720.0 + d * x;
-          x = 1.0 / 120.0 + d * x;
-          x = 1.0 / 24.0 + d * x;
-          x = 1.0 / 6.0 + d * x;
-          x = 0.5 + d * x;
-          x = 1.0 + d * x;
-          x = 1.0 + d * x;
-          e = r3.y * x;
-        }
-      } else {
-        const double rt = rsqrt(T), it = rt * rt;
-        f = 0.88622692545275801365 * rt;  // sqrt(pi)/2 / sqrt(T)
-#pragma unroll
-        for (int m = 0; m < M; ++m) f *= (m + 0.5) * it;
-        e = 0.0;
-      }
-      F[M] = f;
-      if constexpr (M > 0) {
-        const double t2 = T + T;
-#pragma unroll
-        for (int m = M; m > 0; --m) F[m - 1] = (t2 * F[m] + e) * (1.0 / (2 * m - 1));
-      }
-    } else if (T < R(BOYS_TMAX_F)) {
-      const int k = __float2int_rn(T * R(10));
-      const R d = R(k) * R(BOYS_H) - T;
-      const float4 r0 = reinterpret_cast<const float4*>(tab)[k];
-      R f = r0.w;
-      f = r0.z + f * d;
-      f = r0.y + f * d;
-      f = r0.x + f * d;
-      F[M] = f;
-      if constexpr (M > 0) {
-        const R e = exp_t<R>(-T), t2 = T + T;
-#pragma unroll
-        for (int m = M; m > 0; --m) F[m - 1] = (t2 * F[m] + e) * R(1.0 / (2 * m - 1));
-      }
+      boys_eval_d<M>(T, pre, [&](int k, double2& r0, double2& r1, double2& r2) {
+        const double2* P = reinterpret_cast<const double2*>(tab) + k;
+        r0 = P[0], r1 = P[boys_points_d(M)], r2 = P[2 * boys_points_d(M)];
+      }, F);
     } else {
-      const R rt = rsqrt_t<R>(T);
-      const R it = rt * rt;
-      F[0] = R(0.88622692545275801365) * rt;
-      if constexpr (M > 0) {
-        const R e = exp_t<R>(-T);
-        const R h = R(0.5) * it;
-#pragma unroll
-        for (int m = 0; m < M; ++m) F[m + 1] = (R(2 * m + 1) * F[m] - e) * h;
-      }
+      boys_eval_f<M>(T, pre, [&](int k) { return reinterpret_cast<const float4*>(tab)[k]; }, F);
     }
-#pragma unroll
-    for (int m = 0; m <= M; ++m) F[m] *= pre;
   }
 };
 

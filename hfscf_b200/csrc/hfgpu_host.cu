@@ -37,60 +37,129 @@ constexpr double kPrimQuartetCut = 1e-16;
 int pair_class(int la, int lb) { return la * (la + 1) / 2 + lb; }  // la >= lb: ss ps pp ds dp dd
 int quartet_class(int cp, int cq) { return cp * (cp + 1) / 2 + cq; }  // cp >= cq
 
-// Boys table rows (layout in hfgpu_common.cuh): F_m(k h), m < BOYS_NM, from the series
-// e^-T sum_i (2T)^i / (2m+1)(2m+3)...(2m+2i+1) in long double, divided by j! for the j-th
-// Taylor term, and e^-T_k.  `terms` = 7 (FP64 rows) or 4 (FP32 rows).
-template <typename R>
-std::vector<R> boys_table(int terms) {
-  constexpr int NGRID = boys_ngrid<R>();
-  std::vector<long double> F((size_t)NGRID * BOYS_NM), ek(NGRID);
-  for (int k = 0; k < NGRID; ++k) {
-    const long double T = (long double)k * (long double)BOYS_H;
-    for (int m = 0; m < BOYS_NM; ++m) {
+// F_M(T_k), M < nm, on the grid T_k = k h of n points, and e^-T_k: the convergent series
+// e^-T sum_i (2T)^i / (2m+1)(2m+3)...(2m+2i+1) in long double.
+void boys_grid(int n, int nm, long double h, std::vector<long double>& F, std::vector<long double>& ek) {
+  F.resize((size_t)n * nm);
+  ek.resize(n);
+  for (int k = 0; k < n; ++k) {
+    const long double T = k * h;
+    ek[k] = expl(-T);
+    for (int m = 0; m < nm; ++m) {
       long double term = 1.0L / (2 * m + 1), sum = term;
       for (int i = 0; i < 2000; ++i) {
         term *= 2.0L * T / (long double)(2 * m + 2 * i + 3);
         sum += term;
         if (term < sum * 1e-21L) break;
       }
-      F[(size_t)k * BOYS_NM + m] = expl(-T) * sum;
+      F[(size_t)k * nm + m] = ek[k] * sum;
     }
-    ek[k] = expl(-T);
   }
-  std::vector<R> t((size_t)(BOYS_MMAX + 1) * NGRID * BOYS_ROW, R(0));
+}
+
+// FP32 Boys rows (layout in hfgpu_common.cuh): F_{M+j}(T_k) / j!, j = 0..3, and e^-T_k.
+std::vector<float> boys_table_f() {
+  constexpr int NM = BOYS_MMAX + 4;
+  std::vector<long double> F, ek;
+  boys_grid(BOYS_NGRID_F, NM, (long double)BOYS_H_F, F, ek);
+  std::vector<float> t((size_t)(BOYS_MMAX + 1) * BOYS_NGRID_F * BOYS_ROW_F, 0.0f);
   for (int M = 0; M <= BOYS_MMAX; ++M)
-    for (int k = 0; k < NGRID; ++k) {
-      R* row = &t[((size_t)M * NGRID + k) * BOYS_ROW];
+    for (int k = 0; k < BOYS_NGRID_F; ++k) {
+      float* row = &t[((size_t)M * BOYS_NGRID_F + k) * BOYS_ROW_F];
       long double fact = 1.0L;
-      for (int j = 0; j < terms; ++j) {
+      for (int j = 0; j < 4; ++j) {
         if (j > 0) fact *= j;
-        row[j] = (R)(F[(size_t)k * BOYS_NM + M + j] / fact);
+        row[j] = (float)(F[(size_t)k * NM + M + j] / fact);
       }
-      row[terms] = (R)ek[k];
+      row[4] = (float)ek[k];
     }
   return t;
 }
 
-// The same table in the plane layout of BoysShared (hfgpu_common.cuh): per order, FP64 planes
-// j = 0..3 of (row[2j], row[2j+1]) over the grid points; FP32 one plane of row[0..3].
-template <typename R>
-std::vector<R> boys_planes(const std::vector<R>& rows) {
-  constexpr int NGRID = boys_ngrid<R>();
-  const int per = boys_plane_bytes<R>() / (int)sizeof(R);  // values per order
-  std::vector<R> t((size_t)(BOYS_MMAX + 1) * per, R(0));
+// The N Chebyshev points of [-half, half], and the coefficients of the polynomial of degree N - 1
+// through the values v there: Newton's divided differences (in v), expanded from the last one.
+template <int N>
+void cheb_points(long double half, long double* z) {
+  for (int i = 0; i < N; ++i) z[i] = half * cosl(acosl(-1.0L) * (2 * i + 1) / (2 * N));
+}
+template <int N>
+void interpolate(const long double* z, long double* v, long double* c) {
+  for (int j = 1; j < N; ++j)
+    for (int i = N - 1; i >= j; --i) v[i] = (v[i] - v[i - 1]) / (z[i] - z[i - j]);
+  for (int i = 0; i < N; ++i) c[i] = 0.0L;
+  for (int j = N - 1; j >= 0; --j) {
+    for (int i = N - 1; i > 0; --i) c[i] = c[i - 1] - z[j] * c[i];
+    c[0] = v[j] - z[j] * c[0];
+  }
+}
+
+// FP64 Boys rows (layout in hfgpu_common.cuh).  F_M on the interval about T_k comes from the Taylor
+// terms F_{M+j}(T_k) d^j / j!, j < 12, |d| <= 1/32 (the rest is below 1e-27); six Chebyshev points
+// give c4 and c5, and four, of what these leave once they are rounded, c0..c3.
+std::vector<double> boys_table_d() {
+  constexpr int NT = 12, NM = BOYS_MMAX + NT;
+  const long double half = (long double)BOYS_H_D / 2;
+  std::vector<long double> F, ek;
+  boys_grid(BOYS_NGRID_D, NM, (long double)BOYS_H_D, F, ek);
+  long double z6[6], z4[4];
+  cheb_points<6>(half, z6);
+  cheb_points<4>(half, z4);
+  auto bits = [](double x) {
+    unsigned long long u;
+    memcpy(&u, &x, 8);
+    return u;
+  };
+  auto value = [](unsigned long long u) {
+    double x;
+    memcpy(&x, &u, 8);
+    return x;
+  };
+  std::vector<double> t((size_t)(BOYS_MMAX + 1) * BOYS_NGRID_D * BOYS_ROW_D);
   for (int M = 0; M <= BOYS_MMAX; ++M)
-    for (int k = 0; k < NGRID; ++k) {
-      const R* row = &rows[((size_t)M * NGRID + k) * BOYS_ROW];
-      R* o = &t[(size_t)M * per];
-      if (sizeof(R) == 8) {
-        for (int j = 0; j < BOYS_PLANES_D; ++j) {
-          o[((size_t)j * NGRID + k) * 2 + 0] = row[2 * j];
-          o[((size_t)j * NGRID + k) * 2 + 1] = row[2 * j + 1];
-        }
-      } else {
-        for (int j = 0; j < 4; ++j) o[(size_t)k * 4 + j] = row[j];
+    for (int k = 0; k < BOYS_NGRID_D; ++k) {
+      double* row = &t[((size_t)M * BOYS_NGRID_D + k) * BOYS_ROW_D];
+      auto taylor = [&](long double d) {
+        long double s = 0.0L;
+        for (int j = NT - 1; j >= 0; --j) s = F[(size_t)k * NM + M + j] + s * d / (j + 1);
+        return s;
+      };
+      long double v[6], c[6];
+      for (int i = 0; i < 6; ++i) v[i] = taylor(z6[i]);
+      interpolate<6>(z6, v, c);
+      const unsigned long long half_ulp = 0x80000000ull, upper = 0xFFFFFFFF00000000ull;
+      const unsigned long long b4 = (bits((double)c[4]) + half_ulp) & upper;
+      const unsigned long long b5 = ((bits((double)c[5]) + half_ulp) & upper) | (b4 >> 32);
+      const double c4 = value(b4), c5 = value(b5);
+      for (int i = 0; i < 4; ++i) {
+        const long double d = z4[i], d2 = d * d;
+        v[i] = taylor(d) - d2 * d2 * (c4 + d * c5);
       }
+      interpolate<4>(z4, v, c);
+      for (int j = 0; j < 4; ++j) row[j] = (double)c[j];
+      row[4] = c5;
+      row[5] = (double)ek[k];
     }
+  return t;
+}
+
+// The same tables in the plane layout of BoysShared (hfgpu_common.cuh): per order, FP64 planes
+// j = 0..2 of (row[2j], row[2j+1]) over the order's grid points; FP32 one plane of row[0..3].
+std::vector<double> boys_planes_d(const std::vector<double>& rows) {
+  const size_t per = boys_plane_stride<double>() / sizeof(double);  // values per order
+  std::vector<double> t((BOYS_MMAX + 1) * per, 0.0);
+  for (int M = 0; M <= BOYS_MMAX; ++M)
+    for (int k = 0; k < boys_points_d(M); ++k)
+      for (int j = 0; j < BOYS_PLANES_D; ++j)
+        memcpy(&t[M * per + ((size_t)j * boys_points_d(M) + k) * 2],
+               &rows[((size_t)M * BOYS_NGRID_D + k) * BOYS_ROW_D + 2 * j], 16);
+  return t;
+}
+std::vector<float> boys_planes_f(const std::vector<float>& rows) {
+  const size_t per = boys_plane_stride<float>() / sizeof(float);
+  std::vector<float> t((BOYS_MMAX + 1) * per, 0.0f);
+  for (int M = 0; M <= BOYS_MMAX; ++M)
+    for (int k = 0; k < BOYS_NGRID_F; ++k)
+      memcpy(&t[M * per + (size_t)k * 4], &rows[((size_t)M * BOYS_NGRID_F + k) * BOYS_ROW_F], 16);
   return t;
 }
 
@@ -1758,10 +1827,10 @@ int hfgpu_create(const hfgpu_basis* b, const hfgpu_opts* opts, hfgpu_handle** ou
   h->own_stream = true;
   // the tables are constants: computed once per process (the long-double series take milliseconds),
   // uploaded per handle
-  static const std::vector<double> bt = boys_table<double>(7);
-  static const std::vector<float> btf = boys_table<float>(4);
-  static const std::vector<double> bpd = boys_planes(bt);
-  static const std::vector<float> bpf = boys_planes(btf);
+  static const std::vector<double> bt = boys_table_d();
+  static const std::vector<float> btf = boys_table_f();
+  static const std::vector<double> bpd = boys_planes_d(bt);
+  static const std::vector<float> bpf = boys_planes_f(btf);
   if (h->d_boys_d.ensure(sizeof(double) * bt.size()) || h->d_boys_f.ensure(sizeof(float) * btf.size()) ||
       h->d_boys_pd.ensure(sizeof(double) * bpd.size()) || h->d_boys_pf.ensure(sizeof(float) * bpf.size()) ||
       h->d_status.ensure(sizeof(int)) || h->d_abort.ensure(sizeof(int)) ||

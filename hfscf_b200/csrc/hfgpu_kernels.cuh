@@ -252,7 +252,7 @@ struct QuartetArgs {
   int nseg;
   int seg_off[4];
   int staged;           // 1: the persistent form with the Boys table staged in shared memory (low L)
-  const R* boys_planes; // the Boys table in plane layout, one block of boys_plane_bytes<R>() per order
+  const R* boys_planes; // the Boys table in plane layout, boys_plane_stride<R>() bytes per order
   int* status;          // device status word (HFGPU_DEV_STAGE_TIMEOUT when a staging wait ran out)
   int stage_test;       // 1: arm the staging barrier without a copy, so that its wait runs out (test only)
   const int* abort_flag;  // device word the host sets to stop persistent launches early (nullptr: none)
@@ -388,8 +388,8 @@ __global__ void __launch_bounds__(128) quartet_staged_kernel(QuartetArgs<R> qa, 
   extern __shared__ __align__(16) unsigned char staged_smem[];
   __shared__ unsigned long long stage_bar;
   R* tab = reinterpret_cast<R*>(staged_smem);
-  const unsigned char* src = reinterpret_cast<const unsigned char*>(qa.boys_planes) + (size_t)L * boys_plane_bytes<R>();
-  if (!stage_to_shared(tab, src, boys_plane_bytes<R>(), &stage_bar, qa.status, qa.stage_test == 0)) return;
+  const unsigned char* src = reinterpret_cast<const unsigned char*>(qa.boys_planes) + (size_t)L * boys_plane_stride<R>();
+  if (!stage_to_shared(tab, src, boys_plane_bytes<R>(L), &stage_bar, qa.status, qa.stage_test == 0)) return;
   const BoysShared<R, L> boys{tab};
   nq = launch_count(qa, nq);
   const int warps = gridDim.x * (blockDim.x >> 5);
