@@ -917,6 +917,7 @@ static void launch_quartet_impl(const QuartetArgs<R>& a, const int2* q, int nq, 
     const int pad = 100 * 1024;
     auto k = quartet_kernel<{la}, {lb}, {lc}, {ld}, R>;
     cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, pad);
+    cudaFuncSetAttribute(k, cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutDefault);
     k<<<(nq + bs - 1) / bs, bs, pad, s>>>(a, q, nq);
     return;
   }}
@@ -924,11 +925,15 @@ static void launch_quartet_impl(const QuartetArgs<R>& a, const int2* q, int nq, 
     const int bs = a.block > 0 ? a.block : 64;
     if constexpr (CC::kCapBlocks > 0) {{
       if (a.capped) {{
-        quartet_kernel<{la}, {lb}, {lc}, {ld}, R, CC::kCapBlocks><<<(nq + bs - 1) / bs, bs, 0, s>>>(a, q, nq);
+        auto k = quartet_kernel<{la}, {lb}, {lc}, {ld}, R, CC::kCapBlocks>;
+        prefer_l1(k);
+        k<<<(nq + bs - 1) / bs, bs, 0, s>>>(a, q, nq);
         return;
       }}
     }}
-    quartet_kernel<{la}, {lb}, {lc}, {ld}, R><<<(nq + bs - 1) / bs, bs, 0, s>>>(a, q, nq);
+    auto k = quartet_kernel<{la}, {lb}, {lc}, {ld}, R>;
+    prefer_l1(k);
+    k<<<(nq + bs - 1) / bs, bs, 0, s>>>(a, q, nq);
     return;
   }}
   if constexpr (kWarp) {{
@@ -957,11 +962,15 @@ template <typename CC, typename R>
 static bool launch_primwarp_impl(const QuartetArgs<R>& a, const int2* q, int nq, cudaStream_t s) {{
   if constexpr (CC::kPrimWarp) {{
     // a.group lanes per quartet, 128-thread blocks
+    auto go = [&](auto k, int per) {{
+      prefer_l1(k);
+      k<<<(nq + per - 1) / per, 128, 0, s>>>(a, q, nq);
+    }};
     switch (a.group) {{
-      case 4: quartet_primwarp_kernel<{la}, {lb}, {lc}, {ld}, R, 4><<<(nq + 31) / 32, 128, 0, s>>>(a, q, nq); break;
-      case 8: quartet_primwarp_kernel<{la}, {lb}, {lc}, {ld}, R, 8><<<(nq + 15) / 16, 128, 0, s>>>(a, q, nq); break;
-      case 16: quartet_primwarp_kernel<{la}, {lb}, {lc}, {ld}, R, 16><<<(nq + 7) / 8, 128, 0, s>>>(a, q, nq); break;
-      default: quartet_primwarp_kernel<{la}, {lb}, {lc}, {ld}, R, 32><<<(nq + 3) / 4, 128, 0, s>>>(a, q, nq); break;
+      case 4: go(quartet_primwarp_kernel<{la}, {lb}, {lc}, {ld}, R, 4>, 32); break;
+      case 8: go(quartet_primwarp_kernel<{la}, {lb}, {lc}, {ld}, R, 8>, 16); break;
+      case 16: go(quartet_primwarp_kernel<{la}, {lb}, {lc}, {ld}, R, 16>, 8); break;
+      default: go(quartet_primwarp_kernel<{la}, {lb}, {lc}, {ld}, R, 32>, 4); break;
     }}
     return true;
   }} else {{
@@ -977,18 +986,22 @@ template <typename R>
 static void launch_grad(const GradArgs<R>& a, int pure, const int2* q, int nq, int grid, cudaStream_t s) {{
   if (nq <= 0) return;
   const size_t sm = sizeof(double) * 3 * a.smem_atoms;
+  auto go = [&](auto k) {{
+    prefer_l1(k, sm);
+    k<<<grid, 128, sm, s>>>(a, pure, q, nq);
+  }};
   if constexpr (ClassCode<{la}, {lb}, {lc}, {ld}>::kGradPasses == 4) {{
     // one launch per accumulator set, one after the other on the stream; each adds its part
-    grad_kernel<{la}, {lb}, {lc}, {ld}, R, 0><<<grid, 128, sm, s>>>(a, pure, q, nq);
-    grad_kernel<{la}, {lb}, {lc}, {ld}, R, 1><<<grid, 128, sm, s>>>(a, pure, q, nq);
-    grad_kernel<{la}, {lb}, {lc}, {ld}, R, 2><<<grid, 128, sm, s>>>(a, pure, q, nq);
-    grad_kernel<{la}, {lb}, {lc}, {ld}, R, 3><<<grid, 128, sm, s>>>(a, pure, q, nq);
+    go(grad_kernel<{la}, {lb}, {lc}, {ld}, R, 0>);
+    go(grad_kernel<{la}, {lb}, {lc}, {ld}, R, 1>);
+    go(grad_kernel<{la}, {lb}, {lc}, {ld}, R, 2>);
+    go(grad_kernel<{la}, {lb}, {lc}, {ld}, R, 3>);
   }} else if constexpr (ClassCode<{la}, {lb}, {lc}, {ld}>::kGradPasses == 2) {{
     // one launch per pair of accumulator sets (U with A, B with C)
-    grad_kernel<{la}, {lb}, {lc}, {ld}, R, 0><<<grid, 128, sm, s>>>(a, pure, q, nq);
-    grad_kernel<{la}, {lb}, {lc}, {ld}, R, 1><<<grid, 128, sm, s>>>(a, pure, q, nq);
+    go(grad_kernel<{la}, {lb}, {lc}, {ld}, R, 0>);
+    go(grad_kernel<{la}, {lb}, {lc}, {ld}, R, 1>);
   }} else {{
-    grad_kernel<{la}, {lb}, {lc}, {ld}, R><<<grid, 128, sm, s>>>(a, pure, q, nq);
+    go(grad_kernel<{la}, {lb}, {lc}, {ld}, R>);
   }}
 }}
 template <typename CC, int NCART>
@@ -1063,7 +1076,7 @@ extern const RysLaunchers rys_launchers_{t};
 const RysLaunchers rys_launchers_{t} = {{{la}, {lb}, {lc}, {ld}, {gv}, {p64}, {hv},
     {{{gd}}},
     {{{gf}}},
-    {{{hd}}}, {qp}, {qf}}};
+    {{{hd}}}, {qf}}};
 }}  // namespace hfgpu
 """
 
@@ -1071,14 +1084,11 @@ const RysLaunchers rys_launchers_{t} = {{{la}, {lb}, {lc}, {ld}, {gv}, {p64}, {h
 RYS_THREE_MAX_CART = {(1, "double"): 162, (1, "float"): 0, (2, "double"): 81}
 
 
-# Undifferentiated integrals by Rys quadrature, one warp per quartet: the classes that have it and the
-# average number of primitive quartets per quartet up to which it is the default (0: only when the
-# schedule asks).  Against the fastest thread form, us: n-octane (dd|dd) 34 against 293, (dd|dp) 57
-# against 183, (dd|pp) 75 against 139, (dp|dp) 145 against 193, but (dd|ds) 72 against 57 and (dp|pp) 348
-# against 178; anthracene, with longer contractions, (dd|pp) 600 against 510 at 4.0 primitive quartets
-# and (dp|dp) 1360 against 720 at 4.1, (dd|dp) 537 against 800 at 2.0.
-RYS_QUARTET_PRIMS = {(2, 1, 1, 1): 0, (2, 1, 2, 0): 0, (2, 1, 2, 1): 3, (2, 2, 1, 1): 3, (2, 2, 2, 0): 0,
-                     (2, 2, 2, 1): 1000, (2, 2, 2, 2): 1000}
+# Undifferentiated integrals by Rys quadrature, one warp per quartet: the classes that have it.  Alone
+# against the fastest thread form, us: n-octane (dd|dd) 34 against 293, (dd|dp) 57 against 183, (dd|pp) 75
+# against 139, (dp|dp) 145 against 193, but (dd|ds) 72 against 57 and (dp|pp) 348 against 178; anthracene,
+# with longer contractions, (dd|pp) 600 against 510 and (dp|dp) 1360 against 720, (dd|dp) 537 against 800.
+RYS_QUARTET = ((2, 1, 1, 1), (2, 1, 2, 0), (2, 1, 2, 1), (2, 2, 1, 1), (2, 2, 2, 0), (2, 2, 2, 1), (2, 2, 2, 2))
 
 
 def rys_inst(c, t):
@@ -1095,8 +1105,8 @@ def rys_inst(c, t):
 
     gv, p64, hv = rys_defaults(c)
     return RYS_INST_TEMPLATE.format(t=t, la=c[0], lb=c[1], lc=c[2], ld=c[3], gv=gv, p64=p64, hv=hv, gd=row(1, "double"),
-                                    gf=row(1, "float"), hd=row(2, "double"), qp=RYS_QUARTET_PRIMS.get(c, 0),
-                                    qf=f"&launch_rys_quartet<{cl}>" if c in RYS_QUARTET_PRIMS else "nullptr")
+                                    gf=row(1, "float"), hd=row(2, "double"),
+                                    qf=f"&launch_rys_quartet<{cl}>" if c in RYS_QUARTET else "nullptr")
 
 
 def rys_groups(la, lb, lc, ld):

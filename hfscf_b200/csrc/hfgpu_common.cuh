@@ -223,6 +223,7 @@ __host__ __device__ constexpr int npure_of(int L) { return 2 * L + 1; }
 // back: boys_plane_bytes<R>(M) bytes.
 // ---------------------------------------------------------------------------
 #define BOYS_PLANES_D 3
+#define BOYS_STAGED_MMAX 4       // orders that are staged (classes of la + lb + lc + ld up to it)
 
 // Grid points of order M that an FP64 evaluation can reach.
 __host__ __device__ constexpr int boys_points_d(int M) { return (int)(boys_tmax_d(M) * 16.0) + 1; }
@@ -233,7 +234,7 @@ __host__ __device__ constexpr int boys_plane_bytes(int M) {  // 27.7 kB (M = 0) 
 }
 template <typename R>
 __host__ __device__ constexpr int boys_plane_stride() {
-  return 16 * (sizeof(R) == 8 ? BOYS_PLANES_D * BOYS_NGRID_D : BOYS_NGRID_F);
+  return boys_plane_bytes<R>(BOYS_STAGED_MMAX);
 }
 
 template <typename R, int MS>
@@ -242,7 +243,7 @@ struct BoysShared {
 
   template <int M>
   __device__ __forceinline__ void eval(R T, R pre, R* F) const {
-    static_assert(M == MS, "the staged table holds one order");
+    static_assert(M == MS && M <= BOYS_STAGED_MMAX, "the staged table holds one order");
     if constexpr (sizeof(R) == 8) {
       boys_eval_d<M>(T, pre, [&](int k, double2& r0, double2& r1, double2& r2) {
         const double2* P = reinterpret_cast<const double2*>(tab) + k;

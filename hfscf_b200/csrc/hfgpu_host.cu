@@ -142,12 +142,13 @@ std::vector<double> boys_table_d() {
   return t;
 }
 
-// The same tables in the plane layout of BoysShared (hfgpu_common.cuh): per order, FP64 planes
-// j = 0..2 of (row[2j], row[2j+1]) over the order's grid points; FP32 one plane of row[0..3].
+// The same tables in the plane layout of BoysShared (hfgpu_common.cuh), for the orders that are staged:
+// per order, FP64 planes j = 0..2 of (row[2j], row[2j+1]) over the order's grid points; FP32 one plane
+// of row[0..3].
 std::vector<double> boys_planes_d(const std::vector<double>& rows) {
   const size_t per = boys_plane_stride<double>() / sizeof(double);  // values per order
-  std::vector<double> t((BOYS_MMAX + 1) * per, 0.0);
-  for (int M = 0; M <= BOYS_MMAX; ++M)
+  std::vector<double> t((BOYS_STAGED_MMAX + 1) * per, 0.0);
+  for (int M = 0; M <= BOYS_STAGED_MMAX; ++M)
     for (int k = 0; k < boys_points_d(M); ++k)
       for (int j = 0; j < BOYS_PLANES_D; ++j)
         memcpy(&t[M * per + ((size_t)j * boys_points_d(M) + k) * 2],
@@ -156,8 +157,8 @@ std::vector<double> boys_planes_d(const std::vector<double>& rows) {
 }
 std::vector<float> boys_planes_f(const std::vector<float>& rows) {
   const size_t per = boys_plane_stride<float>() / sizeof(float);
-  std::vector<float> t((BOYS_MMAX + 1) * per, 0.0f);
-  for (int M = 0; M <= BOYS_MMAX; ++M)
+  std::vector<float> t((BOYS_STAGED_MMAX + 1) * per, 0.0f);
+  for (int M = 0; M <= BOYS_STAGED_MMAX; ++M)
     for (int k = 0; k < BOYS_NGRID_F; ++k)
       memcpy(&t[M * per + (size_t)k * 4], &rows[((size_t)M * BOYS_NGRID_F + k) * BOYS_ROW_F], 16);
   return t;
@@ -307,19 +308,22 @@ int class_warp_max(const hfgpu_handle* h, int c) {
 int class_warp_threads(const hfgpu_handle* h, int c) { return h->sched_warp[c] == 2 ? 128 : 32; }
 
 // Whether an FP64 launch of nq quartets of class c runs one warp per quartet by Rys quadrature:
-// schedule entry 1 or 2; by default the classes and average primitive-quartet counts where it measured
-// faster than one thread per quartet (rys_jk_prims in gen_eri.py), up to opts.warp_max_quartets.
+// schedule entry 1 or 2; by default, up to opts.warp_max_quartets quartets, classes of few primitive
+// quartets in small builds.  There the class's longest thread would be the build's ((dd|dd) alone 190-230
+// us): (H2O)2/6-31G* 475 -> 197 us per build, propane/6-31G** 655 -> 343, (H2O)4/cc-pVDZ 1285 -> 1115,
+// (H2O)5/cc-pVDZ 1717 -> 1629, hexane/6-31G** 1257 -> 1183.  Elsewhere other classes hide it, and
+// the form's shared memory takes L1 cache from theirs: octane/6-31G** (75 million primitive quartets)
+// 2155 us either way, (H2O)6/cc-pVDZ (131 million) 2958 -> 3015, (H2O)8/cc-pVDZ 4723 -> 4900, and with
+// classes of more primitive quartets on it octane 2270.
 bool use_rys_quartet(const hfgpu_handle* h, int c, long long nq) {
-  const hfgpu::RysLaunchers* Y = hfgpu::kRysLaunchers[c];
-  if (!Y->quartet) return false;
+  if (!hfgpu::kRysLaunchers[c]->quartet) return false;
   const int w = h->sched_warp[c];
   if (w >= 0) return w > 0;
-  // few primitive quartets in all: one warp per quartet finishes first in every class ((dp|ds) of propane
-  // 36 against 55 us, of (H2O)3/cc-pVDZ 55 against 92, but 155 against 80 for the 110,000 of (H2O)8)
-  constexpr long long kFewPrims = 30000;
-  return nq <= h->opts.warp_max_quartets &&
-         (h->q_prims[c] <= kFewPrims ||
-          h->q_prims[c] <= Y->quartet_prims * std::max<double>(1.0, double(h->q_end[c] - h->q_beg[c])));
+  constexpr long long kFewPrims = 20000, kSmallBuild = 80000000;
+  if (nq > h->opts.warp_max_quartets || h->q_prims[c] > kFewPrims) return false;
+  long long total = 0;
+  for (long long p : h->q_prims) total += p;
+  return total <= kSmallBuild;
 }
 
 // FP64 launch of class c over quartets q[0, nq); false when its shared memory could not be had.

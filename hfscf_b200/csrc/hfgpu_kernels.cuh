@@ -367,6 +367,20 @@ __device__ __forceinline__ void quartet_thread(const QuartetArgs<R>& qa, const B
   }
 }
 
+// Asks for the largest L1 cache for kernel k, whose blocks use `bytes` of shared memory (none, or the
+// gradient's few sums): room for four blocks, about what its registers admit.  Kernels of several classes
+// share an SM, and left to itself the driver carves out shared memory for those that use much of it and
+// leaves it carved for these, whose Boys rows and spills then miss: with one class on the Rys form,
+// whichever, the J/K build of anthracene took 18.6 ms against 15.3, (H2O)8/cc-pVDZ 6.6 against 4.9, octane
+// 2.50 against 2.26; the gradient of octane 8.96 against 7.93, of anthracene (mixed) 71.8 against 58.4.
+// The Rys forms keep the driver's choice: their carve-out capped at half slowed octane's gradient to
+// 10.1 ms and its Hessian from 37.3 to 40.7.
+template <typename K>
+inline void prefer_l1(K* k, size_t bytes = 0) {
+  const size_t percent = bytes ? (4 * (bytes + 1024) * 100 + 228 * 1024 - 1) / (228 * 1024) : 0;
+  cudaFuncSetAttribute(k, cudaFuncAttributePreferredSharedMemoryCarveout, percent < 100 ? (int)percent : 100);
+}
+
 // MINB > 1: the register-capped variant (at least MINB blocks of 128 threads per SM) of the
 // small classes, for more warps in flight.
 template <int LA, int LB, int LC, int LD, typename R, int MINB = 1>

@@ -29,9 +29,7 @@ struct RysLaunchers {
                                cudaStream_t);
   bool (*hess[kRysVariants])(const GradArgs<double>&, const RysOut&, int pure, const int2* q, int nq, int max_blocks,
                              cudaStream_t);
-  // undifferentiated integrals, one warp per quartet (the large classes; null otherwise): default up to
-  // quartet_prims primitive quartets per quartet on average
-  double quartet_prims;
+  // undifferentiated integrals, one warp per quartet (the large classes; null otherwise)
   bool (*quartet)(const QuartetArgs<double>&, const double* tab, const int2* q, int nq, cudaStream_t);
 };
 
