@@ -886,7 +886,7 @@ INST_TEMPLATE = """// GENERATED by gen_eri.py -- do not edit.
 #include "../hfgpu_launch.h"
 
 namespace hfgpu {{
-// Large classes: one warp per quartet when the class has too few quartets to keep
+// Large classes in FP32: one warp per quartet when the class has too few quartets to keep
 // the GPU busy with one (spilling, latency-bound) thread per quartet; one thread
 // per quartet otherwise.
 template <typename CC, typename R>
@@ -1503,7 +1503,7 @@ def gen_grad_table(la, lb, lc, ld):
 
 
 # ---------------------------------------------------------------------------
-# Warp mode: the large energy classes run one warp per quartet.  The VRR and
+# Warp mode (FP32): the large energy classes run one warp per quartet.  The VRR and
 # HRR are levelised (an op's inputs come from earlier levels only), so the 32
 # lanes execute one level's ops in parallel out of shared memory, with a
 # __syncwarp between levels.  Slots are reused once their last reader's level

@@ -260,13 +260,12 @@ struct hfgpu_handle {
   cudaEvent_t ev[2 * 21 + 2] = {};
   bool ev_used[21] = {};
   // per-class launch schedule (hfgpu_autotune / hfgpu_set_schedule): threads per block of
-  // the thread-per-quartet form, warp-over-primitives form for the many-primitive parts,
-  // warp-per-quartet form (-1 = follow opts.warp_max_quartets)
+  // the thread-per-quartet form, lanes per quartet for the many-primitive parts (-1: primwarp_group),
+  // form of the large classes (-1: use_rys_quartet, class_warp_max)
   int sched_block[21], sched_primwarp[21], sched_warp[21], sched_cap[21];
   unsigned class_mask = ~0u;            // classes a J/K build launches (autotuning runs one at a time)
-  // gradient form per class (hfgpu_autotune_grad): 1 warp per quartet, 0 one thread per
-  // quartet, 3/4 (5/6) block of four (eight) warps per quartet (whole / split), -1 the default
-  // (grad_form_of)
+  // gradient form per class (hfgpu_autotune_grad): 0 one thread per quartet, 1 .. 6 a group of threads
+  // by Rys quadrature, -1 the default (grad_form_of)
   int grad_form[21];
   unsigned grad_class_mask = ~0u;       // classes a gradient launches (autotuning runs one at a time)
   // Hessian form (hfgpu_set_hess_form): -1 by class, 0 one thread per quartet, 1 and 2 a group of
@@ -616,6 +615,9 @@ int build_pairs(hfgpu_handle* h) {
   HF_CUDA(h, h->d_prim_f.ensure(sizeof(PrimPair<float>) * np));
   HF_CUDA(h, h->d_alpha_d.ensure(sizeof(double) * 2 * np));
   HF_CUDA(h, h->d_alpha_f.ensure(sizeof(float) * 2 * np));
+  // the Hessian's half matrix now, unless large, so that a first Hessian call may be inside a capture
+  const size_t hess_bytes = sizeof(double) * 9 * (size_t)h->natoms * h->natoms;
+  if (!h->batched && hess_bytes <= (16u << 20)) HF_CUDA(h, h->d_hess.ensure(hess_bytes));
   cudaStream_t s = h->stream;
   HF_CUDA(h, cudaMemcpyAsync(h->d_pairs.p, h->pairs.data(), sizeof(PairInfo) * h->pairs.size(), cudaMemcpyHostToDevice, s));
   if (!pd.empty()) {

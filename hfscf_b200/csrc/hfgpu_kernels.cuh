@@ -175,13 +175,6 @@ __device__ __forceinline__ void finish_block(const R* cart, double* V) {
   }
 }
 
-template <int LA, int LB, int LC, int LD, typename R>
-__device__ __forceinline__ void cart_block(const PairInfo& P, const PairInfo& Q, const PrimPair<R>* prims,
-                                           const BoysTable<R>& boys, R* cart) {
-  ClassCode<LA, LB, LC, LD>::template eri<R>(prims + P.prim_off, P.nprim, prims + Q.prim_off, Q.nprim,
-                                              R(P.ABx), R(P.ABy), R(P.ABz), R(Q.ABx), R(Q.ABy), R(Q.ABz), boys, cart);
-}
-
 __device__ __forceinline__ long long packed_index(long long i, long long j, long long k, long long l) {
   const long long ij = i > j ? i * (i + 1) / 2 + j : j * (j + 1) / 2 + i;
   const long long kl = k > l ? k * (k + 1) / 2 + l : l * (l + 1) / 2 + k;

@@ -304,8 +304,8 @@ class Engine:
 
     def autotune_grad(self, D, precision=FP64, repeats=2) -> np.ndarray:
         """hfgpu_autotune_grad on density D (host array or device tensor): the gradient form per
-        class (0 thread, 1 warp, 2 warp split per accumulator set, 3 block of four warps, 4 block
-        split per set, 5 and 6 the same with eight warps, -1 no choice)."""
+        class (0 one thread per quartet; 1, 3, 5 the smallest, middle and largest group of threads per
+        quartet by Rys quadrature, as 2, 4, 6; -1 no choice)."""
         import torch
         Dd = D if isinstance(D, torch.Tensor) else torch.from_numpy(_c(D)).to(torch.device("cuda", self._opts.device))
         forms = np.zeros(NUM_CLASSES, dtype=np.int32)
@@ -314,8 +314,8 @@ class Engine:
         return forms
 
     def set_grad_forms(self, forms):
-        """hfgpu_set_grad_forms: the gradient form per class (-1, 0 thread, 1 warp, 2 warp split,
-        3 block, 4 block split, 5 block of eight warps, 6 its split)."""
+        """hfgpu_set_grad_forms: the gradient form per class (-1, 0 thread, 1 .. 6 a group of
+        threads by Rys quadrature, as autotune_grad returns them)."""
         f = np.ascontiguousarray(np.broadcast_to(np.asarray(forms, dtype=np.int32), (NUM_CLASSES,)))
         self._check(lib().hfgpu_set_grad_forms(self.h, f.ctypes.data_as(_ip)))
 
@@ -385,14 +385,15 @@ class Engine:
         return H
 
     def set_hess_form(self, form: int):
-        """hfgpu_set_hess_form: -1 by class (default), 0 thread (global scratch), 1 block, 2 warp per
-        quartet, 3 thread on straight-line register code where the class has it."""
+        """hfgpu_set_hess_form: -1 by class (default), 0 thread (global scratch), 1 and 2 Rys quadrature
+        with the class's largest and smallest group of threads per quartet, 3 thread on straight-line
+        register code where the class has it."""
         self._check(lib().hfgpu_set_hess_form(self.h, ctypes.c_int(form)))
 
     def autotune_hess(self, D, repeats=2):
         """hfgpu_autotune_hess on density D (host array, device tensor or device pointer): per
-        class the fastest of the thread, block, warp and straight-line forms; returns the chosen
-        forms (0 thread, 1 block, 2 warp, 3 straight-line)."""
+        class the fastest of the thread, Rys (largest and smallest group) and straight-line forms;
+        returns the chosen forms (0, 1, 2, 3)."""
         import torch
         if isinstance(D, int):
             ptr = D

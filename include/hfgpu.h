@@ -65,8 +65,8 @@ typedef struct {
                               with HFGPU_MIXED; default 1e-12 as for full builds: a looser 1e-10 made the
                               incremental SCF of n-octane take 44 iterations instead of 24) */
   int device;              /* CUDA device ordinal (default 0) */
-  int warp_max_quartets;   /* classes whose default is one warp per quartet: so when the class has at most this
-                              many quartets, one thread per quartet otherwise (default 2^30 = always; -1 = never) */
+  int warp_max_quartets;   /* classes whose default is one warp per quartet: only when the class has at most
+                              this many quartets (default 2^30 = no limit; -1 = never) */
   int grad_warp_max_waves;    /* gradient of (dp|dp) (dd|pp) (dd|ds) (dd|dp) (dd|dd) before any
                                  hfgpu_autotune_grad / hfgpu_set_grad_forms: > 0 (default 48) a group of
                                  threads per quartet by Rys quadrature, 0 = one thread per quartet on
@@ -307,9 +307,9 @@ int hfgpu_setup_times(const hfgpu_handle* h, double* ms);
  *   [2] form of the classes (dp|pp) (dp|ds) (dp|dp) (dd|pp) (dd|ds) (dd|dp) (dd|dd): 2/1 = one warp
  *       per quartet by Rys quadrature in FP64, and in FP32 the block-per-quartet form (128 threads per
  *       quartet) / warp-per-quartet form (four quartets per 128-thread block) over op tables; 0 =
- *       thread forms; -1 = the measured default: FP64 the Rys form for (dd|dp), (dd|dd) and, with few
- *       primitive quartets per quartet, (dp|dp) and (dd|pp), FP32 the warp form for (dd|dp) and (dd|dd),
- *       both up to opts.warp_max_quartets quartets, thread forms otherwise;
+ *       thread forms; -1 = the measured default, up to opts.warp_max_quartets quartets: FP64 the Rys form
+ *       for classes of at most 20,000 primitive quartets in builds of at most 80 million, FP32 the warp
+ *       form for (dd|dp) and (dd|dd); thread forms otherwise;
  *   [3] variant of the thread-per-quartet form: 0 plain; 1 register-capped, for more warps
  *       per SM (the small classes (ps|ss) ... (dp|ss) have one); 2 persistent, with the
  *       class's Boys table staged into shared memory by one bulk (TMA) copy per block (the
