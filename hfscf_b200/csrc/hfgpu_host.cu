@@ -891,7 +891,7 @@ int build_quartets(hfgpu_handle* h) {
     HF_CUDA(h, cudaMemcpyAsync(h->d_quart.p, all.get(), sizeof(int2) * (size_t)total, cudaMemcpyHostToDevice,
                                h->stream));
   {
-    // launch table of the density-screened builds (see launch_counts_kernel)
+    // launch table of the density-screened builds (see density_bounds_kernel)
     const int nslot = hfgpu::kNumClasses * 4;
     std::vector<long long> lt((size_t)nslot * (2 + kBuckets), 0);
     for (int c = 0; c < hfgpu::kNumClasses; ++c) {
