@@ -79,11 +79,10 @@ __device__ __forceinline__ float rsqrt_t<float>(float x) { return rsqrtf(x); }
 //              e^-T = e^-T_k e^d with e^-T_k tabulated and e^d, |d| <= h/2, from its degree-7 Taylor
 //              polynomial (remainder below (h/2)^8 / 8! = 3e-17).  FP32: h = 0.1, the Taylor
 //              expansion sum_j F_{M+j}(T_k) d^j / j!, j = 0..3, and the library's exponential;
-//   T >= tmax: F_0 = sqrt(pi/T)/2 (erf(sqrt T) = 1 to double precision there); FP64
-//              F_M = (2M-1)!!/2^(M+1) sqrt(pi) T^-(M+1/2) and the same downward recursion with
-//              e^-T = 0, so that the lanes of a warp on both sides part only for F_M (a library
-//              exponential on the far side made the anthracene J/K classes up to (pp|ps) 6-10% slower); FP32 the
-//              upward recursion F_{m+1} = ((2m+1) F_m - e^-T) / (2T).
+//   T >= tmax: F_0 = sqrt(pi/T)/2 (erf(sqrt T) = 1 to double precision there) and the upward
+//              recursion F_{m+1} = ((2m+1) F_m - e^-T) / (2T), in FP64 without e^-T (a library
+//              exponential on the far side made the anthracene J/K classes up to (pp|ps) 6-10% slower).
+//              Upward from F_0, not down from F_M: F_10 underflows from T = 1e29 on, F_0 nowhere.
 //
 // FP64 row of (order M, grid point k), rows of one order contiguous: 48 bytes, three 16-byte loads,
 // since the low classes wait for the L1 wavefronts of these rows (one per lane and load).  Values
@@ -115,7 +114,6 @@ __host__ __device__ constexpr double boys_tmax_d(int M) {
 // The FP64 evaluation; row(k, r0, r1, r2) reads the row of grid point k of order M.
 template <int M, class Row>
 __device__ __forceinline__ void boys_eval_d(double T, double pre, const Row& row, double* F) {
-  double f, e;
   if (T < boys_tmax_d(M)) {
     // nearest grid index without int/float conversions (they go through the narrow XU
     // pipe): adding 1.5 * 2^52 leaves round(T / h) in the low mantissa bits
@@ -123,12 +121,13 @@ __device__ __forceinline__ void boys_eval_d(double T, double pre, const Row& row
     const double d = (sh - 6755399441055744.0) * BOYS_H_D - T;  // T_k - T, exact
     double2 r0, r1, r2;
     row(__double2loint(sh), r0, r1, r2);
-    f = r2.x;
+    double f = r2.x;
     f = __hiloint2double(__double2loint(r2.x), 0) + f * d;
     f = r1.y + f * d;
     f = r1.x + f * d;
     f = r0.y + f * d;
     f = r0.x + f * d;
+    F[M] = f;
     if constexpr (M > 0) {
       double x = 1.0 / 5040.0;
       x = 1.0 / 720.0 + d * x;
@@ -138,20 +137,15 @@ __device__ __forceinline__ void boys_eval_d(double T, double pre, const Row& row
       x = 0.5 + d * x;
       x = 1.0 + d * x;
       x = 1.0 + d * x;
-      e = r2.y * x;
+      const double e = r2.y * x, t2 = T + T;
+#pragma unroll
+      for (int m = M; m > 0; --m) F[m - 1] = (t2 * F[m] + e) * (1.0 / (2 * m - 1));
     }
   } else {
     const double rt = rsqrt(T), it = rt * rt;
-    f = 0.88622692545275801365 * rt;  // sqrt(pi)/2 / sqrt(T)
+    F[0] = 0.88622692545275801365 * rt;  // sqrt(pi)/2 / sqrt(T)
 #pragma unroll
-    for (int m = 0; m < M; ++m) f *= (m + 0.5) * it;
-    e = 0.0;
-  }
-  F[M] = f;
-  if constexpr (M > 0) {
-    const double t2 = T + T;
-#pragma unroll
-    for (int m = M; m > 0; --m) F[m - 1] = (t2 * F[m] + e) * (1.0 / (2 * m - 1));
+    for (int m = 0; m < M; ++m) F[m + 1] = F[m] * ((m + 0.5) * it);
   }
 #pragma unroll
   for (int m = 0; m <= M; ++m) F[m] *= pre;

@@ -1,0 +1,32 @@
+"""The FP64 Boys function (hfgpu_boys) beyond the table.
+
+Every finite T >= 0 is accepted, and for large T the value is the complete integral
+F_n(T) = (2n-1)!! / 2^(n+1) sqrt(pi) T^-(n+1/2) (the rest, below e^-T, is far below the last digit).
+Tolerance: the evaluation takes two or three rounded operations per order, below 1e-14 relative in all, and
+1e-307 absolute where F_n is subnormal (above T = 1e307, where 1/T is, every F_n but F_0 is zero).
+"""
+import numpy as np
+import pytest
+
+from hfscf_b200 import basis as B
+from hfscf_b200 import engine as E
+from hfscf_b200 import molecules as M
+
+pytestmark = pytest.mark.gpu
+
+
+def _engine():
+    Z, x = M.water(np.random.default_rng(1))
+    return E.Engine(B.build_basis("sto-3g", Z, np.asarray(x) * B.ANGSTROM_TO_BOHR))
+
+
+@pytest.mark.parametrize("m", range(11))
+def test_boys_of_large_arguments(m):
+    T = np.concatenate([10.0 ** np.arange(2, 308, 7), [3e28, 2e29, 3e35, 1e200, 1.7e308]])
+    with _engine() as eng:
+        F = eng.boys(m, T)
+    t = T.astype(np.longdouble)
+    ref = np.sqrt(np.longdouble("3.14159265358979323846264338327950288") / t) / 2
+    for n in range(m + 1):
+        assert np.all(np.abs(F[:, n] - ref) <= 1e-14 * ref + np.longdouble(1e-307)), n
+        ref = ref * (n + np.longdouble(0.5)) / t
