@@ -896,7 +896,8 @@ static void launch_quartet_impl(const QuartetArgs<R>& a, const int2* q, int nq, 
       // persistent: about as many blocks as the GPU holds at once (each stages the Boys table once)
       auto k = quartet_staged_kernel<{la}, {lb}, {lc}, {ld}, R>;
       const int bs = a.block > 0 ? a.block : 64;
-      const int smem = boys_plane_bytes<R>({la} + {lb} + {lc} + {ld});
+      constexpr int smem = boys_plane_bytes<R>({la} + {lb} + {lc} + {ld});
+      if constexpr (smem > 48 * 1024) cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
       int dev = 0, sms = 148, per_sm = 1;
       cudaGetDevice(&dev);
       cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);

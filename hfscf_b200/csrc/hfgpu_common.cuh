@@ -74,10 +74,10 @@ __device__ __forceinline__ float rsqrt_t<float>(float x) { return rsqrtf(x); }
 // Method (Gill, Johnson & Pople, Int. J. Quantum Chem. 40, 745 (1991); Helgaker,
 // Jorgensen & Olsen, "Molecular Electronic-Structure Theory", sec. 9.8.2):
 //   T <  tmax: F_M from a polynomial in d = T_k - T about the nearest grid point T_k = k h, then the
-//              stable downward recursion F_{m-1} = (2T F_m + e^-T) / (2m - 1).  FP64: h = 1/16 (so
+//              stable downward recursion F_{m-1} = (2T F_m + e^-T) / (2m - 1).  FP64: h = 1/32 (so
 //              that T_k and d are exact), the degree-5 interpolation polynomial of the interval, and
-//              e^-T = e^-T_k e^d with e^-T_k tabulated and e^d, |d| <= h/2, from its degree-7 Taylor
-//              polynomial (remainder below (h/2)^8 / 8! = 3e-17).  FP32: h = 0.1, the Taylor
+//              e^-T = e^-T_k e^d with e^-T_k tabulated and e^d, |d| <= h/2, from its degree-6 Taylor
+//              polynomial (remainder below (h/2)^7 / 7! = 5e-17).  FP32: h = 0.1, the Taylor
 //              expansion sum_j F_{M+j}(T_k) d^j / j!, j = 0..3, and the library's exponential;
 //   T >= tmax: F_0 = sqrt(pi/T)/2 (erf(sqrt T) = 1 to double precision there) and the upward
 //              recursion F_{m+1} = ((2m+1) F_m - e^-T) / (2T), in FP64 without e^-T (a library
@@ -89,23 +89,26 @@ __device__ __forceinline__ float rsqrt_t<float>(float x) { return rsqrtf(x); }
 // c0, c1, c2, c3 in full; the fifth 8 bytes hold the upper halves of c4 (in the low word) and of
 // c5 (in the high word): read as one double they are c5, and c4 is the low word over a zero one;
 // then e^-T_k.  c0..c3 are fitted to what c4 and c5 leave as rounded, so that the rounding of c4
-// and c5 costs only its share beyond degree 3, 2^-21 (h/2)^4 / 8 of c4.  Against 80-bit values the
-// largest relative error of F_M is 6e-15 (M = 0) to 5e-14 (M = 10), 1.5 to 1.8 times below that of the
-// 64-byte row of seven Taylor terms at h = 0.1 before, with which anthracene's J/K build took 19.0 ms
-// against 18.4, that of 512 water molecules 19.5 against 18.8 and anthracene's mixed gradient 73.7
-// against 72.3.
+// and c5 costs only its share beyond degree 3, 2^-21 (h/2)^4 / 8 of c4: 2e-17 of F_0, 1e-16 of F_10.
+// Against 80-bit values over T in [0, 70] the relative error of F_M is 3e-16 at most and 6e-17 on average
+// (M = 0) to 4e-15 and 2e-16 (M = 10).  The 64-byte row of seven Taylor terms at h = 0.1 before it had
+// 6e-15 and 9e-17 to 9e-14 and 2e-15, and this row at h = 1/16 6e-15 and 1.2e-16 to 5e-14 and 3.6e-15 (a
+// larger mean, because the interpolation error fills the interval and the Taylor error only its ends).
+// The four loads of the 64-byte row cost anthracene's J/K build 3% (19.0 ms against 18.4 at the time); the
+// twice as long table of h = 1/32 costs it 2% of that again (15.5 -> 15.8 ms, octane 2.22 -> 2.25).
 // FP32 row: F_{M+j}(T_k) / j!, j = 0..3, then e^-T_k and padding (32 bytes).
 // ---------------------------------------------------------------------------
-#define BOYS_H_D 0.0625
+#define BOYS_H_D 0.03125
 #define BOYS_H_F 0.1
-// Grid points (T_k = 0 .. 56 in FP64, 36 in FP32) and the end of the table's use.  FP64, order M: the T
-// from which e^-T / 2T is below 2e-14 of F_M (below 2e-15 up to M = 6), so that the asymptotic side
-// needs no exponential.
-#define BOYS_NGRID_D 897
+// Grid points (T_k = 0 .. 63 in FP64, 36 in FP32) and the end of the table's use.  FP64, order M: the
+// first whole T at which F_M without e^-T and with erf = 1 is within 1e-16 of F_M, so that the asymptotic
+// side needs no exponential.
+#define BOYS_NGRID_D 2017
 #define BOYS_NGRID_F 361
 #define BOYS_TMAX_F 36.0
 __host__ __device__ constexpr double boys_tmax_d(int M) {
-  return M == 0 ? 36.0 : (M == 1 ? 38.0 : (M == 2 ? 40.0 : (M <= 4 ? 45.0 : (M <= 6 ? 50.0 : (M <= 8 ? 53.0 : 56.0)))));
+  constexpr double t[11] = {36.0, 39.0, 43.0, 46.0, 49.0, 51.0, 54.0, 56.0, 58.0, 61.0, 63.0};
+  return t[M];
 }
 #define BOYS_MMAX 10             // orders M = 0 .. 10 have rows
 #define BOYS_ROW_D 6             // values per FP64 row
@@ -117,7 +120,7 @@ __device__ __forceinline__ void boys_eval_d(double T, double pre, const Row& row
   if (T < boys_tmax_d(M)) {
     // nearest grid index without int/float conversions (they go through the narrow XU
     // pipe): adding 1.5 * 2^52 leaves round(T / h) in the low mantissa bits
-    const double sh = T * 16.0 + 6755399441055744.0;
+    const double sh = T * 32.0 + 6755399441055744.0;
     const double d = (sh - 6755399441055744.0) * BOYS_H_D - T;  // T_k - T, exact
     double2 r0, r1, r2;
     row(__double2loint(sh), r0, r1, r2);
@@ -129,8 +132,7 @@ __device__ __forceinline__ void boys_eval_d(double T, double pre, const Row& row
     f = r0.x + f * d;
     F[M] = f;
     if constexpr (M > 0) {
-      double x = 1.0 / 5040.0;
-      x = 1.0 / 720.0 + d * x;
+      double x = 1.0 / 720.0;
       x = 1.0 / 120.0 + d * x;
       x = 1.0 / 24.0 + d * x;
       x = 1.0 / 6.0 + d * x;
@@ -221,10 +223,10 @@ __host__ __device__ constexpr int npure_of(int L) { return 2 * L + 1; }
 #define BOYS_STAGED_MMAX 4       // orders that are staged (classes of la + lb + lc + ld up to it)
 
 // Grid points of order M that an FP64 evaluation can reach.
-__host__ __device__ constexpr int boys_points_d(int M) { return (int)(boys_tmax_d(M) * 16.0) + 1; }
+__host__ __device__ constexpr int boys_points_d(int M) { return (int)(boys_tmax_d(M) * 32.0) + 1; }
 
 template <typename R>
-__host__ __device__ constexpr int boys_plane_bytes(int M) {  // 27.7 kB (M = 0) to 34.6 kB (M = 4) in FP64, 5.8 kB in FP32
+__host__ __device__ constexpr int boys_plane_bytes(int M) {  // 55 kB (M = 0) to 75 kB (M = 4) in FP64, 5.8 kB in FP32
   return 16 * (sizeof(R) == 8 ? BOYS_PLANES_D * boys_points_d(M) : BOYS_NGRID_F);
 }
 template <typename R>

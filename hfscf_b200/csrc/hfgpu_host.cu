@@ -37,23 +37,24 @@ constexpr double kPrimQuartetCut = 1e-16;
 int pair_class(int la, int lb) { return la * (la + 1) / 2 + lb; }  // la >= lb: ss ps pp ds dp dd
 int quartet_class(int cp, int cq) { return cp * (cp + 1) / 2 + cq; }  // cp >= cq
 
-// F_M(T_k), M < nm, on the grid T_k = k h of n points, and e^-T_k: the convergent series
-// e^-T sum_i (2T)^i / (2m+1)(2m+3)...(2m+2i+1) in long double.
+// F_M(T_k), M < nm, on the grid T_k = k h of n points, and e^-T_k, in long double: the convergent series
+// e^-T sum_i (2T)^i / (2m+1)(2m+3)...(2m+2i+1) for the highest order, the stable downward recursion
+// F_{m-1} = (2T F_m + e^-T) / (2m-1) for the others.
 void boys_grid(int n, int nm, long double h, std::vector<long double>& F, std::vector<long double>& ek) {
   F.resize((size_t)n * nm);
   ek.resize(n);
   for (int k = 0; k < n; ++k) {
     const long double T = k * h;
     ek[k] = expl(-T);
-    for (int m = 0; m < nm; ++m) {
-      long double term = 1.0L / (2 * m + 1), sum = term;
-      for (int i = 0; i < 2000; ++i) {
-        term *= 2.0L * T / (long double)(2 * m + 2 * i + 3);
-        sum += term;
-        if (term < sum * 1e-21L) break;
-      }
-      F[(size_t)k * nm + m] = ek[k] * sum;
+    long double* f = &F[(size_t)k * nm];
+    long double term = 1.0L / (2 * nm - 1), sum = term;
+    for (int i = 0; i < 2000; ++i) {
+      term *= 2.0L * T / (long double)(2 * (nm - 1) + 2 * i + 3);
+      sum += term;
+      if (term < sum * 1e-21L) break;
     }
+    f[nm - 1] = ek[k] * sum;
+    for (int m = nm - 1; m > 0; --m) f[m - 1] = (2.0L * T * f[m] + ek[k]) / (2 * m - 1);
   }
 }
 
@@ -94,7 +95,7 @@ void interpolate(const long double* z, long double* v, long double* c) {
 }
 
 // FP64 Boys rows (layout in hfgpu_common.cuh).  F_M on the interval about T_k comes from the Taylor
-// terms F_{M+j}(T_k) d^j / j!, j < 12, |d| <= 1/32 (the rest is below 1e-27); six Chebyshev points
+// terms F_{M+j}(T_k) d^j / j!, j < 12, |d| <= 1/64 (the rest is below 1e-30); six Chebyshev points
 // give c4 and c5, and four, of what these leave once they are rounded, c0..c3.
 std::vector<double> boys_table_d() {
   constexpr int NT = 12, NM = BOYS_MMAX + NT;
