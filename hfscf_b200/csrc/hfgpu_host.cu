@@ -1466,7 +1466,6 @@ static int jk_device_impl(hfgpu_handle* h, const double* DJ, int nK, const doubl
 // totals fit in kGradSmemBytes, and then no more than kGradMaxBlocks blocks for the
 // straight-line classes (their grid-stride loop takes the rest), so that the flush at the
 // end of each block stays a small number of atomics.
-constexpr int kGradSmemBytes = 24 * 1024;
 constexpr int kGradMaxBlocks = 2048;
 // blocks of a straight-line gradient launch: opts.reserved[1] when set (> 0), else kGradMaxBlocks
 static int grad_max_blocks(const hfgpu_handle* h) {

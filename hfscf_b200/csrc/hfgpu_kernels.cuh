@@ -33,6 +33,9 @@ struct JKArgs {
   unsigned long long* __restrict__ counters;  // per class: computed, skipped by density, primitive quartets
 };
 
+// Most shared memory that a gradient's per-block sums take (smem_atoms of GradArgs): up to 1024 atoms.
+constexpr int kGradSmemBytes = 24 * 1024;
+
 template <typename R>
 struct GradArgs {
   const PairInfo* __restrict__ pairs;

@@ -269,6 +269,16 @@ constexpr int rys_block() {
                        : (64 / G * D::group(G) * (int)sizeof(R) <= 72 * 1024 ? 64 : 32));
 }
 
+// Lets kernel k take `bytes` of dynamic shared memory where that is above the 48 KB of any kernel.  MOST, the
+// most that any launch of k can ask for, is what is set: the limit is the kernel's, not the launch's, and
+// a handle on another thread may be about to launch k with more sums of its own.
+template <size_t MOST, typename K>
+inline bool allow_shared(K* k, size_t bytes) {
+  static_assert(MOST <= 227 * 1024, "shared memory of a block");
+  return bytes <= 48 * 1024 ||
+         cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)MOST) == cudaSuccess;
+}
+
 // Launches class (LA LB|LC LD) at derivative order ORD with G threads per quartet over quartets
 // q[0, nq), at most max_blocks blocks (0: one group of quartets per block).
 template <int LA, int LB, int LC, int LD, int ORD, typename R, int G>
@@ -277,11 +287,10 @@ static bool launch_rys(const GradArgs<R>& a, const RysOut& o, int pure, const in
   if (nq <= 0) return true;
   using D = RysDims<LA, LB, LC, LD, ORD>;
   constexpr int BLOCK = rys_block<D, R, G>(), GROUPS = BLOCK / G;
-  const size_t bytes = (size_t)GROUPS * D::group(G) * sizeof(R) + (size_t)D::NCART * sizeof(int) +
-                       (ORD == 1 ? 3 * sizeof(double) * (size_t)o.smem_atoms : 0);
+  constexpr size_t kTables = (size_t)GROUPS * D::group(G) * sizeof(R) + (size_t)D::NCART * sizeof(int);
+  const size_t bytes = kTables + (ORD == 1 ? 3 * sizeof(double) * (size_t)o.smem_atoms : 0);
   auto k = rys_deriv_kernel<LA, LB, LC, LD, ORD, R, G, BLOCK>;
-  if (bytes > 48 * 1024 && cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes) != cudaSuccess)
-    return false;
+  if (!allow_shared<kTables + (ORD == 1 ? kGradSmemBytes : 0)>(k, bytes)) return false;
   int grid = (nq + GROUPS - 1) / GROUPS;
   if (max_blocks > 0 && grid > max_blocks) grid = max_blocks;
   k<<<grid, BLOCK, bytes, s>>>(a, o, pure, q, nq);

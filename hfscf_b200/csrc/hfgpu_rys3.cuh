@@ -188,11 +188,10 @@ static bool launch_rys3(const GradArgs<R>& a, const RysOut& o, int pure, const i
   if (nq <= 0) return true;
   using D = Rys3Dims<LA, LB, LC, LD, ORD>;
   constexpr int BLOCK = 64, SLOTS = BLOCK / 32 * 10, QB = SLOTS / SPLIT;
-  const size_t bytes = (size_t)SLOTS * D::kQuartet * sizeof(R) + 2 * (size_t)D::NCART * sizeof(int) +
-                       (ORD == 1 ? 3 * sizeof(double) * (size_t)o.smem_atoms : 0);
+  constexpr size_t kTables = (size_t)SLOTS * D::kQuartet * sizeof(R) + 2 * (size_t)D::NCART * sizeof(int);
+  const size_t bytes = kTables + (ORD == 1 ? 3 * sizeof(double) * (size_t)o.smem_atoms : 0);
   auto k = rys3_kernel<LA, LB, LC, LD, ORD, R, BLOCK, SPLIT>;
-  if (bytes > 48 * 1024 && cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes) != cudaSuccess)
-    return false;
+  if (!allow_shared<kTables + (ORD == 1 ? kGradSmemBytes : 0)>(k, bytes)) return false;
   int grid = (nq + QB - 1) / QB;
   if (max_blocks > 0 && grid > max_blocks) grid = max_blocks;
   k<<<grid, BLOCK, bytes, s>>>(a, o, pure, q, nq);
