@@ -110,6 +110,13 @@ __host__ __device__ constexpr double boys_tmax_d(int M) {
   constexpr double t[11] = {36.0, 39.0, 43.0, 46.0, 49.0, 51.0, 54.0, 56.0, 58.0, 61.0, 63.0};
   return t[M];
 }
+// Grid points of order M that an FP64 evaluation can reach, and the rows of the orders below M.
+__host__ __device__ constexpr int boys_points_d(int M) { return (int)(boys_tmax_d(M) * 32.0) + 1; }
+__host__ __device__ constexpr int boys_rows_below_d(int M) {
+  int n = 0;
+  for (int m = 0; m < M; ++m) n += boys_points_d(m);
+  return n;
+}
 #define BOYS_MMAX 10             // orders M = 0 .. 10 have rows
 #define BOYS_ROW_D 6             // values per FP64 row
 #define BOYS_ROW_F 8             // values per FP32 row
@@ -117,7 +124,8 @@ __host__ __device__ constexpr double boys_tmax_d(int M) {
 // The FP64 evaluation; row(k, r0, r1, r2) reads the row of grid point k of order M.
 template <int M, class Row>
 __device__ __forceinline__ void boys_eval_d(double T, double pre, const Row& row, double* F) {
-  if (T < boys_tmax_d(M)) {
+  constexpr double tmax = boys_tmax_d(M);
+  if (T < tmax) {
     // nearest grid index without int/float conversions (they go through the narrow XU
     // pipe): adding 1.5 * 2^52 leaves round(T / h) in the low mantissa bits
     const double sh = T * 32.0 + 6755399441055744.0;
@@ -187,14 +195,15 @@ __device__ __forceinline__ void boys_eval_f(float T, float pre, const Row& row, 
 
 template <typename R>
 struct BoysTable {
-  const R* __restrict__ tab;  // [BOYS_MMAX + 1][BOYS_NGRID_D or _F][BOYS_ROW_D or _F]
+  const R* __restrict__ tab;  // per order boys_points_d(M) rows of BOYS_ROW_D, or BOYS_NGRID_F of BOYS_ROW_F
 
   template <int M>
   __device__ __forceinline__ void eval(R T, R pre, R* F) const {
     static_assert(M <= BOYS_MMAX, "Boys order beyond the table");
     if constexpr (sizeof(R) == 8) {
       boys_eval_d<M>(T, pre, [&](int k, double2& r0, double2& r1, double2& r2) {
-        const double2* r = reinterpret_cast<const double2*>(tab + (size_t)M * BOYS_NGRID_D * BOYS_ROW_D) + 3 * k;
+        constexpr int first = boys_rows_below_d(M);
+        const double2* r = reinterpret_cast<const double2*>(tab) + 3 * (first + k);
         r0 = r[0], r1 = r[1], r2 = r[2];
       }, F);
     } else {
@@ -222,9 +231,6 @@ __host__ __device__ constexpr int npure_of(int L) { return 2 * L + 1; }
 #define BOYS_PLANES_D 3
 #define BOYS_STAGED_MMAX 4       // orders that are staged (classes of la + lb + lc + ld up to it)
 
-// Grid points of order M that an FP64 evaluation can reach.
-__host__ __device__ constexpr int boys_points_d(int M) { return (int)(boys_tmax_d(M) * 32.0) + 1; }
-
 template <typename R>
 __host__ __device__ constexpr int boys_plane_bytes(int M) {  // 55 kB (M = 0) to 75 kB (M = 4) in FP64, 5.8 kB in FP32
   return 16 * (sizeof(R) == 8 ? BOYS_PLANES_D * boys_points_d(M) : BOYS_NGRID_F);
@@ -243,8 +249,9 @@ struct BoysShared {
     static_assert(M == MS && M <= BOYS_STAGED_MMAX, "the staged table holds one order");
     if constexpr (sizeof(R) == 8) {
       boys_eval_d<M>(T, pre, [&](int k, double2& r0, double2& r1, double2& r2) {
+        constexpr int n = boys_points_d(M);
         const double2* P = reinterpret_cast<const double2*>(tab) + k;
-        r0 = P[0], r1 = P[boys_points_d(M)], r2 = P[2 * boys_points_d(M)];
+        r0 = P[0], r1 = P[n], r2 = P[2 * n];
       }, F);
     } else {
       boys_eval_f<M>(T, pre, [&](int k) { return reinterpret_cast<const float4*>(tab)[k]; }, F);

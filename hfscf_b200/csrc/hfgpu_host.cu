@@ -115,10 +115,10 @@ std::vector<double> boys_table_d() {
     memcpy(&x, &u, 8);
     return x;
   };
-  std::vector<double> t((size_t)(BOYS_MMAX + 1) * BOYS_NGRID_D * BOYS_ROW_D);
+  std::vector<double> t((size_t)boys_rows_below_d(BOYS_MMAX + 1) * BOYS_ROW_D);
   for (int M = 0; M <= BOYS_MMAX; ++M)
-    for (int k = 0; k < BOYS_NGRID_D; ++k) {
-      double* row = &t[((size_t)M * BOYS_NGRID_D + k) * BOYS_ROW_D];
+    for (int k = 0; k < boys_points_d(M); ++k) {
+      double* row = &t[(size_t)(boys_rows_below_d(M) + k) * BOYS_ROW_D];
       auto taylor = [&](long double d) {
         long double s = 0.0L;
         for (int j = NT - 1; j >= 0; --j) s = F[(size_t)k * NM + M + j] + s * d / (j + 1);
@@ -153,7 +153,7 @@ std::vector<double> boys_planes_d(const std::vector<double>& rows) {
     for (int k = 0; k < boys_points_d(M); ++k)
       for (int j = 0; j < BOYS_PLANES_D; ++j)
         memcpy(&t[M * per + ((size_t)j * boys_points_d(M) + k) * 2],
-               &rows[((size_t)M * BOYS_NGRID_D + k) * BOYS_ROW_D + 2 * j], 16);
+               &rows[(size_t)(boys_rows_below_d(M) + k) * BOYS_ROW_D + 2 * j], 16);
   return t;
 }
 std::vector<float> boys_planes_f(const std::vector<float>& rows) {
