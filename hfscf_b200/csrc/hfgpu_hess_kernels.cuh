@@ -288,7 +288,7 @@ __global__ void __launch_bounds__(128) hess_kernel(GradArgs<double> a, HessOut o
   const Strided<double> h45{a.scratch + tid + (size_t)(Tab::NVSLOT + Tab::NHSLOT) * a.scratch_threads,
                             a.scratch_threads};
   const int np = a.nparts > 1 ? a.nparts : 1, p0 = np > 1 ? a.part : 0;
-  for (int t = tid; t < nq; t += nthr) {
+  for (long long t = tid; t < nq; t += nthr) {
     const int2 pq = quartets[(size_t)t * np + p0];
     const PairInfo P = a.pairs[pq.x];
     const PairInfo Q = a.pairs[pq.y];
@@ -377,11 +377,12 @@ __global__ void __launch_bounds__(kHessLineThreads) hess_line_kernel(GradArgs<do
   const Strided<double> h45{hess_sh + threadIdx.x, kHessLineStride};
   const int np = a.nparts > 1 ? a.nparts : 1, p0 = np > 1 ? a.part : 0;
   // whole warps stay in the loop together (lanes past the end add nothing), for hess_add_warp
-  for (int t = tid; t - (int)(threadIdx.x & 31) < nq; t += nthr) {
-    const bool valid = t < nq;
+  const int lane = threadIdx.x & 31;
+  for (int t0 = tid - lane; t0 < nq;) {  // t0, the warp's first quartet, never passes nq (t0 + nthr can pass 2^31)
+    const bool valid = lane < nq - t0;
     int at[4] = {0, 0, 0, 0};
     if (valid) {
-      const int2 pq = quartets[(size_t)t * np + p0];
+      const int2 pq = quartets[(size_t)(t0 + lane) * np + p0];
       const PairInfo P = a.pairs[pq.x];
       const PairInfo Q = a.pairs[pq.y];
       at[0] = P.atom_a;
@@ -394,5 +395,7 @@ __global__ void __launch_bounds__(kHessLineThreads) hess_line_kernel(GradArgs<do
         hess_line_quartet<LA, LB, LC, LD, false, Line>(a, pq, P, Q, h45);
     }
     hess_add_warp(valid, hess_sh + (threadIdx.x & ~31), kHessLineStride, 1, at, o.hess, 3 * o.natoms);
+    if (nthr >= nq - t0) break;
+    t0 += nthr;
   }
 }

@@ -125,7 +125,7 @@ __global__ void __launch_bounds__(BLOCK) rys_deriv_kernel(GradArgs<R> a, RysOut 
     for (int i = threadIdx.x; i < 3 * o.smem_atoms; i += BLOCK) gsum[i] = 0.0;
   __syncthreads();
   const int np = a.nparts > 1 ? a.nparts : 1, p0 = np > 1 ? a.part : 0;
-  for (int q0 = blockIdx.x * GROUPS; q0 < nq; q0 += gridDim.x * GROUPS) {
+  for (long long q0 = rys_first(blockIdx.x, 1, 0, GROUPS); q0 < nq; q0 += rys_stride(gridDim.x, 1, GROUPS)) {
     // groups of a warp run in step: one past the end works on quartet nq - 1 with no primitives
     const bool live = q0 + grp < nq;
     const int2 pq = quartets[(size_t)(live ? q0 + grp : nq - 1) * np + p0];
@@ -291,8 +291,6 @@ static bool launch_rys(const GradArgs<R>& a, const RysOut& o, int pure, const in
   const size_t bytes = kTables + (ORD == 1 ? 3 * sizeof(double) * (size_t)o.smem_atoms : 0);
   auto k = rys_deriv_kernel<LA, LB, LC, LD, ORD, R, G, BLOCK>;
   if (!allow_shared<kTables + (ORD == 1 ? kGradSmemBytes : 0)>(k, bytes)) return false;
-  int grid = (nq + GROUPS - 1) / GROUPS;
-  if (max_blocks > 0 && grid > max_blocks) grid = max_blocks;
-  k<<<grid, BLOCK, bytes, s>>>(a, o, pure, q, nq);
+  k<<<rys_blocks(nq, 1, GROUPS, max_blocks), BLOCK, bytes, s>>>(a, o, pure, q, nq);
   return true;
 }

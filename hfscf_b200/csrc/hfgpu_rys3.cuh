@@ -44,8 +44,8 @@ __global__ void __launch_bounds__(BLOCK) rys3_kernel(GradArgs<R> a, RysOut o, in
     for (int i = threadIdx.x; i < 3 * o.smem_atoms; i += BLOCK) gsum[i] = 0.0;
   __syncthreads();
   const int np = a.nparts > 1 ? a.nparts : 1, p0 = np > 1 ? a.part : 0;
-  for (int q0 = (blockIdx.x * WARPS + warp) * QW; q0 < nq; q0 += gridDim.x * WARPS * QW) {
-    const int qi = q0 + slot / SPLIT;
+  for (long long q0 = rys_first(blockIdx.x, WARPS, warp, QW); q0 < nq; q0 += rys_stride(gridDim.x, WARPS, QW)) {
+    const long long qi = q0 + slot / SPLIT;
     const bool live = qi < nq;
     const int2 pq = quartets[(size_t)(live ? qi : nq - 1) * np + p0];
     const PairInfo P = a.pairs[pq.x];
@@ -192,8 +192,6 @@ static bool launch_rys3(const GradArgs<R>& a, const RysOut& o, int pure, const i
   const size_t bytes = kTables + (ORD == 1 ? 3 * sizeof(double) * (size_t)o.smem_atoms : 0);
   auto k = rys3_kernel<LA, LB, LC, LD, ORD, R, BLOCK, SPLIT>;
   if (!allow_shared<kTables + (ORD == 1 ? kGradSmemBytes : 0)>(k, bytes)) return false;
-  int grid = (nq + QB - 1) / QB;
-  if (max_blocks > 0 && grid > max_blocks) grid = max_blocks;
-  k<<<grid, BLOCK, bytes, s>>>(a, o, pure, q, nq);
+  k<<<rys_blocks(nq, 1, QB, max_blocks), BLOCK, bytes, s>>>(a, o, pure, q, nq);
   return true;
 }

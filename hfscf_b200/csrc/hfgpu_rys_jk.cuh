@@ -26,8 +26,8 @@ __global__ void __launch_bounds__(BLOCK) rys_quartet_kernel(QuartetArgs<double> 
   __syncthreads();
   const JKArgs<R>& a = qa.jk;
   nq = launch_count(qa, nq);
-  for (int qi = blockIdx.x * WARPS + warp; qi < nq; qi += gridDim.x * WARPS) {
-    const int2 pq = quartets[quartet_slot(qa, qi)];
+  for (long long qi = rys_first(blockIdx.x, WARPS, warp, 1); qi < nq; qi += rys_stride(gridDim.x, WARPS, 1)) {
+    const int2 pq = quartets[quartet_slot(qa, (int)qi)];
     const PairInfo P = a.pairs[pq.x];
     const PairInfo Q = a.pairs[pq.y];
     bool skip = false;
@@ -117,6 +117,6 @@ static bool launch_rys_quartet(const QuartetArgs<double>& a, const double* tab, 
   auto k = rys_quartet_kernel<LA, LB, LC, LD, BLOCK>;
   if (bytes > 48 * 1024 && cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes) != cudaSuccess)
     return false;
-  k<<<(nq + BLOCK / 32 - 1) / (BLOCK / 32), BLOCK, bytes, s>>>(a, tab, q, nq);
+  k<<<rys_blocks(nq, BLOCK / 32, 1, 0), BLOCK, bytes, s>>>(a, tab, q, nq);
   return true;
 }

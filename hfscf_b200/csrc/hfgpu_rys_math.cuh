@@ -6,6 +6,21 @@
 
 #include "generated/rys_layout.cuh"
 
+// Walk of a launch's quartets, in 64 bits: without a block limit the stride covers the whole list, so that
+// a 32-bit index would pass 2^31 in its first step from 2^30 quartets on, turn negative and read in front
+// of the list.  Each of the `walkers` of a block (its warps, or one) takes `per` quartets at a time.
+__host__ __device__ constexpr long long rys_first(unsigned block, int walkers, int walker, int per) {
+  return ((long long)block * walkers + walker) * per;
+}
+__host__ __device__ constexpr long long rys_stride(unsigned blocks, int walkers, int per) {
+  return (long long)blocks * walkers * per;
+}
+// Blocks of a launch over nq quartets, at most `most` (0: no limit).
+__host__ __device__ constexpr unsigned rys_blocks(long long nq, int walkers, int per, int most) {
+  const long long n = (nq + (long long)walkers * per - 1) / ((long long)walkers * per);
+  return (unsigned)(most > 0 && n > most ? most : n);
+}
+
 // Value v of the n-point rule at T: squared root v (v < n) or weight v - n.
 template <int N>
 __device__ __forceinline__ double rys_value(const double* __restrict__ tab, double T, int v) {
