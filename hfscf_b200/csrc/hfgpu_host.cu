@@ -668,11 +668,16 @@ int compute_schwarz(hfgpu_handle* h) {
   for (int c = 0; c < kPairClasses; ++c) {
     const int b = h->class_begin[c], e = h->class_begin[c + 1];
     if (e <= b) continue;
-    qa.warp_max = class_warp_max(h, quartet_class(c, c));
-    qa.warp_threads = class_warp_threads(h, quartet_class(c, c));
-    qa.block = h->sched_block[quartet_class(c, c)];
-    qa.capped = h->sched_cap[quartet_class(c, c)];
-    if (!launch_quartet_d(h, quartet_class(c, c), qa, h->d_quart.as<int2>() + b, e - b, h->stream))
+    // One form per class whatever the schedule, the options and the lists of an earlier geometry say: the
+    // factors decide which side of the cut-off a quartet is on, and the same geometry gives the same ones.
+    // Rys quadrature where the class has it: there are few diagonal quartets, and one thread each would be
+    // latency alone.
+    const int qc = quartet_class(c, c);
+    const int2* q = h->d_quart.as<int2>() + b;
+    qa.block = hfgpu::kClassLaunchers[qc]->block_default;
+    if (!hfgpu::kRysLaunchers[qc]->quartet)
+      hfgpu::kClassLaunchers[qc]->quartet_d(qa, q, e - b, h->stream);
+    else if (!hfgpu::kRysLaunchers[qc]->quartet(qa, h->rys_tab, q, e - b, h->stream))
       return fail(h, HFGPU_ERR_CUDA, "schwarz launch: shared memory");
     HF_CHECK_LAUNCH(h, "schwarz kernel");
   }
