@@ -269,8 +269,8 @@ struct hfgpu_handle {
   // by Rys quadrature, -1 the default (grad_form_of)
   int grad_form[21];
   unsigned grad_class_mask = ~0u;       // classes a gradient launches (autotuning runs one at a time)
-  // Hessian form (hfgpu_set_hess_form): -1 by class, 0 one thread per quartet, 1 and 2 a group of
-  // threads per quartet by Rys quadrature (largest, smallest group), 3 one thread per quartet on
+  // Hessian form (hfgpu_set_hess_form): -1 by class, 0 one thread per quartet, 1 and 2 Rys quadrature
+  // (the largest group of threads per quartet, the class's measured form), 3 one thread per quartet on
   // straight-line code (where the class has it)
   int hess_form = -1;
   int purify_blocks = -1;               // co-resident blocks of the cooperative purification (0: not available)
@@ -2153,6 +2153,11 @@ int hfgpu_grad2e_uhf_backward(hfgpu_handle* h, const double* Da, const double* D
 constexpr size_t kHessScratchBudget = (size_t)2 << 30;
 constexpr long long kHessLineGrid = 4 * 148;     // straight-line form: at most four blocks per SM, grid-stride
 
+// The default form of a class's Hessian (see form_of in hess_device_impl).
+static int hess_default_form(const hfgpu_handle* h, int c) {
+  return hfgpu::kRysLaunchers[c]->hess_variant < 0 && !rys_split_pays(h, c, 0.25) ? 3 : 2;
+}
+
 static int hess_device_impl(hfgpu_handle* h, const double* DJ, double cJ, int nK, const double* DK, double cK,
                             double* hess) {
   if (!h->have_geometry) return fail(h, HFGPU_ERR_STATE, "no geometry set");
@@ -2182,15 +2187,16 @@ static int hess_device_impl(hfgpu_handle* h, const double* DJ, double cJ, int nK
     thr = std::min<long long>(thr, ((nq + 127) / 128) * 128);
     return std::max<long long>(128, thr / 128 * 128);
   };
-  // form per class: 0 one thread per quartet on global scratch, 1 and 2 a group of threads per quartet
-  // by Rys quadrature (1 the largest group of the class, 2 the smallest), 3 one thread per quartet on
+  // form per class: 0 one thread per quartet on global scratch, 1 and 2 Rys quadrature (1 the class's
+  // largest group of threads per quartet, 2 what was measured best of the rest: three threads, ten such
+  // triples where quartets are few, or the larger classes' group), 3 one thread per quartet on
   // straight-line register code (the classes that have it; a class without it takes the default).
-  // Default: Rys quadrature with the class's measured group size, or the straight-line form
+  // Default: form 2, or form 3 for a class without a Rys default unless its quartets are few
   // (rys_defaults in gen_eri.py).
   auto form_of = [&](int c) -> int {
     int f = h->hess_cls_form[c] >= 0 ? h->hess_cls_form[c] : h->hess_form;
     if (f == 3 && !hfgpu::kHessLaunchers[c]->has_line) f = -1;
-    return f < 0 && hfgpu::kRysLaunchers[c]->hess_variant < 0 && !rys_split_pays(h, c, 0.25) ? 3 : f;
+    return f < 0 ? hess_default_form(h, c) : f;
   };
   // classes largest first, round-robin over the auxiliary streams; each stream's slice is the
   // largest need of its classes
@@ -2235,8 +2241,8 @@ static int hess_device_impl(hfgpu_handle* h, const double* DJ, double cJ, int nK
     }
     if (form_of(c) != 0) {
       const hfgpu::RysLaunchers* Y = hfgpu::kRysLaunchers[c];
-      int v = form_of(c) == 1 ? 2 : (form_of(c) == 2 ? 0 : Y->hess_variant);
-      if (form_of(c) < 0 && Y->hess[hfgpu::kRysSplit] && rys_split_pays(h, c, 0.25)) v = hfgpu::kRysSplit;
+      int v = form_of(c) == 1 ? 2 : (Y->hess_variant < 0 ? hfgpu::kRysThree : Y->hess_variant);
+      if (form_of(c) != 1 && Y->hess[hfgpu::kRysSplit] && rys_split_pays(h, c, 0.25)) v = hfgpu::kRysSplit;
       if (!Y->hess[v](gd, ro, h->pure, q + h->q_beg[c], (int)nq, 0, h->aux[stream_of[c]]))
         return fail(h, HFGPU_ERR_CUDA, "Hessian launch: shared memory");
       HF_CHECK_LAUNCH(h, "hess kernel");
@@ -2773,9 +2779,8 @@ int hfgpu_set_grad_forms(hfgpu_handle* h, const int* forms) {
   return HFGPU_OK;
 }
 
-// Hessian form per class: each class alone, one thread (global scratch), Rys quadrature with the
-// largest or the smallest group of threads per quartet, or one thread on straight-line code where the
-// class has it, on RHF weights of the device density D; the fastest is kept.
+// Hessian form per class: each class alone in forms 0 to 3 (hess_device_impl), one of which is its
+// default, on RHF weights of the device density D; the fastest is kept where whole Hessians gain.
 int hfgpu_autotune_hess(hfgpu_handle* h, const double* D, int repeats, int* forms) {
   if (!h || !D) return HFGPU_ERR_INVALID;
   DeviceGuard dev_guard(h);
@@ -2826,6 +2831,18 @@ int hfgpu_autotune_hess(hfgpu_handle* h, const double* D, int repeats, int* form
     }
     h->hess_cls_form[c] = best_form;
   }
+  // the classes of a call share the GPU, so the fastest forms alone need not be together: whole Hessians
+  // in them (butane/cc-pVDZ 20.5 ms) against whole Hessians in the defaults (18.4)
+  h->hess_class_mask = ~0u;
+  float alone_ms = 0.f, default_ms = 0.f;
+  if ((rc = tuner_time(h, hessian, repeats, e0, e1, restore.flush, &alone_ms))) return rc;
+  int keep[hfgpu::kNumClasses];
+  for (int c = 0; c < hfgpu::kNumClasses; ++c) {
+    keep[c] = h->hess_cls_form[c];
+    if (keep[c] >= 0) h->hess_cls_form[c] = hess_default_form(h, c);
+  }
+  if ((rc = tuner_time(h, hessian, repeats, e0, e1, restore.flush, &default_ms))) return rc;
+  if (alone_ms < default_ms) std::copy(keep, keep + hfgpu::kNumClasses, h->hess_cls_form);
   if (forms)
     for (int c = 0; c < hfgpu::kNumClasses; ++c) forms[c] = h->hess_cls_form[c];
   hb.release();

@@ -385,14 +385,14 @@ class Engine:
         return H
 
     def set_hess_form(self, form: int):
-        """hfgpu_set_hess_form: -1 by class (default), 0 thread (global scratch), 1 and 2 Rys quadrature
-        with the class's largest and smallest group of threads per quartet, 3 thread on straight-line
-        register code where the class has it."""
+        """hfgpu_set_hess_form: -1 by class (default), 0 thread (global scratch), 1 Rys quadrature with the
+        class's largest group of threads per quartet, 2 Rys quadrature as the default takes it, 3 thread
+        on straight-line register code where the class has it."""
         self._check(lib().hfgpu_set_hess_form(self.h, ctypes.c_int(form)))
 
     def autotune_hess(self, D, repeats=2):
         """hfgpu_autotune_hess on density D (host array, device tensor or device pointer): per
-        class the fastest of the thread, Rys (largest and smallest group) and straight-line forms;
+        class the fastest of the thread, Rys (largest group, default) and straight-line forms;
         returns the chosen forms (0, 1, 2, 3)."""
         import torch
         if isinstance(D, int):

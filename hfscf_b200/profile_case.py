@@ -49,7 +49,7 @@ def main(argv=None):
                     help="thread-form variant for every class (schedule column 3: 0 plain, 1 capped, "
                          "2 staged persistent)")
     ap.add_argument("--hess-form", type=int, choices=(-1, 0, 1, 2, 3), default=-1,
-                    help="hess: -1 default per class, 0 one thread, 1 / 2 largest / smallest Rys group, 3 straight-line")
+                    help="hess: -1 default per class, 0 one thread, 1 / 2 Rys quadrature, largest group / as by default, 3 straight-line")
     a = ap.parse_args(argv)
     if not torch.cuda.is_available():
         raise SystemExit("profile_case needs a CUDA device")

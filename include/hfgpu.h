@@ -142,15 +142,16 @@ int hfgpu_hess2e_uhf(hfgpu_handle* h, const double* Da, const double* Db, double
  * with three threads per quartet, or a group of threads for the larger classes, and one thread per
  * quartet on straight-line register code for (ss|ss); 0 one thread per quartet on global scratch
  * everywhere, 1 Rys quadrature with the class's largest group of threads per quartet everywhere,
- * 2 with its smallest group, 3 the straight-line form wherever the class has it ((ss|ss), (ps|ss),
+ * 2 Rys quadrature as the default takes it everywhere, 3 the straight-line form wherever the class has it ((ss|ss), (ps|ss),
  * (ps|ps), (pp|ss), (pp|ps), (ds|ss), (ds|ps), (dp|ss); the default elsewhere).  The results agree
  * to rounding. */
 int hfgpu_set_hess_form(hfgpu_handle* h, int form);
-/* Per class (HFGPU_NUM_CLASSES ints: 0 thread, 1 largest group, 2 smallest group, 3 straight-line, -1 the rule of
- * hfgpu_set_hess_form), as hfgpu_autotune_hess returns them. */
+/* Per class (HFGPU_NUM_CLASSES ints: 0 thread, 1 largest group, 2 the Rys form of the default, 3 straight-line,
+ * -1 the rule of hfgpu_set_hess_form), as hfgpu_autotune_hess returns them. */
 int hfgpu_set_hess_forms(hfgpu_handle* h, const int* forms);
 /* Times every class alone in each form on RHF weights of the device density D (median of
- * `repeats` runs, L2 flushed before each) and keeps the faster per class; forms (may be NULL)
+ * `repeats` runs, L2 flushed before each) and keeps the fastest per class, or the defaults where a whole
+ * Hessian is faster with those; forms (may be NULL)
  * receives the choice.  No counterpart in the reference (which has one CPU code path). */
 int hfgpu_autotune_hess(hfgpu_handle* h, const double* D, int repeats, int* forms);
 
