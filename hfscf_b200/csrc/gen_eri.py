@@ -1097,14 +1097,19 @@ def rys_inst(c, t):
     n = ncart(c[0]) * ncart(c[1]) * ncart(c[2]) * ncart(c[3])
     cl = ", ".join(map(str, c))
 
+    gv, p64, hv = rys_defaults(c)
+
     def row(order, real):
-        fns = [f"&launch_rys<{cl}, {order}, {real}, {g}>" for g in rys_groups(*c)]
+        # the group sizes that a form or a default reaches: gradients all three of the op-table classes,
+        # Hessians the largest (form 1) and the default
+        reached = (0, 1, 2) if order == 1 and gv >= 0 else ((2, hv) if order == 2 else ())
+        fns = [f"&launch_rys<{cl}, {order}, {real}, {g}>" if k in reached else "nullptr"
+               for k, g in enumerate(rys_groups(*c))]
         for split in (1, 10):
             fns.append(f"&launch_rys3<{cl}, {order}, {real}, {split}>" if n <= RYS_THREE_MAX_CART[order, real]
                        else "nullptr")
         return ", ".join(fns)
 
-    gv, p64, hv = rys_defaults(c)
     return RYS_INST_TEMPLATE.format(t=t, la=c[0], lb=c[1], lc=c[2], ld=c[3], gv=gv, p64=p64, hv=hv, gd=row(1, "double"),
                                     gf=row(1, "float"), hd=row(2, "double"),
                                     qf=f"&launch_rys_quartet<{cl}>" if c in RYS_QUARTET else "nullptr")

@@ -11,8 +11,8 @@ struct RysOut;
 
 namespace hfgpu {
 
-// Variants: groups of threads over shared-memory tables, fewest, middle and most threads per quartet,
-// and (null for the larger classes) three threads per quartet, one per direction (kRysThree), or ten such
+// Variants: groups of threads over shared-memory tables, fewest, middle and most threads per quartet (null
+// where no form or default reaches them), and (null for the larger classes) three threads per quartet, one per direction (kRysThree), or ten such
 // triples per quartet (kRysSplit).
 constexpr int kRysVariants = 5, kRysThree = 3, kRysSplit = 4;
 
