@@ -18,11 +18,21 @@
 #pragma once
 #include "hfgpu_kernels.cuh"
 
-// Hessian output of a launch: 3 natoms x 3 natoms, row-major, half of it (HessEntry).
+// Hessian output of a launch: 3 natoms x 3 natoms, row-major, half of it (HessEntry), in `copies` (a power
+// of two) partial sums one after another, of which a block adds into one: the rounding of a sum grows
+// with its size, and each copy's is a share of the whole.  What a Hessian leaves of translational
+// invariance shows it (the entries largely cancel over the atoms): (H2O)4 and n-octane at their SCF
+// densities 6e-13 to 2e-12 with one copy, 4e-13 to 1.3e-12 with 32, and no less with 128 or 512 (what is left
+// comes from the quartets); random densities 5 to 7 times less than with one.  Times as with one copy.
 struct HessOut {
   double* __restrict__ hess;
   int natoms;
+  int copies;
 };
+
+__device__ __forceinline__ double* hess_copy(double* hess, int natoms, int copies) {
+  return hess + (size_t)(blockIdx.x & (copies - 1)) * 9 * natoms * natoms;
+}
 
 // Executor of a table-mode Hessian class.  Weight sets, in the generator's order:
 // 1, 2a_a, 2a_b, 2a_c, (2a_a)^2, (2a_b)^2, (2a_c)^2, 2a_a 2a_b, 2a_a 2a_c, 2a_b 2a_c.
@@ -213,12 +223,14 @@ __device__ __forceinline__ void hess_add_warp(bool valid, const double* h45, int
   __syncwarp();
 }
 
-// hess += U + U^T.
-static __global__ void hess_finish_kernel(const double* __restrict__ U, double* __restrict__ hess, int n3) {
-  const size_t e = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (e >= (size_t)n3 * n3) return;
-  const size_t r = e / n3, c = e % n3;
-  hess[e] += U[e] + U[c * n3 + r];
+// hess += U + U^T, U the sum of the copies.
+static __global__ void hess_finish_kernel(const double* __restrict__ U, double* __restrict__ hess, int n3, int copies) {
+  const size_t e = (size_t)blockIdx.x * blockDim.x + threadIdx.x, nn = (size_t)n3 * n3;
+  if (e >= nn) return;
+  const size_t r = e / n3, t = e % n3 * n3 + r;
+  double v = 0.0;
+  for (int k = 0; k < copies; ++k) v += U[k * nn + e] + U[k * nn + t];
+  hess[e] += v;
 }
 
 template <int LA, int LB, int LC, int LD, bool PURE, typename Tab>
@@ -297,7 +309,7 @@ __global__ void __launch_bounds__(128) hess_kernel(GradArgs<double> a, HessOut o
     else
       hess_quartet<LA, LB, LC, LD, false, Tab>(a, tid, pq, P, Q);
     const int at[4] = {P.atom_a, P.atom_b, Q.atom_a, Q.atom_b};
-    hess_add_block(h45, at, o.hess, 3 * o.natoms, 0, 1);
+    hess_add_block(h45, at, hess_copy(o.hess, o.natoms, o.copies), 3 * o.natoms, 0, 1);
   }
 }
 
@@ -394,7 +406,8 @@ __global__ void __launch_bounds__(kHessLineThreads) hess_line_kernel(GradArgs<do
       else
         hess_line_quartet<LA, LB, LC, LD, false, Line>(a, pq, P, Q, h45);
     }
-    hess_add_warp(valid, hess_sh + (threadIdx.x & ~31), kHessLineStride, 1, at, o.hess, 3 * o.natoms);
+    hess_add_warp(valid, hess_sh + (threadIdx.x & ~31), kHessLineStride, 1, at,
+                  hess_copy(o.hess, o.natoms, o.copies), 3 * o.natoms);
     if (nthr >= nq - t0) break;
     t0 += nthr;
   }

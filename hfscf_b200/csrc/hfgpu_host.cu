@@ -371,6 +371,14 @@ int primwarp_group(const hfgpu_handle* h, int c, int seg, long long nq, bool fp3
   return best;
 }
 
+// Partial sums of a Hessian (HessOut): 32 while all together stay within 4 MB, which the L2 cache holds
+// beside everything else (up to 42 atoms; one copy from 242 atoms on).
+int hess_copies(const hfgpu_handle* h) {
+  int copies = 32;
+  while (copies > 1 && sizeof(double) * 9 * (size_t)h->natoms * h->natoms * copies > ((size_t)4 << 20)) copies /= 2;
+  return copies;
+}
+
 int cuda_fail(hfgpu_handle* h, cudaError_t e, const char* where) {
   return fail(h, e == cudaErrorMemoryAllocation ? HFGPU_ERR_NOMEM : HFGPU_ERR_CUDA,
               std::string(where) + ": " + cudaGetErrorString(e));
@@ -617,7 +625,7 @@ int build_pairs(hfgpu_handle* h) {
   HF_CUDA(h, h->d_alpha_d.ensure(sizeof(double) * 2 * np));
   HF_CUDA(h, h->d_alpha_f.ensure(sizeof(float) * 2 * np));
   // the Hessian's half matrix now, unless large, so that a first Hessian call may be inside a capture
-  const size_t hess_bytes = sizeof(double) * 9 * (size_t)h->natoms * h->natoms;
+  const size_t hess_bytes = sizeof(double) * 9 * (size_t)h->natoms * h->natoms * hess_copies(h);
   if (!h->batched && hess_bytes <= (16u << 20)) HF_CUDA(h, h->d_hess.ensure(hess_bytes));
   cudaStream_t s = h->stream;
   HF_CUDA(h, cudaMemcpyAsync(h->d_pairs.p, h->pairs.data(), sizeof(PairInfo) * h->pairs.size(), cudaMemcpyHostToDevice, s));
@@ -1564,7 +1572,7 @@ static int grad_device_impl(hfgpu_handle* h, const double* DJ, double cJ, int nK
   gf.mol_off = gd.mol_off;
   gf.mol_n = gd.mol_n;
   gd.smem_atoms = gf.smem_atoms = grad_smem_atoms(h);
-  const RysOut ro{h->rys_tab, nullptr, h->natoms, gd.smem_atoms};
+  const RysOut ro{h->rys_tab, nullptr, h->natoms, gd.smem_atoms, 1};
   gd.part = gf.part = h->part;
   gd.nparts = gf.nparts = h->nparts;
   const int2* q = h->d_quart.as<int2>();
@@ -2175,12 +2183,13 @@ static int hess_device_impl(hfgpu_handle* h, const double* DJ, double cJ, int nK
   gd.part = h->part;
   gd.nparts = h->nparts;
   const size_t n3 = 3 * (size_t)h->natoms;
-  // the classes add into U, hess += U + U^T at the end
-  HF_CUDA(h, h->d_hess.ensure(sizeof(double) * n3 * n3));
+  // the classes add into the copies of U, hess += U + U^T at the end
+  const int copies = hess_copies(h);
+  HF_CUDA(h, h->d_hess.ensure(sizeof(double) * n3 * n3 * copies));
   double* U = h->d_hess.as<double>();
-  HF_CUDA(h, cudaMemsetAsync(U, 0, sizeof(double) * n3 * n3, h->stream));
-  HessOut o{U, h->natoms};
-  RysOut ro{h->rys_tab, U, h->natoms, 0};
+  HF_CUDA(h, cudaMemsetAsync(U, 0, sizeof(double) * n3 * n3 * copies, h->stream));
+  HessOut o{U, h->natoms, copies};
+  RysOut ro{h->rys_tab, U, h->natoms, 0, copies};
   const int2* q = h->d_quart.as<int2>();
   auto threads_of = [&](int slots, long long nq) -> long long {
     long long thr = (long long)(kHessScratchBudget / ((size_t)slots * sizeof(double)));
@@ -2259,7 +2268,7 @@ static int hess_device_impl(hfgpu_handle* h, const double* DJ, double cJ, int nK
     HF_CHECK_LAUNCH(h, "hess kernel");
   }
   if ((rc = join_streams(h))) return rc;
-  hess_finish_kernel<<<(unsigned)((n3 * n3 + 255) / 256), 256, 0, h->stream>>>(U, hess, (int)n3);
+  hess_finish_kernel<<<(unsigned)((n3 * n3 + 255) / 256), 256, 0, h->stream>>>(U, hess, (int)n3, copies);
   HF_CHECK_LAUNCH(h, "hess finish kernel");
   return HFGPU_OK;
 }

@@ -93,13 +93,13 @@ __device__ __forceinline__ void rys_weights(const GradArgs<R>& a, int pure, cons
   }
 }
 
-// Output of a launch: order 1 GradArgs::grad; order 2 hess, 3 natoms x 3 natoms row-major, half of it
-// (HessEntry).
+// Output of a launch: order 1 GradArgs::grad; order 2 hess and copies as in HessOut.
 struct RysOut {
   const double* __restrict__ tab;  // quadrature tables
   double* __restrict__ hess;
   int natoms;
   int smem_atoms;  // order 1: > 0 = the block sums its 3 x smem_atoms entries in shared memory first
+  int copies;
 };
 
 // G threads per quartet, BLOCK threads per block (BLOCK = G when G > 32), grid-stride over quartets.
@@ -248,7 +248,7 @@ __global__ void __launch_bounds__(BLOCK) rys_deriv_kernel(GradArgs<R> a, RysOut 
         for (int x = 0; x < 45; ++x) h45[x] = acc[x];
       rys_sync<G>();
       const int at[4] = {P.atom_a, P.atom_b, Q.atom_a, Q.atom_b};
-      if (live) hess_add_block(h45, at, o.hess, 3 * o.natoms, lane, G);
+      if (live) hess_add_block(h45, at, hess_copy(o.hess, o.natoms, o.copies), 3 * o.natoms, lane, G);
     }
     rys_sync<G>();
   }

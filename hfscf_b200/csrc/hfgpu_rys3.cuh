@@ -171,7 +171,7 @@ __global__ void __launch_bounds__(BLOCK) rys3_kernel(GradArgs<R> a, RysOut o, in
           h45[r < c ? rys_tri(r, c) : rys_tri(c, r)] = acc[6 + 3 * A + B];
         }
       const int at[4] = {P.atom_a, P.atom_b, Q.atom_a, Q.atom_b};
-      hess_add_warp(lead && d == 0 && live, base, 1, 15, at, o.hess, 3 * o.natoms);
+      hess_add_warp(lead && d == 0 && live, base, 1, 15, at, hess_copy(o.hess, o.natoms, o.copies), 3 * o.natoms);
     }
     __syncwarp();
   }
