@@ -1145,6 +1145,10 @@ RYS_HESS_THREE_MAX_CART = 81
 # at 2.9 per quartet (dp|pp) takes 1.20 against 1.84, on anthracene at 7.9 6.0 against 5.3; (pp|pp)
 # 0.48 / 1.25 and 2.0 / 4.5 at 4.1 and 15.4; (pp|ps), (ds|ps) and smaller lose even at 6.  FP64 only: in
 # FP32 its rounding moved the mixed gradient of anthracene by 1.6e-9 of its norm.
+# The groups also serve the FP32 share of the op-table classes: with every quartet in FP32 their error against
+# FP64 is a third of the op tables' (rms relative to the largest entry, mean of ten cases, tables and
+# groups: (dp|dp) 4.8e-7 and 1.7e-7, (dd|pp) 1.9e-7 and 6e-8, (dd|ds) 2.2e-7 and 8e-8, (dd|dp) 2.4e-7 and 8e-8,
+# (dd|dd) 2.9e-7 and 7e-8).
 RYS_GRAD_THREE_PRIMS = {(1, 1, 1, 1): 1000, (2, 0, 1, 1): 20, (2, 0, 2, 0): 1000, (2, 1, 1, 0): 9, (2, 1, 1, 1): 6,
                         (2, 1, 2, 0): 11, (2, 2, 0, 0): 1000, (2, 2, 1, 0): 8}
 

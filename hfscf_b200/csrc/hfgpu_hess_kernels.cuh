@@ -21,7 +21,7 @@
 // Hessian output of a launch: 3 natoms x 3 natoms, row-major, half of it (HessEntry), in `copies` (a power
 // of two) partial sums one after another, of which a block adds into one: the rounding of a sum grows
 // with its size, and each copy's is a share of the whole.  What a Hessian leaves of translational
-// invariance shows it (the entries largely cancel over the atoms): (H2O)4 and n-octane at their SCF
+// invariance shows it (the entries largely cancel over the atoms): (H2O)4 and n-octane at their core-guess
 // densities 6e-13 to 2e-12 with one copy, 4e-13 to 1.3e-12 with 32, and no less with 128 or 512 (what is left
 // comes from the quartets); random densities 5 to 7 times less than with one.  Times as with one copy.
 struct HessOut {
