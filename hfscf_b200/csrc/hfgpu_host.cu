@@ -2476,7 +2476,9 @@ int hfgpu_batch_eigh(hfgpu_handle* h, const double* A, double* W, double* V, int
   int rc = dev_guard.rc;
   if (rc) return rc;
   const size_t smem = jacobi_smem_bytes(nmax);
-  HF_CUDA(h, cudaFuncSetAttribute(batch_jacobi_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  // the kernel's limit, not this launch's: another thread may be about to launch it for larger molecules
+  HF_CUDA(h, cudaFuncSetAttribute(batch_jacobi_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                  (int)jacobi_smem_bytes(kJacobiMaxN)));
   const int* mol_n = reinterpret_cast<const int*>(h->d_mol.as<long long>() + h->nmol);
   batch_jacobi_kernel<<<h->nmol, kJacobiThreads, smem, h->stream>>>(A, nmax, mol_n, W, V, 30, sweeps);
   HF_CHECK_LAUNCH(h, "batched eigensolver");
@@ -2494,7 +2496,8 @@ int hfgpu_batch_purify_device(hfgpu_handle* h, const double* Fo, const int* nocc
   int rc = dev_guard.rc;
   if (rc) return rc;
   const size_t smem = batch_purify_smem_bytes(nmax);
-  HF_CUDA(h, cudaFuncSetAttribute(batch_purify_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  HF_CUDA(h, cudaFuncSetAttribute(batch_purify_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                  (int)batch_purify_smem_bytes(kBatchPurifyMaxN)));  // as for batch_jacobi_kernel
   const int* mol_n = reinterpret_cast<const int*>(h->d_mol.as<long long>() + h->nmol);
   batch_purify_kernel<<<h->nmol, kBatchPurifyThreads, smem, h->stream>>>(Fo, nmax, mol_n, nocc, max_steps, 1e-11, P,
                                                                           err);

@@ -1,6 +1,7 @@
 """Two handles on two host threads: a kernel's attributes belong to the kernel, so what one handle's launch
-sets must suit the other's.  Gradients of molecules of different size run in loops at the same time; every
-call succeeds and agrees with the same call alone (1e-10, the summation order of the atomic adds).
+sets must suit the other's.  Gradients of molecules of different size, or the batched eigensolver and
+purification, run in loops at the same time; every call succeeds, and gradients agree with the same call
+alone (1e-10, the summation order of the atomic adds).
 """
 import threading
 
@@ -50,3 +51,41 @@ def test_gradients_of_two_handles_on_two_threads():
     finally:
         for eng in engines:
             eng.close()
+
+
+def test_batched_linear_algebra_of_two_handles_on_two_threads():
+    import torch
+
+    from hfscf_b200 import batch
+    cases = []
+    for carbons in (2, 3):  # 60 and 85 functions: both kernels above 48 KB of shared memory, in different size
+        bs = _case(carbons)[0]
+        n = bs.nbf
+        A = np.random.default_rng(carbons).normal(size=(n, n))
+        cases.append((batch.BatchEngine([bs]), torch.from_numpy((A + A.T) / 2).cuda().reshape(1, n, n).contiguous(),
+                      torch.empty((1, n), dtype=torch.float64, device="cuda"),
+                      torch.empty((1, n, n), dtype=torch.float64, device="cuda"),
+                      torch.tensor([n // 3], dtype=torch.int32, device="cuda"),
+                      torch.empty(1, dtype=torch.float64, device="cuda")))
+    torch.cuda.synchronize()
+    failures = []
+    start = threading.Barrier(len(cases))
+
+    def loop(be, A, W, V, nocc, err):
+        start.wait()
+        try:
+            for _ in range(400):
+                be.eigh(A, W, V)
+                be.purify(A, nocc, V, err)
+        except E.HfgpuError as e:
+            failures.append(str(e))
+
+    threads = [threading.Thread(target=loop, args=c) for c in cases]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    torch.cuda.synchronize()
+    for c in cases:
+        c[0].close()
+    assert not failures, failures
