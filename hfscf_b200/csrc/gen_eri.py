@@ -897,7 +897,6 @@ static void launch_quartet_impl(const QuartetArgs<R>& a, const int2* q, int nq, 
       auto k = quartet_staged_kernel<{la}, {lb}, {lc}, {ld}, R>;
       const int bs = a.block > 0 ? a.block : 64;
       constexpr int smem = boys_plane_bytes<R>({la} + {lb} + {lc} + {ld});
-      if constexpr (smem > 48 * 1024) cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
       int dev = 0, sms = 148, per_sm = 1;
       cudaGetDevice(&dev);
       cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);

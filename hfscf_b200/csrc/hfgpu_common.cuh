@@ -121,33 +121,29 @@ __host__ __device__ constexpr int boys_rows_below_d(int M) {
 #define BOYS_ROW_D 6             // values per FP64 row
 #define BOYS_ROW_F 8             // values per FP32 row
 
-// The FP64 evaluation; row(k, r0, r1, r2) reads the row of grid point k of order M.
-template <int M, class Row>
+// The FP64 evaluation on the grid of 1/INVH: row(k, c, ek) reads the NC coefficients and e^-T_k of grid
+// point k of order M; e^d from its Taylor polynomial of degree NE.
+template <int M, int INVH, int NC, int NE, class Row>
 __device__ __forceinline__ void boys_eval_d(double T, double pre, const Row& row, double* F) {
   constexpr double tmax = boys_tmax_d(M);
   if (T < tmax) {
     // nearest grid index without int/float conversions (they go through the narrow XU
     // pipe): adding 1.5 * 2^52 leaves round(T / h) in the low mantissa bits
-    const double sh = T * 32.0 + 6755399441055744.0;
-    const double d = (sh - 6755399441055744.0) * BOYS_H_D - T;  // T_k - T, exact
-    double2 r0, r1, r2;
-    row(__double2loint(sh), r0, r1, r2);
-    double f = r2.x;
-    f = __hiloint2double(__double2loint(r2.x), 0) + f * d;
-    f = r1.y + f * d;
-    f = r1.x + f * d;
-    f = r0.y + f * d;
-    f = r0.x + f * d;
+    const double sh = T * INVH + 6755399441055744.0;
+    const double d = (sh - 6755399441055744.0) * (1.0 / INVH) - T;  // T_k - T, exact
+    double c[NC], ek;
+    row(__double2loint(sh), c, ek);
+    double f = c[NC - 1];
+#pragma unroll
+    for (int j = NC - 2; j >= 0; --j) f = c[j] + f * d;
     F[M] = f;
     if constexpr (M > 0) {
-      double x = 1.0 / 720.0;
-      x = 1.0 / 120.0 + d * x;
-      x = 1.0 / 24.0 + d * x;
-      x = 1.0 / 6.0 + d * x;
-      x = 0.5 + d * x;
-      x = 1.0 + d * x;
-      x = 1.0 + d * x;
-      const double e = r2.y * x, t2 = T + T;
+      constexpr double inv_fact[9] = {1.0,         1.0,         0.5,          1.0 / 6.0,    1.0 / 24.0,
+                                      1.0 / 120.0, 1.0 / 720.0, 1.0 / 5040.0, 1.0 / 40320.0};
+      double x = inv_fact[NE];
+#pragma unroll
+      for (int j = NE - 1; j >= 0; --j) x = inv_fact[j] + d * x;
+      const double e = ek * x, t2 = T + T;
 #pragma unroll
       for (int m = M; m > 0; --m) F[m - 1] = (t2 * F[m] + e) * (1.0 / (2 * m - 1));
     }
@@ -201,10 +197,14 @@ struct BoysTable {
   __device__ __forceinline__ void eval(R T, R pre, R* F) const {
     static_assert(M <= BOYS_MMAX, "Boys order beyond the table");
     if constexpr (sizeof(R) == 8) {
-      boys_eval_d<M>(T, pre, [&](int k, double2& r0, double2& r1, double2& r2) {
+      boys_eval_d<M, 32, 6, 6>(T, pre, [&](int k, double* c, double& ek) {
         constexpr int first = boys_rows_below_d(M);
         const double2* r = reinterpret_cast<const double2*>(tab) + 3 * (first + k);
-        r0 = r[0], r1 = r[1], r2 = r[2];
+        const double2 r0 = r[0], r1 = r[1], r2 = r[2];
+        c[0] = r0.x, c[1] = r0.y, c[2] = r1.x, c[3] = r1.y;
+        c[4] = __hiloint2double(__double2loint(r2.x), 0);
+        c[5] = r2.x;
+        ek = r2.y;
       }, F);
     } else {
       boys_eval_f<M>(T, pre, [&](int k) {
@@ -220,20 +220,26 @@ __host__ __device__ constexpr int npure_of(int L) { return 2 * L + 1; }
 // ---------------------------------------------------------------------------
 // Boys table of one order staged in shared memory.
 //
-// The same evaluation, reading the table of the kernel's single order MS from shared memory,
-// where a block puts it once with one bulk copy (stage_to_shared).  The
-// rows are stored as planes: FP64 plane j (j = 0..2) holds the j-th 16 bytes of every grid
-// point's row, so the three loads of one evaluation go to three planes and the lanes of a warp,
-// holding different T, spread over the banks by grid point; FP32 has one plane of float4 (values
-// 0..3).  Global layout: per order, boys_plane_stride<R>() bytes from the last, its planes back to
-// back: boys_plane_bytes<R>(M) bytes.
+// A block puts the table of the kernel's single order MS there once with one bulk copy
+// (stage_to_shared).  FP64: the grid of 1/8 with the eight full coefficients of the degree-7 interpolation
+// polynomial (its error, (h/2)^8 / (8! 2^7) F_{M+8}, is below 5e-17 of F_M) and e^d to degree 8, because a
+// block's residency hangs on the bytes: 20.8 kB (M = 0) to 28.3 kB (M = 4) against 55 to 75 kB of the rows
+// above, with which J/K builds in this form took 3.25 ms on n-octane and 28.1 on
+// anthracene, 2.33 and 18.2 with these (2.37 and 19.8 with rows of 48 bytes on the grid of 1/16).
+// Values are stored as planes: planes j = 0..3 of (c_2j, c_2j+1) over the grid points and one plane of
+// e^-T_k, so that the lanes of a warp, holding different T, spread over the banks by grid point; FP32 has
+// one plane of float4 (the Taylor terms 0..3 of its rows).  Global layout: per order, boys_plane_stride<R>()
+// bytes from the last, its planes back to back: boys_plane_bytes<R>(M) bytes.
 // ---------------------------------------------------------------------------
-#define BOYS_PLANES_D 3
+#define BOYS_STAGED_INVH 8
+#define BOYS_STAGED_COEF 8
 #define BOYS_STAGED_MMAX 4       // orders that are staged (classes of la + lb + lc + ld up to it)
 
+__host__ __device__ constexpr int boys_staged_points_d(int M) { return (int)(boys_tmax_d(M) * BOYS_STAGED_INVH) + 1; }
+
 template <typename R>
-__host__ __device__ constexpr int boys_plane_bytes(int M) {  // 55 kB (M = 0) to 75 kB (M = 4) in FP64, 5.8 kB in FP32
-  return 16 * (sizeof(R) == 8 ? BOYS_PLANES_D * boys_points_d(M) : BOYS_NGRID_F);
+__host__ __device__ constexpr int boys_plane_bytes(int M) {  // a multiple of 16; 5.8 kB in FP32
+  return (sizeof(R) == 8 ? (8 * (BOYS_STAGED_COEF + 1) * boys_staged_points_d(M) + 15) / 16 : BOYS_NGRID_F) * 16;
 }
 template <typename R>
 __host__ __device__ constexpr int boys_plane_stride() {
@@ -248,10 +254,16 @@ struct BoysShared {
   __device__ __forceinline__ void eval(R T, R pre, R* F) const {
     static_assert(M == MS && M <= BOYS_STAGED_MMAX, "the staged table holds one order");
     if constexpr (sizeof(R) == 8) {
-      boys_eval_d<M>(T, pre, [&](int k, double2& r0, double2& r1, double2& r2) {
-        constexpr int n = boys_points_d(M);
+      boys_eval_d<M, BOYS_STAGED_INVH, BOYS_STAGED_COEF, 8>(T, pre, [&](int k, double* c, double& ek) {
+        constexpr int n = boys_staged_points_d(M);
         const double2* P = reinterpret_cast<const double2*>(tab) + k;
-        r0 = P[0], r1 = P[n], r2 = P[2 * n];
+#pragma unroll
+        for (int j = 0; j < BOYS_STAGED_COEF / 2; ++j) {
+          const double2 v = P[j * n];
+          c[2 * j] = v.x;
+          c[2 * j + 1] = v.y;
+        }
+        ek = M > 0 ? tab[BOYS_STAGED_COEF * n + k] : 0.0;
       }, F);
     } else {
       boys_eval_f<M>(T, pre, [&](int k) { return reinterpret_cast<const float4*>(tab)[k]; }, F);

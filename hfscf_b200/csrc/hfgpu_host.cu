@@ -143,17 +143,29 @@ std::vector<double> boys_table_d() {
   return t;
 }
 
-// The same tables in the plane layout of BoysShared (hfgpu_common.cuh), for the orders that are staged:
-// per order, FP64 planes j = 0..2 of (row[2j], row[2j+1]) over the order's grid points; FP32 one plane
-// of row[0..3].
-std::vector<double> boys_planes_d(const std::vector<double>& rows) {
+// The tables of the staged orders in the plane layout of BoysShared (hfgpu_common.cuh).
+std::vector<double> boys_planes_d() {
+  constexpr int NC = BOYS_STAGED_COEF, NT = 14, NM = BOYS_STAGED_MMAX + NT;
+  constexpr long double h = 1.0L / BOYS_STAGED_INVH;  // Taylor terms j < 14, |d| <= 1/16: the rest is below 1e-27
+  std::vector<long double> F, ek;
+  boys_grid(boys_staged_points_d(BOYS_STAGED_MMAX), NM, h, F, ek);
+  long double z[NC], v[NC], c[NC];
+  cheb_points<NC>(h / 2, z);
   const size_t per = boys_plane_stride<double>() / sizeof(double);  // values per order
   std::vector<double> t((BOYS_STAGED_MMAX + 1) * per, 0.0);
-  for (int M = 0; M <= BOYS_STAGED_MMAX; ++M)
-    for (int k = 0; k < boys_points_d(M); ++k)
-      for (int j = 0; j < BOYS_PLANES_D; ++j)
-        memcpy(&t[M * per + ((size_t)j * boys_points_d(M) + k) * 2],
-               &rows[(size_t)(boys_rows_below_d(M) + k) * BOYS_ROW_D + 2 * j], 16);
+  for (int M = 0; M <= BOYS_STAGED_MMAX; ++M) {
+    const int n = boys_staged_points_d(M);
+    double* o = &t[M * per];
+    for (int k = 0; k < n; ++k) {
+      for (int i = 0; i < NC; ++i) {
+        v[i] = 0.0L;
+        for (int j = NT - 1; j >= 0; --j) v[i] = F[(size_t)k * NM + M + j] + v[i] * z[i] / (j + 1);
+      }
+      interpolate<NC>(z, v, c);
+      for (int j = 0; j < NC; ++j) o[((size_t)(j / 2) * n + k) * 2 + j % 2] = (double)c[j];
+      o[(size_t)NC * n + k] = (double)ek[k];
+    }
+  }
   return t;
 }
 std::vector<float> boys_planes_f(const std::vector<float>& rows) {
@@ -1848,7 +1860,7 @@ int hfgpu_create(const hfgpu_basis* b, const hfgpu_opts* opts, hfgpu_handle** ou
   // uploaded per handle
   static const std::vector<double> bt = boys_table_d();
   static const std::vector<float> btf = boys_table_f();
-  static const std::vector<double> bpd = boys_planes_d(bt);
+  static const std::vector<double> bpd = boys_planes_d();
   static const std::vector<float> bpf = boys_planes_f(btf);
   if (h->d_boys_d.ensure(sizeof(double) * bt.size()) || h->d_boys_f.ensure(sizeof(float) * btf.size()) ||
       h->d_boys_pd.ensure(sizeof(double) * bpd.size()) || h->d_boys_pf.ensure(sizeof(float) * bpf.size()) ||
