@@ -2669,6 +2669,18 @@ int hfgpu_autotune(hfgpu_handle* h, const double* D, int precision, int repeats,
   auto build = [&]() { return jk_device_impl(h, D, 1, D, nullptr, nullptr, precision); };
   int start[4 * 21];
   hfgpu_get_schedule(h, start);
+  // The schedule that is kept and returned names its lanes: a class left to the rule (-1) takes what the
+  // rule gives its many-primitive segments on these lists, the larger of the two.
+  for (int c = 0; c < hfgpu::kNumClasses; ++c) {
+    if (start[4 * c + 1] >= 0) continue;
+    const long long beg[2] = {h->q_beg[c], h->q_mid[c]}, end[2] = {h->q_hik1[c], h->q_hik2[c]};
+    int lanes = hfgpu::kClassLaunchers[c]->has_primwarp ? 0 : 1;
+    for (int k = 0; k < 2; ++k) {
+      const long long nq = (end[k] - beg[k] + h->nparts - 1) / h->nparts;
+      lanes = std::max(lanes, primwarp_group(h, c, 2 * k, nq, precision == HFGPU_MIXED && k == 1));
+    }
+    start[4 * c + 1] = lanes;
+  }
   // best candidate per class and kind of form: 0 thread per quartet, 1 primitive-split for
   // the many-primitive segments, 2 warp per quartet
   struct Cand {
@@ -2681,6 +2693,7 @@ int hfgpu_autotune(hfgpu_handle* h, const double* D, int precision, int repeats,
     return wp >= 1 ? 2 : (L->has_primwarp && pw > 0 ? 1 : (cap == 2 && L->has_staged ? 3 : 0));
   };
   for (int c = 0; c < hfgpu::kNumClasses; ++c) {
+    h->sched_primwarp[c] = start[4 * c + 1];
     if (h->q_end[c] <= h->q_beg[c]) continue;
     const hfgpu::ClassLaunchers* L = hfgpu::kClassLaunchers[c];
     h->class_mask = 1u << c;

@@ -324,7 +324,8 @@ int hfgpu_setup_times(const hfgpu_handle* h, double* ms);
  * keeps the fastest; then, on whole builds, tries per class the best candidate of each other
  * kind of form (thread, primitive-split, warp or block) and keeps it where the build gets at least 1%
  * faster; keeps the result only if whole builds with it beat whole builds with the schedule
- * it started from, and returns the schedule in `schedule` (may be NULL).  Last, it times the
+ * it started from (a -1 of [1] replaced by what it gives on these lists), and returns the
+ * schedule in `schedule` (may be NULL).  Last, it times the
  * classes of a build one after another on one stream against concurrently on six and keeps
  * the serial order where it is at least 1% faster (the handle keeps that choice; it is not
  * part of the schedule array).  Every timing is the median of separately timed runs, each
